@@ -279,11 +279,13 @@ __global__ void __launch_bounds__(TC_NT, IP ? 3 : 2)
   // of the step, kc = (q / 8) % 4.  A warp reads 8 rows x 64 bytes (coalesced) and every 8-lane phase of
   // a 16-byte shared-memory access covers one 128-byte core matrix (no bank conflicts).
   auto prow = [](int q) { return (q & 7) + 8 * (q >> 5); };
+  // row offsets may be negative: a batch rebases every system's rows onto system 0's arrays
+  constexpr int64_t NO_ROW = INT64_MIN;
   int64_t arow[4];
 #pragma unroll
   for (int i = 0; i < 4; i++) {
     const int r = m0 + prow(tid + TC_NT * i);
-    arow[i] = r < M ? aoff[r] : -1;
+    arow[i] = r < M ? aoff[r] : NO_ROW;
   }
   const int kq = ((tid >> 3) & 3) * 4;
   // raw A pieces (zero-filled outside the rows and K) and the operator rows of step c (absolute index),
@@ -314,7 +316,7 @@ __global__ void __launch_bounds__(TC_NT, IP ? 3 : 2)
       const int k = k0 + kq;
       const int left = K - k;
       const uint32_t dst = smem_u32(raw_piece(st, c, tid + TC_NT * i));
-      const bool any = arow[i] >= 0 && left > 0;
+      const bool any = arow[i] != NO_ROW && left > 0;
       const float* src = any ? A + arow[i] + k : A;  // a chunk that reads nothing still names A
       if constexpr (VA == 16) {
         const uint32_t valid = any ? (uint32_t)(left >= 4 ? 16 : 4 * left) : 0u;
