@@ -6,7 +6,7 @@
 //                                                        (pinv factors), scaled scatter (0.5^l)
 //   M2M   fmm_scale_invariant.h:233-253 / fmm.h:221-241  row gather + library GEMM per level, K = 8 nsurf
 //   P2L   fmm_base.h:127-154                             k_p2l
-//   M2L   fmm_scale_invariant.h:407-440, 560-646;        real kernels: k_m2l_fwd_r + k_hadamard_dt/_rt (opt-in:
+//   M2L   fmm_scale_invariant.h:407-440, 560-646;        real kernels: k_m2l_fwd_r + k_hadamard_h (opt-in:
 //         fmm.h:395-446, 631-788                         k_hadamard_dc on tcgen05) + k_m2l_bwd_r (FP64:
 //                                                        k_hadamard, k_m2l_bwd); complex kernel (p <= 12): k_m2l_fwd_c
 //                                                        + Hadamard + k_m2l_bwd_c; real p > 10 or p > 12:
@@ -19,6 +19,7 @@
 //   M2P   fmm_base.h:97-124                              far part: k_eval (Laplace mixed: k_far_lap)
 //   P2P   fmm_base.h:82-94                               near part: k_near (Laplace mixed: k_near_lap_f2)
 // Results stay in tree order until get_values scatters them (python/exafmm.cpp:194-207).
+#include <cuda_fp16.h>
 #include <cufft.h>
 
 #include <algorithm>
@@ -1085,11 +1086,11 @@ void transpose(const CT* in, CT* out, int64_t R, int64_t C, cudaStream_t s) {
 
 // Hadamard product per frequency (fmm_scale_invariant.h:343-399; intrinsics.h matmult_8x8x2):
 //   out[f][t][tc] = sum_ipos sum_sc T[ipos][f][sc*8 + tc] * in[f][src(t, ipos)][sc]
-// The FP64 path's form runs on the FP64 tensor cores (k_hadamard_d64), the mixed path's forms on the
-// TF32 tensor cores (k_hadamard_dt, k_hadamard_rt below).
+// The FP64 path's form runs on the FP64 tensor cores (k_hadamard_d64), the mixed path's on the FP16 tensor
+// cores with split operands (k_hadamard_h below).
 
 // Hadamard product of the FP64 path on the FP64 tensor cores (DMMA, mma.sync m8n8k4 f64), dense form for
-// every target: per frequency, D[target][16] = A[target][26 x 16] B[26 x 16][16] as in k_hadamard_dt,
+// every target: per frequency, D[target][16] = A[target][26 x 16] B[26 x 16][16] as in k_hadamard_h,
 // accumulated in FP64 by the tensor core across the positions.  A warp owns HAD64_TW tiles of 8 targets;
 // per (tile, position) eight DMMAs (4 reduction steps x 2 output halves) add the position's products to the
 // tile's accumulators.  The reduction index of step c is input real 4 t + c, so that a lane (g, t) supplies
@@ -1184,59 +1185,120 @@ __global__ void __launch_bounds__(HAD64_NT, 2)
   }
 }
 
-// M2L Hadamard product of the mixed path on the tensor cores (below).  Targets are split by how many of
-// the 26 relative positions are occupied: dense targets (at least HAD_DENSE_MIN) keep their sums in
-// registers across the positions (k_hadamard_dt); sparse targets -- the deepest nonleaf level, ~7 of 26 --
-// are scheduled by position (k_hadamard_rt): a CTA owns HADR_TT sparse targets at one frequency, their
-// pairs are grouped by position and packed on the host into rounds of HADR_RW pairs that share one 8x8
-// block, and each pair's products are added to its output row with 16-byte vector atomics resolved in
-// L2 (the sums are taken in a run-dependent order) on rows the same CTA zeroed first.
-// Spectra and products are frequency-major, (frequency f, node, child c) at [(f * nnodes + node) * 8 + c]:
-// a CTA (one frequency) reads its sources from one block of the spectra and writes its rows contiguously.
-#ifndef XFMM_HAD_DENSE_MIN
-#define XFMM_HAD_DENSE_MIN 12
-#endif
-constexpr int HAD_DENSE_MIN = XFMM_HAD_DENSE_MIN;  // occupied positions that make a target dense
-#ifndef XFMM_HAD_DENSE_GROUP_MIN
-#define XFMM_HAD_DENSE_GROUP_MIN 256
-#endif
-constexpr int HAD_DENSE_GROUP_MIN = XFMM_HAD_DENSE_GROUP_MIN;  // dense targets a group needs for the dense form
-constexpr int HADR_NT = 256;            // threads per CTA
-constexpr int HADR_TT = 512;            // targets per tile
-constexpr int HADR_RW = 64;             // pairs per round (4 row tiles of 16)
-#ifndef XFMM_HADR_TPC
-#define XFMM_HADR_TPC 4
-#endif
-constexpr int HADR_TPC = XFMM_HADR_TPC;  // default tiles per CTA (one B fill per frequency for all of them)
+// M2L Hadamard product of the mixed path on the tensor cores (k_hadamard_h, below).  Spectra and products are
+// frequency-major, (frequency f, node, child c) at [(f * nrows + node) * 8 + c]: a CTA (one frequency)
+// reads its sources from one block of the spectra and writes its rows contiguously.
+//
+// The mixed path's spectra are stored split: a real x of source node s is the pair of FP16 values
+// h = fp16(2^e x), t = fp16(2^e x - h), with one exponent e per source node (all its children and
+// frequencies), so that 22 bits of x survive as long as |x| is within 2^-17 of the node's bound and the
+// absolute error stays below 2^-39 of that bound elsewhere.  A split spectrum has the size of the FP32
+// one, the products need no conversion (the operator's blocks are split the same way, one exponent per
+// position and frequency), and an FP16 MMA does twice the work of a TF32 one in the same 8 cycles
+// (measured: m16n8k16 f16 and m16n8k8 tf32 both 8.0 cycles per warp and SM quadrant) with the same
+// 11-bit significands.  A child's complex value is the 8 bytes {h.re, h.im, t.re, t.im}.
+using SplitC = uint2;
+__device__ __forceinline__ uint32_t h2_bits(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
+__device__ __forceinline__ float2 h2_float2(uint32_t u) { return __half22float2(*reinterpret_cast<__half2*>(&u)); }
+__device__ __forceinline__ SplitC split16(float re, float im) {
+  const __half2 h = __floats2half2_rn(re, im);
+  const float2 hf = __half22float2(h);
+  return make_uint2(h2_bits(h), h2_bits(__floats2half2_rn(re - hf.x, im - hf.y)));
+}
+// The exponent e of a node whose spectrum values are at most `bound` in magnitude: 2^e bound < 2^15 (FP16
+// holds 2^16), e odd, as the code k = (127 - e) / 2 in 1..126, so that 2^-e is the float whose exponent
+// field is 2 k.
+__device__ __forceinline__ int split_code(float bound) {
+  int e = bound > 0.f ? 14 - ((int)(__float_as_uint(bound) >> 23) - 127) : 1;
+  e = max(-125, min(125, e));
+  if (!(e & 1)) e -= 1;
+  return (127 - e) >> 1;
+}
+__device__ __forceinline__ float split_scale(int code) { return __uint_as_float((uint32_t)(254 - 2 * code) << 23); }
+// Packed sources: the source row in the low 25 bits (2^25 sources would need 206 GB of spectra at the lowest
+// order) and 7 bits of exponent: in the opt-in tcgen05 form's table the source's code (written by
+// k_pack_sources after every forward transform), in a tile's slot list the source's distance from the tile's
+// common exponent (k_tile_codes).  SPLIT_NONE: no source.
+constexpr int SPLIT_ROW_BITS = 25;
+constexpr uint32_t SPLIT_ROW_MASK = (1u << SPLIT_ROW_BITS) - 1;
+constexpr uint32_t SPLIT_NONE = 0xffffffffu;
+__device__ __forceinline__ float split_inv(uint32_t ent) { return __uint_as_float((ent >> 1) & 0x7f000000u); }
+__device__ __forceinline__ float split_inv_code(int code) { return __uint_as_float((uint32_t)code << 24); }
+__global__ void k_pack_sources(const int* __restrict__ in, int64_t n, const int* __restrict__ scode,
+                               uint32_t* __restrict__ out) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    out[i] = in[i] >= 0 ? (uint32_t)in[i] | ((uint32_t)scode[in[i]] << SPLIT_ROW_BITS) : SPLIT_NONE;
+}
 
+// opt-in tcgen05 form (k_hadamard_dc): occupied positions that make a target dense, dense targets a group
+// needs; every other target runs in k_hadamard_h
+constexpr int HAD_DENSE_MIN = 12, HAD_DENSE_GROUP_MIN = 256;
+constexpr int HADC_TT = 512;  // padding of its source table
 
-// Hadamard product, dense form on the tensor cores (FP32 accuracy from three TF32 products).
-// Per frequency the dense product is a real GEMM, D[target][16] = A[target][26 x 16] B[26 x 16][16]:
-// a target's row of A holds its 26 source spectra (8 complex = 16 reals each, zero where a position is
-// empty) and B holds each position's 8x8 complex block as 2x2 real blocks ([re, im] -> [re, im]).
-// Warp-level m16n8k8 TF32 MMAs: A and B are split into TF32 heads and tails, and each position's
-// Ah Bh + Ah Bt + At Bh (small terms first; the tail-tail product, 2^-22 relative, is dropped) is
-// formed in a fresh MMA accumulator and added to FP32 running sums.  The reduction
-// index of each 8-wide step is ordered so that a lane's A fragment is one 16-byte piece of a source
-// spectrum (lane quad t of a row loads reals 4t..4t+3), and the B fragments of every (position, lane)
-// are laid out per frequency in shared memory.  A warp owns 64 targets as 4 tiles of 16 rows.
-#ifndef XFMM_HADT_TILES
-#define XFMM_HADT_TILES 4  // row tiles of 16 targets per warp
-#endif
-constexpr int HADT_NT = 256;                                    // threads per CTA
-constexpr int HADT_TILES = XFMM_HADT_TILES;
-constexpr int HADT_TT = (HADT_NT / 32) * 16 * HADT_TILES;      // targets per CTA tile
-#ifndef XFMM_HADT_TPC
-#define XFMM_HADT_TPC 1
-#endif
-constexpr int HADT_TPC = XFMM_HADT_TPC;                         // CTA tiles per CTA (one B fill for all)
-constexpr size_t HADT_SMEM = (size_t)26 * 4 * 32 * 16;
+// Hadamard product on the tensor cores (FP32 accuracy from three FP16 products).
+// Per frequency the product is a real GEMM, D[target][16] = A[target][26 x 16] B[26 x 16][16]: a target's
+// row of A holds its 26 source spectra (8 complex = 16 reals each, zeros where a position is empty) and B
+// holds each position's 8x8 complex block as 2x2 real blocks ([re, im] -> [re, im]).  Warp-level m16n8k16
+// FP16 MMAs with FP32 accumulators: A and B are FP16 heads and tails, and each position's
+// At Bh + Ah Bt + Ah Bh (small terms first; the tail-tail product, 2^-22 relative, is dropped) is formed in
+// a fresh MMA accumulator, scaled by the block's exponent and added to FP32 running sums in one fused
+// multiply-add (the MMA's own accumulation is not rounded to nearest).
+//
+// A CTA owns a tile of up to 512 targets at one frequency.  The tile's distinct sources (up to 1016, about
+// twice the targets of a spatially compact tile, each used by up to 26 of them) are brought into shared
+// memory once, on a common exponent, and every A fragment is read from there with ldmatrix, whose lanes
+// address the rows of a fragment freely: a gather without register moves at 8 shared-memory cycles per 16
+// targets and position.  Measured, Hadamard stage: 1M bodies, p = 10: 2.95 ms (the same products gathered
+// row by row from L1 at 14 cycles per 16 targets: 4.03; the TF32 form with per-use conversions before it:
+// 5.26); 4M, p = 8, whose deepest level has ~7 of 26 positions occupied: 4.38 (TF32 with packed rounds of
+// pairs and atomics: 6.15); Helmholtz 200k, p = 12: 1.71 (3.55).
+// Bank conflicts: a source's slot is 8 k + (octant of the source in its parent).  The sources of 8 sibling
+// targets at one relative position have 8 different octants, so their 64-byte rows (four 16-byte chunks,
+// swizzled by (slot / 2) % 4) fall on different banks; empty positions read one of 8 zero slots, chosen to
+// stay off the banks of the other rows.
+// Tiles with at most 256, 128 or 64 targets split the 26 positions over 2, 4 or 8 warps per 64 targets.
+// Bounds per 64 targets and position and SM (cycles): MMAs 24 x 8 / 4 = 48; shared memory 32 (A) + 8 (B).
+// At 1M, p = 8 the tensor pipe is 54% and the shared-memory pipe 64% busy: 16 warps per SM hide the rest of
+// the latencies only in part.  Smaller tiles at three CTAs per SM (384 targets, 704 slots) close early in
+// full volumes (p = 10: 3.83 ms); several tiles per CTA gain nothing.
+constexpr int HADH_NT = 256, HADH_TT = 512;      // threads, targets per tile
+constexpr int HADH_SLOTS = 1024;                 // source slots, the first 8 zeros
+constexpr int HADH_TPC = 1;                      // default tiles per CTA
+constexpr int HADH_B = 26 * 2 * 32;              // B fragments (uint4) in shared memory
+constexpr int HADH_FB = HADH_B / 2;              // and as stored
+constexpr size_t HADH_SMEM = (size_t)HADH_SLOTS * 64 + (size_t)HADH_B * 16 + 32 * sizeof(float);
+static_assert(2 * (HADH_SMEM + 1024) <= 228 * 1024, "two CTAs per SM");
+struct HadTile {
+  int nslots;   // slots used (a multiple of 8, the zero slots included)
+  int groups;   // 1, 2, 4 or 8 groups of 64 targets
+  int slot0;    // first entry of the tile in the slot list (source of each slot, -1: none)
+  int row0;     // first entry of the tile in the row list (output row of each target, -1: padding)
+  int64_t tab0; // first entry of the tile in the table: [position][group][lane] of 4 x 16 bits
+};
+struct HadSys {
+  const SplitC* in;       // split spectra [f][nsrc][child]
+  float2* out;            // products [f][target][child]
+  const HadTile* tiles;
+  const uint32_t* slots;  // packed source of each slot (k_tile_codes)
+  const float* tinv;      // per tile: undoes its exponent
+  const uint2* tab;
+  const int* rows;
+  int nsrc, ntrg;
+};
 
-__device__ __forceinline__ void mma_tf32(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                         uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+// not volatile: the compiler interleaves independent accumulators
+__device__ __forceinline__ void mma_f16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                        uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// the same into a fresh accumulator
+__device__ __forceinline__ void mma_f16_new(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                            uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
 }
 // head and tail of x: x = head + tail exactly, head a TF32 value
 __device__ __forceinline__ void tf32_split(float x, uint32_t& h, uint32_t& t) {
@@ -1244,229 +1306,273 @@ __device__ __forceinline__ void tf32_split(float x, uint32_t& h, uint32_t& t) {
   t = tf32_head(x - __uint_as_float(h));
 }
 
-// The B fragments of frequency f for every (position, reduction step c, output half h, lane):
-// sB[(ipos * 4 + c * 2 + h) * 32 + lane] = {b0 head, b1 head, b0 tail, b1 tail}, step c covering the
-// source components 2 t + c and half h the target components 4 h .. 4 h + 3 (t = lane % 4).
-__device__ __forceinline__ void hadt_fill_b(uint4* sB, const float2* __restrict__ T, int f, int nfreq, int tid,
-                                            int nthreads) {
-  for (int e = tid; e < 26 * 4 * 32; e += nthreads) {
-    const int ln = e & 31, q = (e >> 5) & 3, ipos = e >> 7;
-    const int c = q >> 1, h = q & 1, g = ln >> 2, t = ln & 3;
-    const int sc = 2 * t + c, tc = 4 * h + (g >> 1);
-    const float2 m = T[((int64_t)ipos * nfreq + f) * 64 + sc * 8 + tc];
-    // input real (sc, re) -> b0, (sc, im) -> b1; output real (tc, g & 1): re <- (Re m, -Im m), im <- (Im m, Re m)
-    const float v0 = (g & 1) ? m.y : m.x, v1 = (g & 1) ? m.x : -m.y;
-    uint4 b;
-    tf32_split(v0, b.x, b.z);
-    tf32_split(v1, b.y, b.w);
-    sB[e] = b;
-  }
-}
-
-// D (16 x 16) += rows (x0: row g, x1: row g + 8) times the position's B, one fresh MMA accumulator:
-// d[h][0..1] = row g, target component 4 h + t (re, im); d[h][2..3] = row g + 8
-__device__ __forceinline__ void hadt_tile(const float4& x0, const float4& x1, const uint4 (&b)[4], float (&d)[2][4]) {
+// The operator blocks of frequency f as the kernel's B fragments, built once per operator table from its
+// FP64 values: for every (position, output half h, lane) of a warp the four registers {b0 head, b1 head,
+// b0 tail, b1 tail}, scaled by the block's exponent; b0 / b1 are the factors of source components t / t + 4
+// and half h the target components 4 h .. 4 h + 3 (t = lane % 4).  Stored are the lanes of even g = lane / 4
+// (real outputs: (Re, -Im) of a factor), at frag[f * HADH_FB + (ipos * 2 + h) * 16 + 4 (g / 2) + t]; those of
+// g + 1 (imaginary outputs: (Im, Re)) are the same values swapped (hadh_odd).  inv[f * 32 + ipos] undoes the
+// exponent.  One warp per block.
+__global__ void k_m2l_fragments(const double2* __restrict__ T, int nfreq, uint4* __restrict__ frag,
+                                float* __restrict__ inv) {
+  const int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (w >= 26ll * nfreq) return;
+  const int f = (int)(w / 26), ipos = (int)(w % 26);
+  const double2* blk = T + ((int64_t)ipos * nfreq + f) * 64;
+  const double2 u = blk[lane], v = blk[32 + lane];
+  float m = (float)fmax(fmax(fabs(u.x), fabs(u.y)), fmax(fabs(v.x), fabs(v.y)));
 #pragma unroll
-  for (int h = 0; h < 2; h++)
-#pragma unroll
-    for (int i = 0; i < 4; i++) d[h][i] = 0.f;
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  const int code = split_code(m);
+  const double sc = (double)split_scale(code);
+  const int h = lane >> 4, tc = 4 * h + ((lane >> 2) & 3), t = lane & 3;
+  uint32_t hd[2], tl[2];
 #pragma unroll
   for (int c = 0; c < 2; c++) {
-    uint32_t a0h, a0t, a1h, a1t, a2h, a2t, a3h, a3t;
-    tf32_split(c == 0 ? x0.x : x0.z, a0h, a0t);
-    tf32_split(c == 0 ? x1.x : x1.z, a1h, a1t);
-    tf32_split(c == 0 ? x0.y : x0.w, a2h, a2t);
-    tf32_split(c == 0 ? x1.y : x1.w, a3h, a3t);
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-      const uint4 bb = b[c * 2 + h];
-      mma_tf32(d[h], a0t, a1t, a2t, a3t, bb.x, bb.y);
-      mma_tf32(d[h], a0h, a1h, a2h, a3h, bb.z, bb.w);
-      mma_tf32(d[h], a0h, a1h, a2h, a3h, bb.x, bb.y);
-    }
+    const double2 q = blk[(t + 4 * c) * 8 + tc];
+    const double re = q.x * sc, im = -q.y * sc;
+    const __half2 hh = __halves2half2(__double2half(re), __double2half(im));
+    const float2 hf = __half22float2(hh);
+    hd[c] = h2_bits(hh);
+    tl[c] = h2_bits(__halves2half2(__double2half(re - hf.x), __double2half(im - hf.y)));
   }
+  frag[(int64_t)f * HADH_FB + ipos * 32 + lane] = make_uint4(hd[0], hd[1], tl[0], tl[1]);
+  if (lane == 0) inv[(int64_t)f * 32 + ipos] = split_inv_code(code);
+}
+// the registers of lane g + 1 from those of an even g: (Re, -Im) -> (Im, Re) in every half pair
+__device__ __forceinline__ uint4 hadh_odd(const uint4& e) {
+  auto sw = [](uint32_t v) { return __byte_perm(v, v, 0x1032) ^ 0x8000u; };
+  return make_uint4(sw(e.x), sw(e.y), sw(e.z), sw(e.w));
+}
+// After a forward transform, per tile (one CTA each): the largest exponent code of its sources, the common
+// exponent, and the slot list packed with every source's distance d from it (SPLIT_NONE: no source).
+__global__ void __launch_bounds__(256)
+    k_tile_codes(const HadTile* __restrict__ tiles, const int* __restrict__ slots, const int* __restrict__ scode,
+                 uint32_t* __restrict__ pslots, float* __restrict__ tinv) {
+  __shared__ int smax;
+  const HadTile T = tiles[blockIdx.x];
+  if (threadIdx.x == 0) smax = 1;
+  __syncthreads();
+  int src[(HADH_SLOTS + 255) / 256], code[(HADH_SLOTS + 255) / 256], kmax = 1;
+#pragma unroll
+  for (int i = 0; i < (HADH_SLOTS + 255) / 256; i++) {
+    const int q = threadIdx.x + 256 * i;
+    src[i] = q < T.nslots ? slots[T.slot0 + q] : -1;
+    code[i] = src[i] >= 0 ? scode[src[i]] : 0;
+    kmax = max(kmax, code[i]);
+  }
+  atomicMax(&smax, __reduce_max_sync(0xffffffffu, kmax));
+  __syncthreads();
+  kmax = smax;
+#pragma unroll
+  for (int i = 0; i < (HADH_SLOTS + 255) / 256; i++) {
+    const int q = threadIdx.x + 256 * i;
+    if (q < T.nslots)
+      pslots[T.slot0 + q] = src[i] >= 0 ? (uint32_t)src[i] | (uint32_t)(kmax - code[i]) << SPLIT_ROW_BITS : SPLIT_NONE;
+  }
+  if (threadIdx.x == 0) tinv[blockIdx.x] = split_inv_code(kmax);
 }
 
-// Round form on the tensor cores (sparse targets): each round of 64 same-position pairs as 4 row tiles of
-// 16 (pair 16 j + g and 16 j + 8 + g of tile j); lanes t and t ^ 1 trade halves so each adds 16 bytes
-// (two target components of one pair) with a vector atomic.  Rounds [r0, r1) at one frequency: warp wid
-// takes every (HADR_NT / 32)-th round; inf points at the frequency's spectra (+ lane quad offset t), of at
-// its product rows, and the rows were zeroed by the same CTA.
-__device__ __forceinline__ void hadr_rounds(const uint4* sB, const float4* __restrict__ inf, float2* of,
-                                            const int* __restrict__ rpos, const int2* __restrict__ ent, int r0,
-                                            int r1, int wid, int lane) {
-  constexpr int NW = HADR_NT / 32;
-  static_assert(HADR_RW == 64, "a round is 4 row tiles of 16 pairs");
+__device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr)
+               : "memory");
+}
+// Table entry of a slot: 4 slot + swizzle; chunk c of the slot is at 16 (entry ^ c).
+__host__ __device__ __forceinline__ uint32_t hadh_entry(int slot) { return (uint32_t)(4 * slot + ((slot >> 1) & 3)); }
+
+// one tile at frequency f; its first tile also stores the CTA's B fragments and block scales (frag, binv: those
+// of f) into shared memory
+__device__ __forceinline__ void hadh_tile(const HadSys& S, int tile, int f, unsigned char* sA, uint4* sB, float* sInv,
+                                          const uint4* __restrict__ frag, const float* __restrict__ binv, bool first,
+                                          int tid) {
+  const HadTile T = S.tiles[tile];
+  const int lane = tid & 31, wid = tid >> 5;
+  // ---- the tile's sources: four threads per slot, 16 bytes each
+  const uint4* inf = reinterpret_cast<const uint4*>(S.in + (int64_t)f * S.nsrc * 8);
+  const uint32_t* slots = S.slots + T.slot0;
+  constexpr int QS = HADH_NT / 4, NB = (HADH_SLOTS + QS - 1) / QS;  // slots per round; rounds, all in flight
+  const int c = tid & 3;
+  constexpr int NF = (HADH_FB + HADH_NT - 1) / HADH_NT;
+  uint4 fb[NF];
+  if (first) {
+#pragma unroll
+    for (int i = 0; i < NF; i++) fb[i] = __ldg(frag + min(tid + HADH_NT * i, HADH_FB - 1));
+  }
+  uint32_t src[NB];
+#pragma unroll
+  for (int i = 0; i < NB; i++) {
+    const int q = (tid >> 2) + QS * i;
+    src[i] = q < T.nslots ? slots[q] : SPLIT_NONE;
+  }
+  uint4 v[NB];
+#pragma unroll
+  for (int i = 0; i < NB; i++) {
+    const uint32_t e = src[i];
+    v[i] = e != SPLIT_NONE ? __ldg(inf + (int64_t)(e & SPLIT_ROW_MASK) * 4 + c) : make_uint4(0u, 0u, 0u, 0u);
+  }
+#pragma unroll
+  for (int i = 0; i < NB; i++) {
+    const int q = (tid >> 2) + QS * i;
+    if (q >= T.nslots) break;
+    const int d = (int)(src[i] >> SPLIT_ROW_BITS);  // 2^(-2 d) brings the source to the common exponent
+    uint4 w = v[i];
+    if (d > 0) {
+      const __half2 m = __float2half2_rn(__uint_as_float((uint32_t)max(0, 127 - 2 * d) << 23));
+      w.x = h2_bits(__hmul2(*reinterpret_cast<__half2*>(&w.x), m));
+      w.y = h2_bits(__hmul2(*reinterpret_cast<__half2*>(&w.y), m));
+      w.z = h2_bits(__hmul2(*reinterpret_cast<__half2*>(&w.z), m));
+      w.w = h2_bits(__hmul2(*reinterpret_cast<__half2*>(&w.w), m));
+    }
+    // global pieces are children 2c, 2c + 1 as {head, tail, head, tail}; shared chunks are heads of
+    // children 0-3 and 4-7, then tails
+    const uint32_t e = hadh_entry(q);
+    *reinterpret_cast<uint2*>(sA + 16 * (e ^ (c >> 1)) + 8 * (c & 1)) = make_uint2(w.x, w.z);
+    *reinterpret_cast<uint2*>(sA + 16 * (e ^ (2 + (c >> 1))) + 8 * (c & 1)) = make_uint2(w.y, w.w);
+  }
+  if (first) {
+#pragma unroll
+    for (int i = 0; i < NF; i++) {
+      const int e = tid + HADH_NT * i, ln = e & 15;  // stored lane 4 (g / 2) + t
+      if (e >= HADH_FB) break;
+      uint4* o = sB + (e >> 4) * 32 + (ln >> 2) * 8 + (ln & 3);
+      o[0] = fb[i];
+      o[4] = hadh_odd(fb[i]);
+    }
+    if (tid < 26) sInv[tid] = binv[tid];
+  }
+  __syncthreads();
+  // ---- products: group gr of 64 targets, positions ps, ps + np, ...
+  const int gr = wid % T.groups, ps = wid / T.groups, np = (HADH_NT / 32) / T.groups;
   const int g = lane >> 2, t = lane & 3;
-  // a round's pairs (source, output row) and their spectra, all loads in flight at once
-  auto load_round = [&](int r, int2 (&ee)[4][2], float4 (&xx)[4][2]) {
+  const uint32_t a0 = tc5::smem_u32(sA);
+  const uint32_t ch = (uint32_t)(lane >> 4);
+  const uint2* tab = S.tab + T.tab0 + gr * 32 + lane;
+  const int pstep = T.groups * 32;
+  float acc[4][2][4];
 #pragma unroll
-    for (int j = 0; j < 4; j++)
-#pragma unroll
-      for (int rr = 0; rr < 2; rr++) ee[j][rr] = ent[(int64_t)r * HADR_RW + 16 * j + 8 * rr + g];
-#pragma unroll
-    for (int j = 0; j < 4; j++)
-#pragma unroll
-      for (int rr = 0; rr < 2; rr++)
-        xx[j][rr] = ee[j][rr].x >= 0 ? __ldg(inf + (int64_t)ee[j][rr].x * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
-  };
-  for (int r = r0 + wid; r < r1; r += NW) {
-    const int ipos = rpos[r];
-    uint4 b[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) b[q] = sB[(ipos * 4 + q) * 32 + lane];
-    int2 ee[4][2];
-    float4 xx[4][2];
-    load_round(r, ee, xx);
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      float d[2][4];
-      hadt_tile(xx[j][0], xx[j][1], b, d);
-      const bool odd = t & 1;
-      const int2 e = odd ? ee[j][1] : ee[j][0];
-#pragma unroll
-      for (int h = 0; h < 2; h++) {
-        // even t keeps row g (components 4h + t, 4h + t + 1); odd t keeps row g + 8 (4h + t - 1, 4h + t)
-        const float2 send = odd ? make_float2(d[h][0], d[h][1]) : make_float2(d[h][2], d[h][3]);
-        const float rx = __shfl_xor_sync(0xffffffffu, send.x, 1), ry = __shfl_xor_sync(0xffffffffu, send.y, 1);
-        const float4 v = odd ? make_float4(rx, ry, d[h][2], d[h][3]) : make_float4(d[h][0], d[h][1], rx, ry);
-        if (e.x >= 0) atomicAdd(reinterpret_cast<float4*>(of + (int64_t)e.y * 8 + 4 * h + (t & ~1)), v);
-      }
-    }
-  }
-}
-
-__global__ void __launch_bounds__(HADR_NT, 3)  // 3 blocks/SM measured best (80 registers, a 16-byte spill)
-    k_hadamard_rt(const float2* __restrict__ T, const float2* __restrict__ in, float2* __restrict__ out,
-                  const int* __restrict__ tile_r, const int* __restrict__ rpos, const int2* __restrict__ ent,
-                  const int* __restrict__ rows, int ntiles, int tpc, int nsrc, int ntrg, int nfreq) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  uint4* sB = reinterpret_cast<uint4*>(smem_raw);
-  const int f = blockIdx.y, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  // tiles [tb, te) share this CTA's B fragments of frequency f
-  const int tb = blockIdx.x * tpc, te = min(ntiles, tb + tpc);
-  float2* of = out + (int64_t)f * ntrg * 8;
-  // every product of these tiles' targets at frequency f is added by this CTA: their rows start at zero
-  for (int e = tid; e < (te - tb) * HADR_TT * 4; e += HADR_NT) {
-    const int row = rows[tb * HADR_TT + (e >> 2)];
-    if (row >= 0) reinterpret_cast<float4*>(of + (int64_t)row * 8)[e & 3] = make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-  hadt_fill_b(sB, T, f, nfreq, tid, HADR_NT);
-  __syncthreads();
-  const float4* inf = reinterpret_cast<const float4*>(in + (int64_t)f * nsrc * 8) + (lane & 3);
-  hadr_rounds(sB, inf, of, rpos, ent, tile_r[tb], tile_r[te], wid, lane);
-}
-
-// The round form over the sparse tiles of many systems that share one operator table (a batch of Laplace
-// systems): tiles[k] = (system, its tile), and a CTA covers tiles [tb, te) of the list, possibly of several
-// systems, with one B fill per frequency.
-struct HadSys {
-  const float2* in;     // spectra [f][source][child]
-  float2* out;          // products [f][target][child]
-  const int* tile_r;    // rounds of each sparse tile (CSR)
-  const int* rpos;      // relative position of each round
-  const int2* ent;      // pairs of each round
-  const int* rows;      // HADR_TT output rows per tile
-  int nsrc, ntrg;
-};
-__global__ void __launch_bounds__(HADR_NT, 3)
-    k_hadamard_rt_batch(const float2* __restrict__ T, const HadSys* __restrict__ sys, const int2* __restrict__ tiles,
-                        int ntiles, int tpc, int nfreq) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  uint4* sB = reinterpret_cast<uint4*>(smem_raw);
-  const int f = blockIdx.y, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const int tb = blockIdx.x * tpc, te = min(ntiles, tb + tpc);
-  for (int k = tb; k < te; k++) {
-    const int2 tl = tiles[k];
-    const HadSys& S = sys[tl.x];
-    float2* of = S.out + (int64_t)f * S.ntrg * 8;
-    const int* rows = S.rows + (int64_t)tl.y * HADR_TT;
-    for (int e = tid; e < HADR_TT * 4; e += HADR_NT) {
-      const int row = rows[e >> 2];
-      if (row >= 0) reinterpret_cast<float4*>(of + (int64_t)row * 8)[e & 3] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-  }
-  hadt_fill_b(sB, T, f, nfreq, tid, HADR_NT);
-  __syncthreads();
-  for (int k = tb; k < te; k++) {
-    const int2 tl = tiles[k];
-    const HadSys& S = sys[tl.x];
-    const float4* inf = reinterpret_cast<const float4*>(S.in + (int64_t)f * S.nsrc * 8) + (lane & 3);
-    hadr_rounds(sB, inf, S.out + (int64_t)f * S.ntrg * 8, S.rpos, S.ent, S.tile_r[tl.y], S.tile_r[tl.y + 1], wid,
-                lane);
-  }
-}
-
-// tab: [26][ld] compact source index of dense target k at each position (-1: empty or padding);
-// rows: [ld] output row of dense target k (-1: padding).  ld is a multiple of HADT_TT.
-__global__ void __launch_bounds__(HADT_NT, 2)
-    k_hadamard_dt(const float2* __restrict__ T, const float2* __restrict__ in, float2* __restrict__ out,
-                  const int* __restrict__ tab, int ld, const int* __restrict__ rows, int nsrc, int ntrg, int nfreq) {
-  // sB[(ipos * 4 + c * 2 + h) * 32 + lane] = {b0 head, b1 head, b0 tail, b1 tail} of reduction step c
-  // (source components 2 t + c) and output half h (target components 4 h .. 4 h + 3) for that lane
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  uint4* sB = reinterpret_cast<uint4*>(smem_raw);  // 26 * 4 * 32 entries
-  const int f = blockIdx.y, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  hadt_fill_b(sB, T, f, nfreq, tid, HADT_NT);
-  __syncthreads();
-  const int g = lane >> 2, t = lane & 3;
-  const float4* inf = reinterpret_cast<const float4*>(in + (int64_t)f * nsrc * 8) + t;
-  // CTA tiles [blockIdx.x * HADT_TPC, ...) of HADT_TT targets share this CTA's B fragments of frequency f
-  for (int ct = blockIdx.x * HADT_TPC; ct < min(ld / HADT_TT, (blockIdx.x + 1) * HADT_TPC); ct++) {
-  const int base = ct * HADT_TT + wid * 16 * HADT_TILES + g;  // tile j, rows g / g + 8: base + 16 j (+ 8)
-  float acc[HADT_TILES][2][4];
-#pragma unroll
-  for (int j = 0; j < HADT_TILES; j++)
+  for (int j = 0; j < 4; j++)
 #pragma unroll
     for (int h = 0; h < 2; h++)
 #pragma unroll
       for (int i = 0; i < 4; i++) acc[j][h][i] = 0.f;
-  float4 x[HADT_TILES][2];
-  int srcn[HADT_TILES][2];  // source indices of the next position, loaded one position ahead
+  // table entries two positions ahead
+  uint2 e0 = __ldg(tab + ps * pstep), e1 = __ldg(tab + min(ps + np, 25) * pstep);
+  for (int ipos = ps; ipos < 26; ipos += np) {
+    const uint2 e = e0;
+    e0 = e1;
+    e1 = __ldg(tab + min(ipos + 2 * np, 25) * pstep);
+    const uint4 b[2] = {sB[(ipos * 2) * 32 + lane], sB[(ipos * 2 + 1) * 32 + lane]};
+    const float ib = sInv[ipos];
 #pragma unroll
-  for (int j = 0; j < HADT_TILES; j++)
+    for (int jp = 0; jp < 4; jp += 2) {
+      uint32_t xh[2][4], xt[2][4];
+      const uint32_t ee = jp ? e.y : e.x;
 #pragma unroll
-    for (int r = 0; r < 2; r++) srcn[j][r] = tab[base + 16 * j + 8 * r];
-  for (int ipos = 0; ipos < 26; ipos++) {
-#pragma unroll
-    for (int j = 0; j < HADT_TILES; j++)
-#pragma unroll
-      for (int r = 0; r < 2; r++) {
-        const int src = srcn[j][r];
-        if (ipos + 1 < 26) srcn[j][r] = tab[(ipos + 1) * ld + base + 16 * j + 8 * r];
-        x[j][r] = src >= 0 ? __ldg(inf + (int64_t)src * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int jj = 0; jj < 2; jj++) {
+        const uint32_t en16 = (jj ? ee >> 16 : ee & 0xffffu) ^ ch;
+        ldsm_x4(a0 + (en16 << 4), xh[jj]);
+        ldsm_x4(a0 + ((en16 ^ 2u) << 4), xt[jj]);
       }
-    uint4 b[4];
+      float d[2][2][4];
 #pragma unroll
-    for (int q = 0; q < 4; q++) b[q] = sB[(ipos * 4 + q) * 32 + lane];
+      for (int jj = 0; jj < 2; jj++)
 #pragma unroll
-    for (int j = 0; j < HADT_TILES; j++) {
-      // this position's products in a fresh MMA accumulator, then added to the running sums with
-      // round-to-nearest FP32 adds (the MMA's own accumulation is not rounded to nearest)
-      float d[2][4];
-      hadt_tile(x[j][0], x[j][1], b, d);
+        for (int h = 0; h < 2; h++) mma_f16_new(d[jj][h], xt[jj][0], xt[jj][1], xt[jj][2], xt[jj][3], b[h].x, b[h].y);
 #pragma unroll
-      for (int h = 0; h < 2; h++)
+      for (int jj = 0; jj < 2; jj++)
 #pragma unroll
-        for (int i = 0; i < 4; i++) acc[j][h][i] += d[h][i];
+        for (int h = 0; h < 2; h++) mma_f16(d[jj][h], xh[jj][0], xh[jj][1], xh[jj][2], xh[jj][3], b[h].z, b[h].w);
+#pragma unroll
+      for (int jj = 0; jj < 2; jj++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) mma_f16(d[jj][h], xh[jj][0], xh[jj][1], xh[jj][2], xh[jj][3], b[h].x, b[h].y);
+#pragma unroll
+      for (int jj = 0; jj < 2; jj++)
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+#pragma unroll
+          for (int i = 0; i < 4; i++) acc[jp + jj][h][i] = fmaf(d[jj][h][i], ib, acc[jp + jj][h][i]);
+    }
+  }
+  // ---- the position parts of a group, added in order by its first warp
+  if (np > 1) {
+    __syncthreads();
+    float4* red = reinterpret_cast<float4*>(sA) + wid * 8 * 32 + lane;
+    if (ps > 0) {
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+          red[(2 * j + h) * 32] = make_float4(acc[j][h][0], acc[j][h][1], acc[j][h][2], acc[j][h][3]);
+    }
+    __syncthreads();
+    if (ps > 0) return;
+    for (int k = 1; k < np; k++) {
+      const float4* r = red + k * T.groups * 8 * 32;
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const float4 w = r[(2 * j + h) * 32];
+          acc[j][h][0] += w.x;
+          acc[j][h][1] += w.y;
+          acc[j][h][2] += w.z;
+          acc[j][h][3] += w.w;
+        }
     }
   }
   // D fragment: row g (and g + 8), columns 2t, 2t + 1 of half h = target component 4 h + t (re, im)
-  float2* of = out + (int64_t)f * ntrg * 8;
+  const float inv = S.tinv[tile];
+  float2* of = S.out + (int64_t)f * S.ntrg * 8;
+  const int* rows = S.rows + T.row0 + gr * 64 + g;
 #pragma unroll
-  for (int j = 0; j < HADT_TILES; j++)
+  for (int j = 0; j < 4; j++)
 #pragma unroll
     for (int r = 0; r < 2; r++) {
-      const int row = rows[base + 16 * j + 8 * r];
+      const int row = rows[16 * j + 8 * r];
       if (row < 0) continue;
 #pragma unroll
-      for (int h = 0; h < 2; h++) of[(int64_t)row * 8 + 4 * h + t] = make_float2(acc[j][h][2 * r], acc[j][h][2 * r + 1]);
+      for (int h = 0; h < 2; h++)
+        of[(int64_t)row * 8 + 4 * h + t] = make_float2(acc[j][h][2 * r] * inv, acc[j][h][2 * r + 1] * inv);
     }
+}
+
+// tiles [blockIdx.x * tpc, ...) at frequency blockIdx.y share one copy of the frequency's B fragments
+__global__ void __launch_bounds__(HADH_NT, 2)
+    k_hadamard_h(const uint4* __restrict__ frag, const float* __restrict__ binv, HadSys S, int ntiles, int tpc) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  uint4* sB = reinterpret_cast<uint4*>(smem_raw + (size_t)HADH_SLOTS * 64);
+  float* sInv = reinterpret_cast<float*>(sB + HADH_B);
+  const int f = blockIdx.y, tid = threadIdx.x;
+  const int te = min(ntiles, ((int)blockIdx.x + 1) * tpc);
+  for (int k = blockIdx.x * tpc; k < te; k++) {
+    hadh_tile(S, k, f, smem_raw, sB, sInv, frag + (int64_t)f * HADH_FB, binv + f * 32, k == (int)blockIdx.x * tpc, tid);
+    if (k + 1 < te) __syncthreads();
+  }
+}
+// the same over the tiles of many systems that share one operator table (a batch of Laplace systems):
+// tiles[k] = (system, its tile)
+__global__ void __launch_bounds__(HADH_NT, 2)
+    k_hadamard_h_batch(const uint4* __restrict__ frag, const float* __restrict__ binv, const HadSys* __restrict__ sys,
+                       const int2* __restrict__ tiles, int ntiles, int tpc) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  uint4* sB = reinterpret_cast<uint4*>(smem_raw + (size_t)HADH_SLOTS * 64);
+  float* sInv = reinterpret_cast<float*>(sB + HADH_B);
+  const int f = blockIdx.y, tid = threadIdx.x;
+  const int te = min(ntiles, ((int)blockIdx.x + 1) * tpc);
+  for (int k = blockIdx.x * tpc; k < te; k++) {
+    const int2 tl = tiles[k];
+    hadh_tile(sys[tl.x], tl.y, f, smem_raw, sB, sInv, frag + (int64_t)f * HADH_FB, binv + f * 32,
+              k == (int)blockIdx.x * tpc, tid);
+    if (k + 1 < te) __syncthreads();
   }
 }
 
 // Hadamard product, dense form on the sm_100 tensor cores through tcgen05 (FP32 accuracy from three TF32
-// products, as in k_hadamard_dt), as a warp-specialised pipeline.  A CTA owns 128 dense targets (target
+// products of the spectra's head + tail), as a warp-specialised pipeline.  A CTA owns 128 dense targets (target
 // slot i = TMEM lane i) and HADC_FPB frequencies, i.e. a stream of 26 HADC_FPB positions.
 //   * Warps 0-3 (one per TMEM lane quarter) produce and consume: per position, the 4 lanes of a quad load
 //     one source spectrum as 4 contiguous 16-byte pieces (one position ahead), split it into TF32 head
@@ -1510,13 +1616,18 @@ __host__ __device__ __forceinline__ int hadc_col(int k) {
 __host__ __device__ __forceinline__ uint32_t hadc_boff(int n, int c) {
   return (uint32_t)((c >> 2) * 256 + (n >> 3) * 128 + (n & 7) * 16 + (c & 3) * 4);
 }
-// btab[f] (HADC_BBYTES per frequency): factor m(sc, tc) of position ipos -> the real 2 x 2 block
-// (outputs 2 tc, 2 tc + 1; inputs 2 sc, 2 sc + 1) = [[Re m, -Im m], [Im m, Re m]], TF32 head then tail
-__global__ void k_hadc_btab(const float2* __restrict__ T, int nfreq, unsigned char* __restrict__ btab) {
+// btab[f] (HADC_BBYTES per frequency): factor m(sc, tc) of position ipos (head + tail of the stored
+// fragments) -> the real 2 x 2 block (outputs 2 tc, 2 tc + 1; inputs 2 sc, 2 sc + 1) =
+// [[Re m, -Im m], [Im m, Re m]], TF32 head then tail
+__global__ void k_hadc_btab(const uint4* __restrict__ frag, const float* __restrict__ binv, int nfreq,
+                            unsigned char* __restrict__ btab) {
   const int64_t total = (int64_t)nfreq * 26 * 64;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     const int f = (int)(e / (26 * 64)), ipos = (int)(e / 64 % 26), sc = (int)(e >> 3 & 7), tc = (int)(e & 7);
-    const float2 m = T[((int64_t)ipos * nfreq + f) * 64 + sc * 8 + tc];
+    const uint4 q = frag[(int64_t)f * HADH_FB + (ipos * 2 + (tc >> 2)) * 16 + 4 * (tc & 3) + (sc & 3)];
+    const float2 hd = h2_float2(sc < 4 ? q.x : q.y), tl = h2_float2(sc < 4 ? q.z : q.w);
+    const float bi = binv[f * 32 + ipos];
+    const float2 m = make_float2((hd.x + tl.x) * bi, -(hd.y + tl.y) * bi);
     const float v[4] = {m.x, -m.y, m.y, m.x};
     unsigned char* blk = btab + (int64_t)f * HADC_BBYTES + ipos * 2048;
 #pragma unroll
@@ -1535,8 +1646,8 @@ __device__ __forceinline__ bool hadc_wait(uint32_t mbar, uint32_t parity) {
 }
 
 __global__ void __launch_bounds__(HADC_NT, 2)
-    k_hadamard_dc(const unsigned char* __restrict__ btab, const float2* __restrict__ in, float2* __restrict__ out,
-                  const int* __restrict__ tab, int ld, const int* __restrict__ rows, int nsrc, int ntrg, int nfreq,
+    k_hadamard_dc(const unsigned char* __restrict__ btab, const SplitC* __restrict__ in, float2* __restrict__ out,
+                  const uint32_t* __restrict__ tab, int ld, const int* __restrict__ rows, int nsrc, int ntrg, int nfreq,
                   int* __restrict__ status) {
   using namespace tc5;
   extern __shared__ __align__(16) unsigned char smem_raw[];  // B blocks of the current frequency, gather ring
@@ -1627,7 +1738,7 @@ __global__ void __launch_bounds__(HADC_NT, 2)
 #pragma unroll
     for (int i = 0; i < 16; i++) acc[i] = 0.f;
     auto inf_of = [&](int gi) {
-      return reinterpret_cast<const float4*>(in + (int64_t)(fbeg + gi / 26) * nsrc * 8);
+      return reinterpret_cast<const uint4*>(in + (int64_t)(fbeg + gi / 26) * nsrc * 8);
     };
     auto take = [&](int gp, int s) {  // products of stream position gp (stage s) into the sums
       fence_after_sync();
@@ -1649,14 +1760,15 @@ __global__ void __launch_bounds__(HADC_NT, 2)
     // gather ring: slot r holds, per warp and lane, the lane's 4 spectrum pieces (rows g + 8 i) of one
     // position; each lane reads back only what it copied itself
     const uint32_t ring = sB + HADC_BBYTES + (uint32_t)((wid * 4) * 32 + lane) * 16;
-    auto gather = [&](int gi, int idx) {  // cp.async of position gi into its slot (one commit group)
-      const float4* inf = inf_of(gi);
+    auto gather = [&](int gi, uint32_t ent) {  // cp.async of position gi into its slot (one commit group)
+      const uint4* inf = inf_of(gi);
       const uint32_t slot = ring + (uint32_t)(gi % HADC_R) * (128 * 64);
 #pragma unroll
       for (int i = 0; i < 4; i++) {
-        const int src = __shfl_sync(0xffffffffu, idx, g + 8 * i);
-        cp_async16(slot + i * 32 * 16, src >= 0 ? (const void*)(inf + (int64_t)src * 4 + q) : (const void*)in,
-                   src >= 0 ? 16u : 0u);
+        const uint32_t e = __shfl_sync(0xffffffffu, ent, g + 8 * i);
+        cp_async16(slot + i * 32 * 16,
+                   e != SPLIT_NONE ? (const void*)(inf + (int64_t)(e & SPLIT_ROW_MASK) * 4 + q) : (const void*)in,
+                   e != SPLIT_NONE ? 16u : 0u);
       }
       cp_async_commit();
     };
@@ -1666,7 +1778,7 @@ __global__ void __launch_bounds__(HADC_NT, 2)
       if (i < G) gather(i, tab[(i % 26) * ld + k]);
       else cp_async_commit();
     }
-    int idxn = HADC_D < G ? tab[(HADC_D % 26) * ld + k] : -1;
+    uint32_t idxn = HADC_D < G ? tab[(HADC_D % 26) * ld + k] : SPLIT_NONE;
     for (int gi = 0; gi < G && ok; gi++) {
       const int s = gi % HADC_S;
       if (gi + HADC_D < G) gather(gi + HADC_D, idxn);
@@ -1675,10 +1787,16 @@ __global__ void __launch_bounds__(HADC_NT, 2)
       cp_async_wait<HADC_D>();  // position gi's group has landed
       float4 x[4];
       {
-        const float4* sl = reinterpret_cast<const float4*>(smem_raw + HADC_BBYTES + (size_t)(gi % HADC_R) * (128 * 64)) +
+        const uint32_t entg = tab[(gi % 26) * ld + k];
+        const uint4* sl = reinterpret_cast<const uint4*>(smem_raw + HADC_BBYTES + (size_t)(gi % HADC_R) * (128 * 64)) +
                            (wid * 4) * 32 + lane;
 #pragma unroll
-        for (int i = 0; i < 4; i++) x[i] = sl[i * 32];
+        for (int i = 0; i < 4; i++) {  // head + tail, exponent undone: children 2 q and 2 q + 1
+          const uint4 v = sl[i * 32];
+          const float sc = split_inv(__shfl_sync(0xffffffffu, entg, g + 8 * i));
+          const float2 h0 = h2_float2(v.x), t0 = h2_float2(v.y), h1 = h2_float2(v.z), t1 = h2_float2(v.w);
+          x[i] = make_float4((h0.x + t0.x) * sc, (h0.y + t0.y) * sc, (h1.x + t1.x) * sc, (h1.y + t1.y) * sc);
+        }
       }
       if (gi >= HADC_S) {  // the stage's previous position is done: take its products, then reuse it
         ok = hadc_wait(done0 + 8 * s, ((gi - HADC_S) / HADC_S) & 1);
@@ -1765,6 +1883,40 @@ size_t ft_fwd_smem(int p) {  // k_m2l_bwd's shared memory: [CPB][p][n1][H] + [CP
 template <class R>
 size_t ft_bwd_smem(int p) { return ft_fwd_smem<R>(p); }
 
+// Spectrum values as the forward transforms store them and the Hadamard reads them: split FP16 pairs (mixed),
+// double2 (FP64).
+template <class R> struct Spec;
+template <> struct Spec<float> {
+  using type = SplitC;
+  static __device__ __forceinline__ type make(float2 v, float scale) { return split16(v.x * scale, v.y * scale); }
+};
+template <> struct Spec<double> {
+  using type = double2;
+  static __device__ __forceinline__ type make(double2 v, float) { return v; }
+};
+__device__ __forceinline__ float abs1(float v) { return fabsf(v); }
+__device__ __forceinline__ float abs1(float2 v) { return fabsf(v.x) + fabsf(v.y); }
+// The scale of source node s (children at node0 .. node0 + 7): every spectrum value of a child is at most
+// the sum of its densities' magnitudes.  One warp per child; red: 8 floats of shared memory.  Called by a
+// whole CTA of 256 threads; writes the source's exponent code for k_pack_sources.
+template <class W>
+__device__ __forceinline__ float source_scale(const W* __restrict__ up, int64_t node0, int nsurf, float* red,
+                                              int* __restrict__ scode) {
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const W* u = up + (node0 + wid) * nsurf;
+  float m = 0.f;
+  for (int k = lane; k < nsurf; k += 32) m += abs1(__ldg(u + k));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m += __shfl_xor_sync(0xffffffffu, m, o);
+  if (lane == 0) red[wid] = m;
+  __syncthreads();
+  float b = red[0];
+#pragma unroll
+  for (int c = 1; c < 8; c++) b = fmaxf(b, red[c]);
+  const int code = split_code(b);
+  if (threadIdx.x == 0) *scode = code;
+  return split_scale(code);
+}
 template <class CT>
 __device__ __forceinline__ CT ft_mul(CT a, CT b) {
   return CT{a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x};
@@ -1776,6 +1928,33 @@ __device__ __forceinline__ void ft_load_w(const double* __restrict__ tw, double 
   for (int m = 0; m < N; m++) {
     w[m].x = (decltype(w[m].x))tw[2 * m];
     w[m].y = (decltype(w[m].x))(sign * tw[2 * m + 1]);
+  }
+}
+
+// The cuFFT path (orders beyond the DFT kernels): each source's exponent code ...
+template <class W>
+__global__ void __launch_bounds__(256)
+    k_source_codes(const int* __restrict__ src, const int* __restrict__ child0, const W* __restrict__ up, int nsurf,
+                   int* __restrict__ scode) {
+  __shared__ float red[8];
+  source_scale(up, (int64_t)child0[src[blockIdx.x]], nsurf, red, scode + blockIdx.x);
+}
+// ... and its spectra, rows (source, child) x nfreq, into the split layout [f][source][child]
+__global__ void k_transpose_split(const float2* __restrict__ in, SplitC* __restrict__ out, int ns, int nfreq,
+                                  const int* __restrict__ scode) {
+  __shared__ float2 tile[32][33];
+  const int64_t r0 = (int64_t)blockIdx.y * 32, c0 = (int64_t)blockIdx.x * 32, nr = (int64_t)ns * 8;
+  for (int i = threadIdx.y; i < 32; i += 8) {
+    const int64_t r = r0 + i, c = c0 + threadIdx.x;
+    if (r < nr && c < nfreq) tile[i][threadIdx.x] = in[r * nfreq + c];
+  }
+  __syncthreads();
+  for (int i = threadIdx.y; i < 32; i += 8) {
+    const int64_t c = c0 + i, r = r0 + threadIdx.x;
+    if (r >= nr || c >= nfreq) continue;
+    const float sc = split_scale(scode[r >> 3]);
+    const float2 v = tile[threadIdx.x][i];
+    out[c * nr + r] = split16(v.x * sc, v.y * sc);
   }
 }
 
@@ -1952,7 +2131,7 @@ template <class R, int P>
 __global__ void __launch_bounds__(FT_NT, FtcFwdMinB<R>::v)
     k_m2l_fwd_c(const int* __restrict__ src, int ns, const int* __restrict__ child0,
                 const typename C2<R>::type* __restrict__ up, int nsurf, const int* __restrict__ conv2surf,
-                const double* __restrict__ tw, typename C2<R>::type* __restrict__ spec) {
+                const double* __restrict__ tw, typename Spec<R>::type* __restrict__ spec, int* __restrict__ scode) {
   using CT = typename C2<R>::type;
   constexpr int N = 2 * P, CPB = FtcCpb<R>::v, KS = 2 * FTC_JS;
   const int s = blockIdx.x, ch0 = blockIdx.y * CPB, tid = threadIdx.x;
@@ -1967,6 +2146,11 @@ __global__ void __launch_bounds__(FT_NT, FtcFwdMinB<R>::v)
     sidx[e] = conv2surf[(c * N + b) * N + a];
   }
   const int64_t node0 = (int64_t)child0[src[s]] + ch0;
+  float sc = 1.f;  // the node's power-of-two scale
+  if constexpr (sizeof(R) == 4) {
+    __shared__ float red[8];
+    sc = source_scale(up, node0, nsurf, red, scode + s);
+  }
   const int64_t fstride = (int64_t)N * N * ns * 8;
   for (int j0 = 0; j0 < P; j0 += FTC_JS) {
     __syncthreads();  // sidx and sw ready; the previous slab's sA / sB reads done
@@ -2011,8 +2195,8 @@ __global__ void __launch_bounds__(FT_NT, FtcFwdMinB<R>::v)
       CT x[P];
 #pragma unroll
       for (int c = 0; c < P; c++) x[c] = sB[((c * N + kb) * CPB + ch) * KS + sl];
-      CT* o = spec + ((int64_t)(kb * N + ka) * ns + s) * 8 + ch0 + ch;
-      ftc_dft_p<P>(x, sw, [&](int kc, CT v) { o[kc * fstride] = v; });
+      auto* o = spec + ((int64_t)(kb * N + ka) * ns + s) * 8 + ch0 + ch;
+      ftc_dft_p<P>(x, sw, [&](int kc, CT v) { o[kc * fstride] = Spec<R>::make(v, sc); });
     }
   }
 }
@@ -2146,7 +2330,7 @@ template <class R, int P>
 __global__ void __launch_bounds__(FT_NT, FtrMinB<R>::v)
     k_m2l_fwd_r(const int* __restrict__ src, int ns, const int* __restrict__ child0, const R* __restrict__ up,
                 int nsurf, const int* __restrict__ conv2surf, const double* __restrict__ tw,
-                typename C2<R>::type* __restrict__ spec) {
+                typename Spec<R>::type* __restrict__ spec, int* __restrict__ scode) {
   using CT = typename C2<R>::type;
   constexpr int N = 2 * P, H = P + 1, CPB = FtCpb<R>::v, KS = FTR_KS;
   const int s = blockIdx.x, ch0 = blockIdx.y * CPB, tid = threadIdx.x;
@@ -2161,6 +2345,11 @@ __global__ void __launch_bounds__(FT_NT, FtrMinB<R>::v)
     sidx[e] = conv2surf[(c * N + b) * N + a];
   }
   const int64_t node0 = (int64_t)child0[src[s]] + ch0;
+  float sc = 1.f;  // the node's power-of-two scale
+  if constexpr (sizeof(R) == 4) {
+    __shared__ float red[8];
+    sc = source_scale(up, node0, nsurf, red, scode + s);
+  }
   const int64_t fstride = (int64_t)N * H * ns * 8;  // kc -> kc + 1
   for (int k0 = 0; k0 < H; k0 += KS) {
     __syncthreads();  // sidx and sw ready; the previous slab's reads done
@@ -2207,8 +2396,8 @@ __global__ void __launch_bounds__(FT_NT, FtrMinB<R>::v)
       CT x[P];
 #pragma unroll
       for (int c = 0; c < P; c++) x[c] = sB[((c * N + kb) * CPB + ch) * KS + sl];
-      CT* o = spec + ((int64_t)(kb * H + ka) * ns + s) * 8 + ch0 + ch;
-      ftc_dft_p<P>(x, sw, [&](int kc, CT v) { o[kc * fstride] = v; });
+      auto* o = spec + ((int64_t)(kb * H + ka) * ns + s) * 8 + ch0 + ch;
+      ftc_dft_p<P>(x, sw, [&](int kc, CT v) { o[kc * fstride] = Spec<R>::make(v, sc); });
     }
   }
 }
@@ -2368,16 +2557,22 @@ struct Workspace {
   std::vector<cufftHandle> fwd, bwd;
   // Hadamard tiling: per group, tiles of TT targets; CSR over (tile, ipos) of (local target, source)
   std::vector<int> had_tile0;  // first tile of each group (ngroups + 1)
-  // FP32: sparse targets in the round form (per tile the range of rounds and HADR_TT output rows; per
-  // round its relative position and HADR_RW pairs), dense targets in the dense form (per group a
-  // [26][ld] source table and ld output rows)
-  DBuf<int> hadr_tile, hadr_pos, hadr_row;
-  DBuf<int2> hadr_ent;
+  // mixed path: tiles of k_hadamard_h (per group [had_tile0[g], had_tile0[g + 1])), their source slots,
+  // tables and output rows; scode: every source's exponent code of the last forward transform (one group at
+  // a time)
+  DBuf<HadTile> hadh_tile;
+  DBuf<int> hadh_slots, hadh_rows, scode;
+  DBuf<uint32_t> hadh_pslots;  // k_tile_codes
+  DBuf<float> hadh_tinv;
+  DBuf<uint2> hadh_tab;
+  // FP64, and the dense targets of the tcgen05 form: per group a [26][ld] source table and ld output rows
+  // (hadd_tabp: the table packed with the exponent codes)
   DBuf<int> hadd_tab, hadd_row;
+  DBuf<uint32_t> hadd_tabp;
   std::vector<int64_t> hadd_tab0, hadd_row0;
   std::vector<int> hadd_ld;
-  bool hadt_attr = false, hadrt_attr = false, hadc_attr = false, had64_attr = false;
-  // dense Hadamard targets on tcgen05 (k_hadamard_dc) instead of mma.sync (k_hadamard_dt): chosen when the
+  bool hadh_attr = false, hadc_attr = false, had64_attr = false;
+  // dense Hadamard targets on tcgen05 (k_hadamard_dc) instead of mma.sync (k_hadamard_h): chosen when the
   // workspace is created, by XFMM_HADAMARD_TCGEN05=1 in the environment
   bool had_tc5 = false;
   DBuf<unsigned char> hadc_btab;      // its B blocks per frequency (k_hadc_btab), built for one operator table
@@ -2523,6 +2718,10 @@ Workspace& workspace(Fmm& f, Tree& t, cudaStream_t s) {
   }
   W.specA.alloc((size_t)maxn * 8 * f.nfreq * 2 * rsz);
   W.specB.alloc((size_t)maxn * 8 * f.nfreq * 2 * rsz);
+  if (f.mixed()) {
+    XREQUIRE(maxn < (int)SPLIT_ROW_MASK, XFMM_ERR_UNSUPPORTED, "too many M2L sources");
+    W.scode.alloc(maxn);
+  }
   int dims[3] = {f.n1, f.n1, f.n1};
   cufftType tf = cplx ? (f.mixed() ? CUFFT_C2C : CUFFT_Z2Z) : (f.mixed() ? CUFFT_R2C : CUFFT_D2Z);
   cufftType tb = cplx ? (f.mixed() ? CUFFT_C2C : CUFFT_Z2Z) : (f.mixed() ? CUFFT_C2R : CUFFT_Z2D);
@@ -2542,38 +2741,40 @@ Workspace& workspace(Fmm& f, Tree& t, cudaStream_t s) {
     W.bwd.push_back(hb);
   }
   if (f.mixed()) {
-    // Targets with at least HAD_DENSE_MIN occupied positions go to the dense form, in tiles of HADT_TT
-    // (table [26][ld], padded with -1).  The others go to the round form: tiles of HADR_TT targets;
-    // per tile and relative position the pairs (source index, output row) in rounds
-    // of HADR_RW, padded with source -1.  Both write disjoint rows of the group's output.
-    std::vector<int> tile_r, pos, srow, dtab, drow;
-    std::vector<int2> ent;
+    // Tiles of k_hadamard_h over the targets of each group, level by level (node order within a level is
+    // Morton order: the targets of a tile are spatially compact and share most of their sources).  A tile
+    // closes at HADH_TT targets or when a class of its source slots (the octant of the source in its
+    // parent) is full.  In the tcgen05 mode the dense targets go to its table instead.
+    std::vector<HadTile> tiles;
+    std::vector<int> slots, rows, dtab, drow;
+    std::vector<uint2> tab;
     W.had_tile0.assign(ng + 1, 0);
     W.hadd_tab0.assign(ng, 0);
     W.hadd_row0.assign(ng, 0);
     W.hadd_ld.assign(ng, 0);
-    int ntiles = 0;
+    const std::vector<int> oct = t.octant.download(s, (size_t)t.nnodes);
+    const std::vector<int> msrc = t.m2l_src.download(s, (size_t)t.n_m2l_src);
+    std::vector<int> slot_of(maxn, -1), used;  // slot of each source in the open tile; its sources
+    std::vector<uint32_t> ent(26 * (size_t)HADH_TT);
     for (int g = 0; g < ng; g++) {
-      W.had_tile0[g] = ntiles;
+      W.had_tile0[g] = (int)tiles.size();
       const int tb = t.m2l_trg_off[g], te = t.m2l_trg_off[g + 1];
-      std::vector<int> dense, sparse;
+      const int* snode = msrc.data() + t.m2l_src_off[g];
+      std::vector<int> dense, rest;
       for (int tt = tb; tt < te; tt++) {
         int cnt = 0;
         for (int ipos = 0; ipos < 26; ipos++) cnt += t.h_m2l_tab[26 * (size_t)tt + ipos] >= 0;
-        (cnt >= HAD_DENSE_MIN ? dense : sparse).push_back(tt);
+        (W.had_tc5 && cnt >= HAD_DENSE_MIN ? dense : rest).push_back(tt);
       }
-      // a group with few dense targets would leave most rows of the dense form's tiles (HADT_TT targets,
-      // one tile per frequency) empty; the round form packs its pairs into full rounds instead
       if ((int)dense.size() < HAD_DENSE_GROUP_MIN) {
-        sparse.insert(sparse.end(), dense.begin(), dense.end());
-        std::sort(sparse.begin(), sparse.end());
+        rest.insert(rest.end(), dense.begin(), dense.end());
+        std::sort(rest.begin(), rest.end());
         dense.clear();
       }
-      // dense targets level by level (node order within a level is Morton order): the targets of one
-      // tile are then spatially compact and share most of their sources in L2
-      std::stable_sort(dense.begin(), dense.end(),
-                       [&](int a, int b) { return t.h_level[t.h_m2l_trg[a]] < t.h_level[t.h_m2l_trg[b]]; });
-      const int ld = (int)((dense.size() + HADT_TT - 1) / HADT_TT) * HADT_TT;
+      auto by_level = [&](int a, int b) { return t.h_level[t.h_m2l_trg[a]] < t.h_level[t.h_m2l_trg[b]]; };
+      std::stable_sort(dense.begin(), dense.end(), by_level);
+      std::stable_sort(rest.begin(), rest.end(), by_level);
+      const int ld = (int)((dense.size() + HADC_TT - 1) / HADC_TT) * HADC_TT;
       W.hadd_ld[g] = ld;
       W.hadd_tab0[g] = (int64_t)dtab.size();
       W.hadd_row0[g] = (int64_t)drow.size();
@@ -2585,40 +2786,87 @@ Workspace& workspace(Fmm& f, Tree& t, cudaStream_t s) {
         for (int ipos = 0; ipos < 26; ipos++)
           dtab[W.hadd_tab0[g] + (size_t)ipos * ld + k] = t.h_m2l_tab[26 * (size_t)tt + ipos];
       }
-      for (size_t k0 = 0; k0 < sparse.size(); k0 += HADR_TT, ntiles++) {
-        tile_r.push_back((int)pos.size());
-        const size_t k1 = std::min(sparse.size(), k0 + HADR_TT);
-        for (size_t k = k0; k < k0 + HADR_TT; k++) srow.push_back(k < k1 ? sparse[k] - tb : -1);
-        for (int ipos = 0; ipos < 26; ipos++) {
-          int n = 0;
-          for (size_t k = k0; k < k1; k++) {
-            const int sidx = t.h_m2l_tab[26 * (size_t)sparse[k] + ipos];
-            if (sidx < 0) continue;
-            if (n == 0) {
-              pos.push_back(ipos);
-              ent.resize(ent.size() + HADR_RW, make_int2(-1, 0));
+      for (size_t k0 = 0; k0 < rest.size();) {
+        int fill[8] = {1, 1, 1, 1, 1, 1, 1, 1};  // slots 0 .. 7 are the zeros
+        size_t k1 = k0;
+        for (; k1 < rest.size() && k1 - k0 < (size_t)HADH_TT; k1++) {
+          const int* src = t.h_m2l_tab.data() + 26 * (size_t)rest[k1];
+          int need[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+          bool fits = true;
+          for (int ipos = 0; ipos < 26; ipos++)
+            if (src[ipos] >= 0 && slot_of[src[ipos]] < 0) {
+              const int c = oct[snode[src[ipos]]] & 7;
+              if (fill[c] + ++need[c] > HADH_SLOTS / 8) fits = false;
             }
-            ent[ent.size() - HADR_RW + n] = make_int2(sidx, sparse[k] - tb);  // source, output row
-            if (++n == HADR_RW) n = 0;
-          }
+          if (!fits) break;
+          for (int ipos = 0; ipos < 26; ipos++)
+            if (src[ipos] >= 0 && slot_of[src[ipos]] < 0) {
+              const int c = oct[snode[src[ipos]]] & 7;
+              slot_of[src[ipos]] = 8 * fill[c]++ + c;
+              used.push_back(src[ipos]);
+            }
         }
+        HadTile T;
+        T.nslots = 8 * *std::max_element(fill, fill + 8);
+        const int nt = (int)(k1 - k0);
+        T.groups = (nt + 63) / 64;
+        while ((HADH_NT / 32) % T.groups) T.groups++;
+        T.slot0 = (int)slots.size();
+        T.row0 = (int)rows.size();
+        T.tab0 = (int64_t)tab.size();
+        slots.resize(slots.size() + T.nslots, -1);
+        for (int src : used) slots[T.slot0 + slot_of[src]] = src;
+        for (int k = 0; k < 64 * T.groups; k++) rows.push_back(k < nt ? rest[k0 + k] - tb : -1);
+        // per position the slot of every target; empty rows of a fragment's 8 take zero slots off the
+        // others' banks
+        for (int ipos = 0; ipos < 26; ipos++)
+          for (int k = 0; k < 64 * T.groups; k += 8) {
+            uint32_t classes = 0;
+            int sl[8];
+            for (int i = 0; i < 8; i++) {
+              const int src = k + i < nt ? t.h_m2l_tab[26 * (size_t)rest[k0 + k + i] + ipos] : -1;
+              sl[i] = src >= 0 ? slot_of[src] : -1;
+              if (src >= 0) classes |= 1u << (sl[i] & 7);
+            }
+            int c = 0;
+            for (int i = 0; i < 8; i++) {
+              if (sl[i] < 0) {
+                while (c < 7 && (classes >> c & 1)) c++;
+                sl[i] = c;
+                classes |= 1u << c;
+              }
+              ent[(size_t)ipos * HADH_TT + k + i] = hadh_entry(sl[i]);
+            }
+          }
+        tab.resize(tab.size() + (size_t)26 * T.groups * 32);
+        uint2* o = tab.data() + T.tab0;
+        for (int ipos = 0; ipos < 26; ipos++)
+          for (int gr = 0; gr < T.groups; gr++)
+            for (int ln = 0; ln < 32; ln++) {
+              const uint32_t* e = ent.data() + (size_t)ipos * HADH_TT + 64 * gr + (ln & 15);
+              *o++ = make_uint2(e[0] | e[16] << 16, e[32] | e[48] << 16);
+            }
+        tiles.push_back(T);
+        for (int src : used) slot_of[src] = -1;
+        used.clear();
+        k0 = k1;
       }
     }
-    W.had_tile0[ng] = ntiles;
-    tile_r.push_back((int)pos.size());
-    if (ent.empty()) {
-      pos.push_back(0);
-      ent.resize(HADR_RW, make_int2(-1, 0));
+    W.had_tile0[ng] = (int)tiles.size();
+    if (!tiles.empty()) {
+      W.hadh_tile.upload(tiles, s);
+      W.hadh_slots.upload(slots, s);
+      W.hadh_rows.upload(rows, s);
+      W.hadh_tab.upload(tab, s);
+      W.hadh_pslots.alloc(slots.size());
+      W.hadh_tinv.alloc(tiles.size());
     }
-    if (srow.empty()) srow.push_back(-1);
-    if (dtab.empty()) dtab.push_back(-1);
-    if (drow.empty()) drow.push_back(-1);
-    W.hadr_tile.upload(tile_r, s);
-    W.hadr_pos.upload(pos, s);
-    W.hadr_ent.upload(ent, s);
-    W.hadr_row.upload(srow, s);
-    W.hadd_tab.upload(dtab, s);
-    W.hadd_row.upload(drow, s);
+    if (!dtab.empty()) {
+      W.hadd_tab.upload(dtab, s);
+      W.hadd_row.upload(drow, s);
+      W.hadd_tabp.alloc(dtab.size());
+    }
+    XCUDA(cudaStreamSynchronize(s));  // the host tables are released here
   } else {
     // FP64: every target in the dense form on the FP64 tensor cores (k_hadamard_d64): per group a [26][ld]
     // source table and ld output rows, targets level by level (Morton order inside a level), padded to
@@ -2688,7 +2936,7 @@ void find_close_pairs(Workspace& ws, const NearArgs& na, int n_eval, cudaStream_
 }
 
 constexpr int DOWN_PRE = 1, DOWN_NEAR = 2, DOWN_FAR = 4, DOWN_ALL = 7;
-constexpr int M2L_FWD = 1, M2L_HAD_SPARSE = 2, M2L_HAD_DENSE = 4, M2L_BWD = 8, M2L_ALL = 15;
+constexpr int M2L_FWD = 1, M2L_HAD_TILES = 2, M2L_HAD_DENSE = 4, M2L_BWD = 8, M2L_ALL = 15;
 // parts of the downward pass before the near field: the M2L parts above (P2L with the forward transforms),
 // then L2L, then L2P's check-to-equivalent step
 constexpr int PRE_L2L = 16, PRE_DC2E = 32, PRE_ALL = M2L_ALL | PRE_L2L | PRE_DC2E;
@@ -2767,7 +3015,7 @@ struct Engine {
     XCUDA(cudaEventRecord(ws.ev[2], s));
   }
 
-  // phase: which parts of every group's M2L to run (M2L_FWD, M2L_HAD_SPARSE, M2L_HAD_DENSE, M2L_BWD)
+  // phase: which parts of every group's M2L to run (M2L_FWD, M2L_HAD_TILES, M2L_HAD_DENSE, M2L_BWD)
   static void m2l(Fmm& f, Tree& t, Workspace& ws, cudaStream_t s, int phase = M2L_ALL) {
     const int n = f.nsurf, nconv = f.nconv, nfreq = f.nfreq;
     const int ng = (int)t.m2l_src_off.size() - 1;
@@ -2778,7 +3026,8 @@ struct Engine {
       const int* src = t.m2l_src.p + t.m2l_src_off[g];
       const int* trg = t.m2l_trg.p + t.m2l_trg_off[g];
       const int tab_level = KER == K_LAPLACE ? 0 : g + 1;
-      const CT* T = (const CT*)f.ops[tab_level].m2l_T.p;
+      using SP = typename Spec<R>::type;
+      SP* spec = (SP*)ws.specB.p;
       if (phase & M2L_FWD) {
         XCUDA(cudaEventRecord(ev[0], s));
         // upward equivalent DFT (fmm_scale_invariant.h:560-604) -> specB [f][s][c]
@@ -2792,7 +3041,7 @@ struct Engine {
                 ws.ft_fwd_smem = smem;
               }
               k_m2l_fwd_r<R, PP><<<dim3(ns, 8 / FtCpb<R>::v), FT_NT, smem, s>>>(
-                  src, ns, t.child0.p, (const R*)ws.up.p, n, f.conv_to_surf_up.p, f.dft_tw.p, (CT*)ws.specB.p);
+                  src, ns, t.child0.p, (const R*)ws.up.p, n, f.conv_to_surf_up.p, f.dft_tw.p, spec, ws.scode.p);
             });
             XLAUNCH();
             ws.launches++;
@@ -2806,7 +3055,7 @@ struct Engine {
               ws.ft_fwd_smem = smem;
             }
             k_m2l_fwd_c<R, PP><<<dim3(ns, 8 / FtcCpb<R>::v), FT_NT, smem, s>>>(
-                src, ns, t.child0.p, (const CT*)ws.up.p, n, f.conv_to_surf_up.p, f.dft_tw.p, (CT*)ws.specB.p);
+                src, ns, t.child0.p, (const CT*)ws.up.p, n, f.conv_to_surf_up.p, f.dft_tw.p, spec, ws.scode.p);
           });
           XLAUNCH();
           ws.launches++;
@@ -2819,55 +3068,69 @@ struct Engine {
           XCUFFT2(cufftSetStream(ws.fwd[g], s));
           exec_fwd(ws.fwd[g], ws.grid.p, ws.specA.p);
           ws.launches++;
-          transpose<CT>((const CT*)ws.specA.p, (CT*)ws.specB.p, (int64_t)ns * 8, nfreq, s);  // -> [f][s][c]
+          if constexpr (sizeof(R) == 4) {  // -> [f][s][c], split
+            k_source_codes<W><<<ns, 256, 0, s>>>(src, t.child0.p, (const W*)ws.up.p, n, ws.scode.p);
+            XLAUNCH();
+            const dim3 grid((nfreq + 31) / 32, ((int64_t)ns * 8 + 31) / 32);
+            XREQUIRE(grid.y < 65536, XFMM_ERR_UNSUPPORTED, "transpose too tall");
+            k_transpose_split<<<grid, dim3(32, 8), 0, s>>>((const float2*)ws.specA.p, spec, ns, nfreq, ws.scode.p);
+            XLAUNCH();
+            ws.launches++;
+          } else {
+            transpose<CT>((const CT*)ws.specA.p, (CT*)ws.specB.p, (int64_t)ns * 8, nfreq, s);  // -> [f][s][c]
+          }
+        }
+        if (const int nht = ws.had_tile0[g + 1] - ws.had_tile0[g]; sizeof(R) == 4 && nht > 0) {
+          k_tile_codes<<<nht, 256, 0, s>>>(ws.hadh_tile.p + ws.had_tile0[g], ws.hadh_slots.p, ws.scode.p,
+                                           ws.hadh_pslots.p, ws.hadh_tinv.p + ws.had_tile0[g]);
+          XLAUNCH();
+          ws.launches++;
+        }
+        if (sizeof(R) == 4 && ws.hadd_ld[g] > 0) {  // the tcgen05 form's table
+          const int64_t nd = (int64_t)26 * ws.hadd_ld[g];
+          k_pack_sources<<<std::min<int64_t>(nblk(nd), 148 * 8), 256, 0, s>>>(
+              ws.hadd_tab.p + ws.hadd_tab0[g], nd, ws.scode.p, ws.hadd_tabp.p + ws.hadd_tab0[g]);
+          XLAUNCH();
+          ws.launches++;
         }
         XCUDA(cudaEventRecord(ev[1], s));
       }
-      if (phase & (M2L_HAD_SPARSE | M2L_HAD_DENSE)) {
+      if (phase & (M2L_HAD_TILES | M2L_HAD_DENSE)) {
         // Hadamard product
         const int ntiles = ws.had_tile0[g + 1] - ws.had_tile0[g];
         if constexpr (sizeof(CT) == 8) {
           XREQUIRE(nfreq < 65536, XFMM_ERR_UNSUPPORTED, "too many frequencies for the Hadamard grid");
-          if (ntiles > 0 && (phase & M2L_HAD_SPARSE)) {
-            const int* rows = ws.hadr_row.p + (int64_t)ws.had_tile0[g] * HADR_TT;
-            if (!ws.hadrt_attr) {
-              XCUDA(cudaFuncSetAttribute(k_hadamard_rt, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HADT_SMEM));
-              ws.hadrt_attr = true;
+          if (ntiles > 0 && (phase & M2L_HAD_TILES)) {
+            if (!ws.hadh_attr) {
+              XCUDA(cudaFuncSetAttribute(k_hadamard_h, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HADH_SMEM));
+              ws.hadh_attr = true;
             }
-            const int tpc = t.hadr_tpc > 0 ? t.hadr_tpc : HADR_TPC;
-            k_hadamard_rt<<<dim3((ntiles + tpc - 1) / tpc, nfreq), HADR_NT, HADT_SMEM, s>>>(
-                T, (const CT*)ws.specB.p, (CT*)ws.specA.p, ws.hadr_tile.p + ws.had_tile0[g], ws.hadr_pos.p,
-                ws.hadr_ent.p, rows, ntiles, tpc, ns, nt, nfreq);
+            const int tpc = t.hadr_tpc > 0 ? t.hadr_tpc : HADH_TPC;
+            const HadSys S = had_sys(ws, g, ns, nt);
+            const LevelOps& op = f.ops[tab_level];
+            k_hadamard_h<<<dim3((ntiles + tpc - 1) / tpc, nfreq), HADH_NT, HADH_SMEM, s>>>(
+                (const uint4*)op.m2l_frag.p, op.m2l_binv.p, S, ntiles, tpc);
             XLAUNCH();
             ws.launches++;
           }
-          if (ws.hadd_ld[g] > 0 && ws.had_tc5 && (phase & M2L_HAD_DENSE)) {
+          if (ws.hadd_ld[g] > 0 && (phase & M2L_HAD_DENSE)) {
             if (!ws.hadc_attr) {
               XCUDA(cudaFuncSetAttribute(k_hadamard_dc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HADC_SMEM));
               ws.hadc_attr = true;
             }
-            if (ws.hadc_btab_T != (const void*)T || ws.hadc_btab_nf != nfreq) {  // B blocks in the MMA layout
+            const LevelOps& op = f.ops[tab_level];
+            if (ws.hadc_btab_T != (const void*)op.m2l_frag.p || ws.hadc_btab_nf != nfreq) {  // B blocks in the MMA layout
               ws.hadc_btab.reserve((size_t)nfreq * HADC_BBYTES);
-              k_hadc_btab<<<std::min<int64_t>(nblk((int64_t)nfreq * 26 * 64), 148 * 16), 256, 0, s>>>(T, nfreq,
-                                                                                                    ws.hadc_btab.p);
+              k_hadc_btab<<<std::min<int64_t>(nblk((int64_t)nfreq * 26 * 64), 148 * 16), 256, 0, s>>>(
+                  (const uint4*)op.m2l_frag.p, op.m2l_binv.p, nfreq, ws.hadc_btab.p);
               XLAUNCH();
               ws.launches++;
-              ws.hadc_btab_T = T;
+              ws.hadc_btab_T = op.m2l_frag.p;
               ws.hadc_btab_nf = nfreq;
             }
             k_hadamard_dc<<<dim3(ws.hadd_ld[g] / 128, (nfreq + HADC_FPB - 1) / HADC_FPB), HADC_NT, HADC_SMEM, s>>>(
-                ws.hadc_btab.p, (const CT*)ws.specB.p, (CT*)ws.specA.p, ws.hadd_tab.p + ws.hadd_tab0[g], ws.hadd_ld[g],
+                ws.hadc_btab.p, spec, (CT*)ws.specA.p, ws.hadd_tabp.p + ws.hadd_tab0[g], ws.hadd_ld[g],
                 ws.hadd_row.p + ws.hadd_row0[g], ns, nt, nfreq, ws.status.p);
-            XLAUNCH();
-            ws.launches++;
-          } else if (ws.hadd_ld[g] > 0 && (phase & M2L_HAD_DENSE)) {
-            if (!ws.hadt_attr) {
-              XCUDA(cudaFuncSetAttribute(k_hadamard_dt, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HADT_SMEM));
-              ws.hadt_attr = true;
-            }
-            k_hadamard_dt<<<dim3((ws.hadd_ld[g] / HADT_TT + HADT_TPC - 1) / HADT_TPC, nfreq), HADT_NT, HADT_SMEM, s>>>(
-                T, (const CT*)ws.specB.p, (CT*)ws.specA.p, ws.hadd_tab.p + ws.hadd_tab0[g], ws.hadd_ld[g],
-                ws.hadd_row.p + ws.hadd_row0[g], ns, nt, nfreq);
             XLAUNCH();
             ws.launches++;
           }
@@ -2879,7 +3142,7 @@ struct Engine {
               ws.had64_attr = true;
             }
             k_hadamard_d64<<<dim3(ws.hadd_ld[g] / HAD64_TT, nfreq), HAD64_NT, HAD64_SMEM, s>>>(
-                T, (const CT*)ws.specB.p, (CT*)ws.specA.p, ws.hadd_tab.p + ws.hadd_tab0[g], ws.hadd_ld[g],
+                (const CT*)f.ops[tab_level].m2l_T.p, spec, (CT*)ws.specA.p, ws.hadd_tab.p + ws.hadd_tab0[g], ws.hadd_ld[g],
                 ws.hadd_row.p + ws.hadd_row0[g], ns, nt, nfreq);
             XLAUNCH();
             ws.launches++;
@@ -2964,6 +3227,14 @@ struct Engine {
       if (sizeof(R) == 4) XCUFFT2(cufftExecC2R(h, (cufftComplex*)in, (cufftReal*)out));
       else XCUFFT2(cufftExecZ2D(h, (cufftDoubleComplex*)in, (cufftDoubleReal*)out));
     }
+  }
+
+  // the tiles of group g of the mixed path's Hadamard
+  static HadSys had_sys(Workspace& ws, int g, int ns, int nt) {
+    return HadSys{(const SplitC*)ws.specB.p,           (float2*)ws.specA.p, ws.hadh_tile.p + ws.had_tile0[g],
+                  ws.hadh_pslots.p,                    ws.hadh_tinv.p + ws.had_tile0[g],
+                  ws.hadh_tab.p,                       ws.hadh_rows.p,      ns,
+                  nt};
   }
 
   // the far field (M2P + L2P evaluation), added to the near field's values
@@ -3118,6 +3389,13 @@ void check_ready(const Fmm& f, const Tree& t) {
 }  // namespace
 
 // ================================================================ public (internal API)
+void m2l_fragments(LevelOps& op, const double* T64, int nfreq, cudaStream_t s) {
+  op.m2l_frag.alloc((size_t)nfreq * HADH_FB * sizeof(uint4));
+  op.m2l_binv.alloc((size_t)nfreq * 32);
+  k_m2l_fragments<<<nblk(26ll * nfreq * 32), 256, 0, s>>>((const double2*)T64, nfreq, (uint4*)op.m2l_frag.p,
+                                                          op.m2l_binv.p);
+  XLAUNCH();
+}
 void set_charges(Fmm& f, Tree& t, const double* q, bool on_device, cudaStream_t s) {
   const int64_t n = t.nsrc;
   const int vs = f.is_complex() ? 2 : 1;
@@ -3229,10 +3507,10 @@ struct Batch {
   std::vector<cudaStream_t> streams;
   std::vector<cudaEvent_t> events;
   int near_ctas_per_sm = 0, near_tpl = 2;  // tuning (0: the kernel's resident limit)
-  // mixed Laplace systems sharing one operator table: the sparse M2L Hadamard of every system in one launch
+  // mixed Laplace systems sharing one operator table: the M2L Hadamard of every system in one launch
   bool had_batched = false;
-  const float2* had_T = nullptr;
-  int had_nfreq = 0, had_tpc = HADR_TPC, nhtiles = 0;
+  const LevelOps* had_op = nullptr;
+  int had_nfreq = 0, had_tpc = HADH_TPC, nhtiles = 0;
   DBuf<HadSys> hsys;
   DBuf<int2> htiles;
   // with the shared table also the M2M and L2L of every system, per level one GEMM over all systems' rows
@@ -3327,7 +3605,7 @@ Batch* batch_create(Fmm** fmms, Tree** trees, int n, cudaStream_t s) {
         off += ws.n_close;
       }
     }
-    // one operator table for every system (one Fmm), mixed Laplace (one M2L group): the sparse Hadamard
+    // one operator table for every system (one Fmm), mixed Laplace (one M2L group): the Hadamard
     // tiles of all systems as one list
     bool shared = b->kernel == XFMM_LAPLACE && b->precision == XFMM_MIXED;
     for (int k = 1; k < n && shared; k++) shared = fmms[k] == fmms[0];
@@ -3340,14 +3618,8 @@ Batch* batch_create(Fmm** fmms, Tree** trees, int n, cudaStream_t s) {
         HadSys& h = hs[k];
         h = HadSys{};
         if (t.n_m2l_trg == 0 || t.m2l_src_off.size() != 2) continue;
-        h.in = (const float2*)ws.specB.p;
-        h.out = (float2*)ws.specA.p;
-        h.tile_r = ws.hadr_tile.p + ws.had_tile0[0];
-        h.rpos = ws.hadr_pos.p;
-        h.ent = ws.hadr_ent.p;
-        h.rows = ws.hadr_row.p + (int64_t)ws.had_tile0[0] * HADR_TT;
-        h.nsrc = t.m2l_src_off[1] - t.m2l_src_off[0];
-        h.ntrg = t.m2l_trg_off[1] - t.m2l_trg_off[0];
+        h = Engine<K_LAPLACE, float>::had_sys(ws, 0, t.m2l_src_off[1] - t.m2l_src_off[0],
+                                              t.m2l_trg_off[1] - t.m2l_trg_off[0]);
         for (int j = 0; j < ws.had_tile0[1] - ws.had_tile0[0]; j++) tl.push_back(make_int2(k, j));
       }
       // per-level translations over all systems' rows: offsets rebased onto system 0's up / dn arrays (every
@@ -3438,13 +3710,13 @@ Batch* batch_create(Fmm** fmms, Tree** trees, int n, cudaStream_t s) {
       }
       b->bstatus = w0.status.p;
       b->had_batched = true;
-      b->had_T = (const float2*)fmms[0]->ops[0].m2l_T.p;
+      b->had_op = &fmms[0]->ops[0];
       b->had_nfreq = fmms[0]->nfreq;
       b->nhtiles = (int)tl.size();
       b->hsys.upload(hs, s);
       if (!tl.empty()) b->htiles.upload(tl, s);
       XREQUIRE(b->had_nfreq < 65536, XFMM_ERR_UNSUPPORTED, "too many frequencies for the Hadamard grid");
-      XCUDA(cudaFuncSetAttribute(k_hadamard_rt_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HADT_SMEM));
+      XCUDA(cudaFuncSetAttribute(k_hadamard_h_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HADH_SMEM));
     }
     b->order.resize(n);
     for (int k = 0; k < n; k++) b->order[k] = k;
@@ -3481,7 +3753,7 @@ void batch_set_tuning(Batch* b, int option, int value) {
     b->near_tpl = value;
   } else if (option == XFMM_BATCH_HADAMARD_TILES_PER_CTA) {
     XREQUIRE(value >= 0 && value <= 64, XFMM_ERR_ARG, "Hadamard tiles per CTA must be 0..64");
-    b->had_tpc = value > 0 ? value : HADR_TPC;
+    b->had_tpc = value > 0 ? value : HADH_TPC;
   } else {
     XREQUIRE(false, XFMM_ERR_ARG, "unknown batch tuning option");
   }
@@ -3525,7 +3797,7 @@ void batch_evaluate(Batch* b, const double* const* charges, double* const* outs,
   };
   // before the near field: upward pass, P2L, M2L and L2L per system.  With one shared operator table (mixed
   // Laplace) the parts that share it run as one launch over all systems: the M2M and L2L of each level, and
-  // the sparse M2L Hadamard between the systems' forward and backward transforms.
+  // the M2L Hadamard between the systems' forward and backward transforms.
   const int E = nstreams + 1;
   Fmm& f0 = *b->fmm[0];
   auto per_system = [&](int evbase, int up_parts, int pre_parts, bool first) {
@@ -3574,8 +3846,8 @@ void batch_evaluate(Batch* b, const double* const* charges, double* const* outs,
     per_system(E, 0, M2L_FWD | M2L_HAD_DENSE, false);
     if (b->nhtiles > 0) {
       const int tpc = std::max(1, b->had_tpc);
-      k_hadamard_rt_batch<<<dim3((b->nhtiles + tpc - 1) / tpc, b->had_nfreq), HADR_NT, HADT_SMEM, s>>>(
-          b->had_T, b->hsys.p, b->htiles.p, b->nhtiles, tpc, b->had_nfreq);
+      k_hadamard_h_batch<<<dim3((b->nhtiles + tpc - 1) / tpc, b->had_nfreq), HADH_NT, HADH_SMEM, s>>>(
+          (const uint4*)b->had_op->m2l_frag.p, b->had_op->m2l_binv.p, b->hsys.p, b->htiles.p, b->nhtiles, tpc);
       XLAUNCH();
     }
     per_system(2 * E, 0, M2L_BWD, false);

@@ -586,9 +586,7 @@ void precompute(Fmm& f, int depth, cudaStream_t s) {
       LevelOps& op = f.ops[l];
       const int64_t cnt = 26ll * nfreq * 64 * 2;
       if (single) {
-        op.m2l_T.alloc(cnt * sizeof(float));
-        k_to_single<<<nb(cnt), 256, 0, s>>>(T64.p, (float*)op.m2l_T.p, cnt);
-        XLAUNCH();
+        m2l_fragments(op, (const double*)T64.p, nfreq, s);
       } else {
         op.m2l_T.alloc(cnt * sizeof(double));
         XCUDA(cudaMemcpyAsync(op.m2l_T.p, T64.p, cnt * sizeof(double), cudaMemcpyDeviceToDevice, s));

@@ -148,7 +148,7 @@ struct Tree {
   // persistent staging for host-side charges and results (no allocation per call)
   DBuf<double> stage_q, stage_out;
   DBuf<int> stage_flag;               // non-finite charges found by the device-side check
-  int hadr_tpc = 0;                   // sparse M2L Hadamard: tiles per CTA (0: the built-in default)
+  int hadr_tpc = 0;                   // M2L Hadamard, mixed path: target tiles per CTA (0: the built-in default)
 };
 
 // Precomputed operators of one level (or the single scale-invariant level).
@@ -164,7 +164,11 @@ struct LevelOps {
   DBuf<char> l2p_B1f;  // FP32 copy of l2p_B1 (mixed path, real kernels: the L2P first factor runs in FP32)
   DBuf<char> m2m_B;    // [8n][n]     B[c*n+k][j] = M2M[c][j][k], M2M[c] = (V S+)(U^H K_c)
   DBuf<char> l2l_B;    // [n][8n]     B[k][c*n+j] = M2M[c][k][j] (L2L = M2M^T)
-  DBuf<char> m2l_T;    // [26][nfreq][64] complex: entry [s*8+t] (fmm_scale_invariant.h:549-551)
+  // M2L tables, entry [s*8+t] of [26][nfreq][64] complex (fmm_scale_invariant.h:549-551): FP64, or for the
+  // mixed path the Hadamard's FP16 head/tail fragments per frequency (m2l_fragments)
+  DBuf<char> m2l_T;
+  DBuf<char> m2l_frag;
+  DBuf<float> m2l_binv;  // mixed: [nfreq][32], undoes the exponent of each block
   int rank = 0;        // singular values kept by the pinv threshold: B1 columns / B2 rows beyond are zero
   // the same operators in the form the translation GEMMs (translate.cu) read: real [K][N] row-major, a
   // complex operator expanded to [2K][2N] (expand_operator); FP64 for the pinv factors and the FP64
@@ -204,6 +208,7 @@ void m2l_setup(Fmm& fmm, Tree& t, cudaStream_t s);
 void precompute(Fmm& fmm, int depth, cudaStream_t s);
 void host_surface_base(int p, std::vector<double>& out);
 // evaluate.cu
+void m2l_fragments(LevelOps& op, const double* T64, int nfreq, cudaStream_t s);
 void set_charges(Fmm& fmm, Tree& t, const double* q, bool on_device, cudaStream_t s);
 void clear_values(Fmm& fmm, Tree& t, cudaStream_t s);
 void upward_pass(Fmm& fmm, Tree& t, cudaStream_t s);

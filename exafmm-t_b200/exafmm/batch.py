@@ -6,7 +6,7 @@ share one Fmm object: its scale-invariant operators, precomputed once for the fi
 serve every other radius (the evaluate scales the body-to-check potentials by the ratio of the radii);
 the other kernels' operators depend on the radius, so each of those systems gets its own Fmm object.
 With one shared operator table (mixed Laplace) the work that shares it is one launch over all systems:
-the pseudo-inverse factors of P2M and L2P, the M2M and L2L of each level, the sparse M2L Hadamard between
+the pseudo-inverse factors of P2M and L2P, the M2M and L2L of each level, the M2L Hadamard between
 the systems' forward and backward M2L transforms, and the far field.  The systems are held by one native batch (xfmm_batch_*):
 one evaluate of every system runs each system's stages before and after its near field on concurrent
 streams forked from the batch stream (largest systems first, each to the least-loaded stream), and the
@@ -20,7 +20,7 @@ which in turn waits for it: results may be read on the current stream.
 
 ``autotune()`` captures the graph for each candidate stream count and each candidate tile shape of the
 persistent near-field kernel (CTAs per SM; targets per lane, the height of a warp's target tile), times
-replays on the device and keeps the fastest; then, with those, it does the same for the sparse M2L
+replays on the device and keeps the fastest; then, with those, it does the same for the M2L
 Hadamard's target tiles per CTA (set on every tree through xfmm_set_tuning).
 """
 import ctypes
@@ -69,7 +69,7 @@ class BatchedFmm:
         self.nstreams = 1
         self.near_ctas_per_sm, self.near_tpl = 0, 2  # persistent near field (0: as many CTAs as fit)
         self.tuning = {}        # (streams, CTAs per SM, targets per lane) -> ms per replay
-        self.tiles_per_cta = 0  # sparse Hadamard tiles per CTA on every tree (0: the library default)
+        self.tiles_per_cta = 0  # Hadamard tiles per CTA on every tree (0: the library default)
         self.tile_tuning = {}   # tiles per CTA -> ms per replay, with the chosen shape
 
     @property
@@ -146,7 +146,7 @@ class BatchedFmm:
         return e0.elapsed_time(e1) / reps
 
     def set_tiles_per_cta(self, value):
-        """Sparse M2L Hadamard tiles per CTA (0: the library default) of the batch's one-launch Hadamard
+        """M2L Hadamard tiles per CTA (0: the library default) of the batch's one-launch Hadamard
         (systems sharing one operator set) and of every tree's own; recapture after."""
         for tree in self.trees:
             tree.set_tuning("sparse_hadamard_tiles_per_cta", value)
@@ -157,7 +157,7 @@ class BatchedFmm:
                  tile_candidates=(1, 2, 4, 8)):
         """Capture the graph for each stream count in candidates and each persistent near-field shape
         (CTAs per SM, targets per lane) in near_shapes, time `reps` replays of each on the device (after
-        one untimed replay) and keep the fastest; then, with those, the same for each sparse-Hadamard
+        one untimed replay) and keep the fastest; then, with those, the same for each Hadamard
         tiles-per-CTA value in tile_candidates.  self.tuning maps each (streams, CTAs per SM, targets per
         lane), self.tile_tuning each tile value, to its milliseconds per replay."""
         best = None

@@ -128,8 +128,8 @@ xfmm_status xfmm_stage_times(xfmm_fmm* fmm, xfmm_tree* tree, double* ms14);
 
 /* Tuning options of a tree's evaluate (xfmm_set_tuning). */
 enum {
-  /* mixed path, sparse M2L Hadamard (k_hadamard_rt): target tiles of 512 covered by one CTA, which
-   * builds the frequency's operator fragments once for all of them; 1..64, 0 restores the default (4) */
+  /* mixed path, M2L Hadamard (k_hadamard_h): target tiles (of up to 512) covered by one CTA, which
+   * brings the frequency's operator fragments in once for all of them; 1..64, 0 restores the default (1) */
   XFMM_TUNE_SPARSE_HADAMARD_TILES_PER_CTA = 1
 };
 /* Sets a tuning option for the later evaluates of this tree; results change only within the mixed
@@ -149,7 +149,7 @@ xfmm_status xfmm_set_tuning(xfmm_tree* tree, int option, int value);
  * and the exact close-pair corrections of all systems one more launch.  When every system uses the same
  * xfmm_fmm handle, mixed Laplace with one scale-invariant operator set, the work that shares the operators
  * is one launch over all systems too: the pseudo-inverse factors of P2M and L2P, the M2M and the L2L of
- * each level, the sparse M2L Hadamard between the systems' forward and backward M2L transforms, and the
+ * each level, the M2L Hadamard between the systems' forward and backward M2L transforms, and the
  * far field (a persistent kernel over (system, leaf) items).  Asynchronous on `stream`, no
  * allocation: it may be captured into a CUDA graph (after one evaluate outside the capture). */
 typedef struct xfmm_batch xfmm_batch;
@@ -158,8 +158,8 @@ enum {
   XFMM_BATCH_NEAR_CTAS_PER_SM = 1,
   /* persistent near field: most targets a lane holds, the height of a warp's target tile (1 or 2) */
   XFMM_BATCH_NEAR_TARGETS_PER_LANE = 2,
-  /* one-launch sparse M2L Hadamard of mixed Laplace systems sharing one xfmm_fmm: 512-target tiles per CTA,
-   * which share one operator fill per frequency and may belong to different systems (1..64; 0: 4) */
+  /* one-launch M2L Hadamard of mixed Laplace systems sharing one xfmm_fmm: tiles (of up to 512 targets) per
+   * CTA, which share one operator fill per frequency and may belong to different systems (1..64; 0: 1) */
   XFMM_BATCH_HADAMARD_TILES_PER_CTA = 3
 };
 xfmm_status xfmm_batch_create(xfmm_fmm* const* fmms, xfmm_tree* const* trees, int n, void* stream, xfmm_batch** out);
