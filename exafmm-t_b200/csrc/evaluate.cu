@@ -2541,7 +2541,7 @@ struct Workspace {
   int precision = -1, kernel = -1, p = 0;
   size_t vsz = 0;
   DBuf<char> up, dn, chk;  // working precision
-  DBuf<double> tc_scratch;  // FP64 sums of the split-K tensor-core translations (zero between uses)
+  DBuf<double> tc_scratch;  // tile counters and partial sums of the split-K translations
   DBuf<int4> close_pairs;   // Laplace mixed near field: the close pairs (k_close_scan), found once per tree
   int64_t n_close = -1;     // -1: not searched yet
   DBuf<char> ybuf, eq;     // FP64: pinv intermediate (rows of the kept singular directions), downward
@@ -2613,6 +2613,8 @@ void upload_rows(GemmRows& g, const std::vector<int64_t>& a, const std::vector<i
   g.c.upload(c, s);
   g.al64.upload(al, s);
 }
+
+inline const LevelOps& level_ops(const Fmm& f, int level) { return f.ops[f.kernel == XFMM_LAPLACE ? 0 : level]; }
 
 Workspace& workspace(Fmm& f, Tree& t, cudaStream_t s) {
   Workspace*& w = t.ws[f.precision];
@@ -2687,13 +2689,22 @@ Workspace& workspace(Fmm& f, Tree& t, cudaStream_t s) {
     upload_rows<double>(W.m2m[l], ma, mc, one, s);
     upload_rows<double>(W.l2l[l], la, lc, one, s);
   }
-  if (f.mixed()) {
-    // FP64 scratch of the split-K tensor-core M2M / L2L of the small levels, zeroed once
-    const int cw = cplx ? 2 : 1;
+  {
+    // scratch of the split-K translations (one at a time on the tree's stream), its counters zeroed once
+    const int cw = cplx ? 2 : 1, lap_rows = lap ? t.nleafs : 0;
     int64_t need = 0;
     for (int l = 0; l <= t.depth; l++) {
-      need = std::max(need, tgemm_tc_scratch(W.m2m[l].M, cw * n, cw * 8 * n, 1));
-      need = std::max(need, tgemm_tc_scratch(W.l2l[l].M, cw * 8 * n, cw * n, 1));
+      if (f.mixed()) {
+        need = std::max(need, tgemm_tc_scratch(W.m2m[l].M, cw * n, cw * 8 * n, 1));
+        need = std::max(need, tgemm_tc_scratch(W.l2l[l].M, cw * 8 * n, cw * n, 1));
+      } else {
+        need = std::max(need, tgemm_f64_scratch(W.m2m[l].M, cw * n, cw * 8 * n));
+        need = std::max(need, tgemm_f64_scratch(W.l2l[l].M, cw * 8 * n, cw * n));
+      }
+      // the pseudo-inverse factors (FP64 in both precisions), between n and the kept rank
+      const int m = lap ? lap_rows : W.leaf_level_off[l + 1] - W.leaf_level_off[l];
+      const int rk = cw * level_ops(f, l).rank;
+      need = std::max({need, tgemm_f64_scratch(m, rk, cw * n), tgemm_f64_scratch(m, cw * n, rk)});
     }
     if (need > 0) {
       W.tc_scratch.alloc((size_t)need);
@@ -2908,8 +2919,6 @@ Workspace& workspace(Fmm& f, Tree& t, cudaStream_t s) {
   return W;
 }
 
-inline const LevelOps& level_ops(const Fmm& f, int level) { return f.ops[f.kernel == XFMM_LAPLACE ? 0 : level]; }
-
 template <class RB> const RB* m2l_scale_of(const Tree& t);
 template <> const float* m2l_scale_of<float>(const Tree& t) { return t.m2l_scale.p; }
 template <> const double* m2l_scale_of<double>(const Tree& t) { return t.m2l_scale64.p; }
@@ -2951,6 +2960,10 @@ struct Engine {
   using CT = typename C2<R>::type;              // spectrum value
   static constexpr int CW = KER == K_HELMHOLTZ ? 2 : 1;  // reals per value
 
+  static void split_scratch(TGemm& g, Workspace& ws) {
+    g.scratch = ws.tc_scratch.p;
+    g.scratch_len = (int64_t)ws.tc_scratch.n;
+  }
   static void upward(Fmm& f, Tree& t, Workspace& ws, cudaStream_t s, int parts = UP_ALL) {
     const int n = f.nsurf;
     if (parts & UP_P2M) {
@@ -2984,9 +2997,11 @@ struct Engine {
           const LevelOps& op = level_ops(f, l);
           const int rk = op.rank;
           TGemm g1{m, CW * rk, CW * n, ws.p2m1.a.p + off, ws.p2m1.c.p + off, nullptr, (int64_t)CW * n, 0, (int64_t)CW * n};
+          split_scratch(g1, ws);
           tgemm_f64<R, double>(g1, (const R*)ws.chk.p, op.tg_p2m1.p, (double*)ws.ybuf.p, s);
           TGemm g2{m, CW * n, CW * rk, ws.p2m2.a.p + off, ws.p2m2.c.p + off, ws.p2m2.al64.p + off, (int64_t)CW * n, 0,
                    (int64_t)CW * n};
+          split_scratch(g2, ws);
           tgemm_f64<double, R>(g2, (const double*)ws.ybuf.p, op.tg_p2m2.p, (R*)ws.up.p, s);
           ws.launches += 2;
         }
@@ -3004,8 +3019,7 @@ struct Engine {
       // adds each child's contribution (fmm_scale_invariant.h:243-251)
       TGemm gm{g.M, CW * n, CW * 8 * n, g.a.p, g.c.p, nullptr, (int64_t)CW * n, 1, (int64_t)CW * n};
       gm.status = ws.status.p;
-      gm.scratch = ws.tc_scratch.p;
-      gm.scratch_len = (int64_t)ws.tc_scratch.n;
+      split_scratch(gm, ws);
       if constexpr (sizeof(R) == 4)
         tgemm_tc<float>(gm, (const float*)ws.up.p, op.tg_m2m_h.p, op.tg_m2m_l.p, op.ld_m2m, (float*)ws.up.p, s);
       else
@@ -3317,8 +3331,7 @@ struct Engine {
         const LevelOps& op = level_ops(f, l);
         TGemm gl{g.M, CW * 8 * n, CW * n, g.a.p, g.c.p, nullptr, (int64_t)CW * 8 * n, 1, (int64_t)CW * n};
         gl.status = ws.status.p;
-        gl.scratch = ws.tc_scratch.p;
-        gl.scratch_len = (int64_t)ws.tc_scratch.n;
+        split_scratch(gl, ws);
         if constexpr (sizeof(R) == 4)
           tgemm_tc<float>(gl, (const float*)ws.dn.p, op.tg_l2l_h.p, op.tg_l2l_l.p, op.ld_l2l, (float*)ws.dn.p, s);
         else
@@ -3346,11 +3359,13 @@ struct Engine {
         // densities feed only the leaf's own targets (measured: +0.5e-7 potential error at p = 8, +1e-7
         // at p = 10).
         g1.status = ws.status.p;
+        split_scratch(g1, ws);
         if constexpr (sizeof(R) == 4 && KER != K_HELMHOLTZ)
           tgemm_tc<double>(g1, (const float*)ws.dn.p, op.tg_l2p1_h.p, op.tg_l2p1_l.p, op.ld_l2p1, (double*)ws.ybuf.p, s);
         else
           tgemm_f64<R, double>(g1, (const R*)ws.dn.p, op.tg_l2p1.p, (double*)ws.ybuf.p, s);
         TGemm g2{m, CW * n, CW * rk, ws.l2p2.a.p + off, ws.l2p2.c.p + off, nullptr, (int64_t)CW * n, 0, (int64_t)CW * n};
+        split_scratch(g2, ws);
         tgemm_f64<double, double>(g2, (const double*)ws.ybuf.p, op.tg_l2p2.p, (double*)ws.eq.p, s);
         ws.launches += 2;
       }

@@ -76,6 +76,30 @@ __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
                : "d"(a), "d"(b));
 }
 
+// ---------------------------------------------------------------- split K
+// A level with few row and column tiles leaves most of the chip idle, each of its CTAs walking all of K.  K is
+// then split over blockIdx.z and every part stores its sums into its place of a scratch; they are added in
+// order, so the result does not depend on the order of arrival.  FP64: the part that finishes last (a
+// counter per tile; no part waits for another) adds the tile's parts and writes the rows; the counters
+// stand at the front of the scratch and are zero between uses.  Tensor-core GEMM: a pass over the rows
+// (k_tc_finish), since its wider tiles take many parts (the last of up to 18 parts adding 128 x 64 sums
+// alone measured 0.71 ms for the M2M of a 300k Plummer set against 0.22 with FP64 atomics).
+constexpr int SPLIT_COUNTERS = 4096;  // tiles a split GEMM may have
+constexpr int64_t SPLIT_HEAD = SPLIT_COUNTERS * sizeof(unsigned) / sizeof(double);  // in doubles
+// this CTA's part is stored: true (in every thread) for the last of the tile's parts
+__device__ __forceinline__ bool split_last(unsigned* counter, unsigned parts, int* flag) {
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const bool last = atomicAdd(counter, 1u) == parts - 1;
+    if (last) *counter = 0u;
+    *flag = last;
+  }
+  __syncthreads();
+  __threadfence();
+  return *flag != 0;
+}
+
 // ---------------------------------------------------------------- FP64 (DMMA)
 // C[coff[r] + j] (=|+=) alpha[r] * sum_k A[aoff[r] + k] * B[k * ldb + j], r < M, j < N, k < K.
 // A row-major in shared memory ([BM][BK + 4], as TA), B k-major ([BK][BN + 4]), both filled by cp.async
@@ -91,16 +115,19 @@ template <class TA, class TC, int VA>
 __global__ void __launch_bounds__(TG_NT) k_tgemm_f64(int M, int N, int K, const TA* __restrict__ A,
                                                       const int64_t* __restrict__ aoff, const double* __restrict__ B,
                                                       int64_t ldb, const double* __restrict__ alpha, TC* __restrict__ C,
-                                                      const int64_t* __restrict__ coff, int acc) {
+                                                      const int64_t* __restrict__ coff, int acc,
+                                                      double* __restrict__ scratch) {
   extern __shared__ __align__(16) char tgd_sm[];
   TA* As = reinterpret_cast<TA*>(tgd_sm);
   double* Bs = reinterpret_cast<double*>(tgd_sm + (size_t)TGD_ST * TG_BM * TGD_LDA * sizeof(TA));
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, wm = w >> 1, wn = w & 1;
   const int g = lane >> 2, t = lane & 3;
   const int m0 = blockIdx.x * TG_BM, n0 = blockIdx.y * TG_BN;
-  const int nk = (K + TGD_BK - 1) / TGD_BK;
+  // this CTA's K steps
+  const int nks = (K + TGD_BK - 1) / TGD_BK, per = (nks + gridDim.z - 1) / gridDim.z;
+  const int kb = blockIdx.z * per, nk = max(0, min(nks, kb + per) - kb);
   auto load = [&](int slot, int kt) {
-    const int k0 = kt * TGD_BK;
+    const int k0 = (kb + kt) * TGD_BK;
     tile_async<VA, sizeof(TA)>(
         reinterpret_cast<char*>(As + (size_t)slot * TG_BM * TGD_LDA), TG_BM, TGD_BK, TGD_LDA,
         [&](int i) -> const char* {
@@ -148,6 +175,35 @@ __global__ void __launch_bounds__(TG_NT) k_tgemm_f64(int M, int N, int K, const 
     }
   }
   cp_wait<0>();
+  if (gridDim.z > 1) {
+    __shared__ int flag;
+    const int tile = blockIdx.y * gridDim.x + blockIdx.x, ntiles = gridDim.x * gridDim.y;
+    // element (i, j, h) of thread t of part z: [z][tile][(i, j, h)][t]
+    double* part = scratch + SPLIT_HEAD + threadIdx.x;
+    auto at = [&](int z, int i, int j, int h) -> double* {
+      return part + (((int64_t)z * ntiles + tile) * 32 + (i * 4 + j) * 2 + h) * TG_NT;
+    };
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+      if (m0 + 32 * wm + 8 * i < M)
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+#pragma unroll
+          for (int h = 0; h < 2; h++) *at(blockIdx.z, i, j, h) = c[i][j][h];
+    if (!split_last(reinterpret_cast<unsigned*>(scratch) + tile, gridDim.z, &flag)) return;
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+      for (int j = 0; j < 4; j++) c[i][j][0] = c[i][j][1] = 0.0;
+    for (int z = 0; z < (int)gridDim.z; z++)
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        if (m0 + 32 * wm + 8 * i < M)
+#pragma unroll
+          for (int j = 0; j < 4; j++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) c[i][j][h] += __ldcg(at(z, i, j, h));
+  }
 #pragma unroll
   for (int i = 0; i < 4; i++) {
     const int r = m0 + 32 * wm + 8 * i + g;
@@ -432,39 +488,41 @@ __global__ void __launch_bounds__(TC_NT, IP ? 3 : 2)
   __syncthreads();
   fence_after_sync();
   ok = abort_flag == 0;
-  if (!ok) {
-    if (tid == 0) atomicExch(status, 1);
-  } else if (nc > 0) {
+  if (!ok && tid == 0) atomicExch(status, 1);
+  if (gridDim.z > 1) {
+    // a part of a split K: its FP32 sums to [z][row][column], added by k_tc_finish
+    const int r = m0 + 32 * w + lane, ld = gridDim.y * TC_BN;
+    if (r < M) {
+      float4* o = reinterpret_cast<float4*>(reinterpret_cast<float*>(scratch) + ((int64_t)blockIdx.z * M + r) * ld + n0);
+#pragma unroll
+      for (int j = 0; j < TC_BN; j += 4) o[j / 4] = make_float4(run[j], run[j + 1], run[j + 2], run[j + 3]);
+    }
+  } else if (ok && nc > 0) {
     const int r = m0 + 32 * w + lane;
     if (r < M) {
       const double al = alpha ? alpha[r] : 1.0;
       TC* crow = C + coff[r] + n0;
-      if (gridDim.z > 1) {
-        // a part of a split K: added in FP64 into the scratch row r (k_tc_finish moves it into C)
-        double* srow = scratch + (int64_t)r * N + n0;
 #pragma unroll
-        for (int j = 0; j < TC_BN; j++)
-          if (n0 + j < N) atomicAdd(srow + j, al * (double)run[j]);
-      } else {
-#pragma unroll
-        for (int j = 0; j < TC_BN; j++)
-          if (n0 + j < N) store_out(crow + j, al * (double)run[j], acc);
-      }
+      for (int j = 0; j < TC_BN; j++)
+        if (n0 + j < N) store_out(crow + j, al * (double)run[j], acc);
     }
   }
   if (w == 0) tmem_dealloc(tm, 128);
 }
 
-// C[coff[r] + j] (=|+=) scratch[r][j] for the rows of a split-K tensor-core GEMM, scratch cleared for its
-// next use
+// C[coff[r] + j] (=|+=) alpha[r] * sum over the parts z of part[z][r][j], in FP64 and in order
 template <class TC>
-__global__ void k_tc_finish(int M, int N, double* __restrict__ scratch, TC* __restrict__ C,
-                            const int64_t* __restrict__ coff, int acc) {
+__global__ void k_tc_finish(int M, int N, int ld, int parts, const float* __restrict__ part,
+                            const double* __restrict__ alpha, TC* __restrict__ C, const int64_t* __restrict__ coff,
+                            int acc) {
   const int64_t total = (int64_t)M * N;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     const int r = (int)(e / N), j = (int)(e % N);
-    store_out(C + coff[r] + j, scratch[e], acc);
-    scratch[e] = 0.0;
+    const float* q = part + (int64_t)r * ld + j;
+    double v = 0.0;
+#pragma unroll 4
+    for (int z = 0; z < parts; z++) v += (double)__ldg(q + (int64_t)z * M * ld);
+    store_out(C + coff[r] + j, alpha ? alpha[r] * v : v, acc);
   }
 }
 
@@ -538,22 +596,53 @@ void expand_operator(const void* B, bool b_single, int K, int N, int64_t ldb, bo
   XLAUNCH();
 }
 
+// K parts of an FP64 GEMM: about two CTAs per SM, at least 4 steps of 16 each (a step is 0.55 us alone on an
+// SM).  Unsplit, the M2M of 1 .. 512 parents took 85 us per level at p = 8 however few they were: Laplace
+// 100k, p = 8: M2M 0.80 ms.
+static int tgd_parts(int M, int N, int K) {
+  const int tiles = ((M + TG_BM - 1) / TG_BM) * ((N + TG_BN - 1) / TG_BN), steps = (K + TGD_BK - 1) / TGD_BK;
+  if (M <= 0 || N <= 0 || tiles >= 148) return 1;
+  return std::max(1, std::min((2 * 148 + tiles - 1) / tiles, std::min(steps / 4, 32)));
+}
+int64_t tgemm_f64_scratch(int M, int N, int K) {
+  const int64_t tiles = (int64_t)((M + TG_BM - 1) / TG_BM) * ((N + TG_BN - 1) / TG_BN);
+  const int kz = tgd_parts(M, N, K);
+  return kz > 1 ? SPLIT_HEAD + kz * tiles * TG_BM * TG_BN : 0;
+}
 template <class TA, class TC>
 void tgemm_f64(const TGemm& g, const TA* A, const double* B, TC* C, cudaStream_t s) {
   if (g.M <= 0 || g.N <= 0) return;
   // B rows (ldb doubles) and A rows must start 8-byte aligned; 16-byte copies where they start 16-byte
   // aligned (A offsets multiples of astep elements)
   XREQUIRE(g.ldb % 2 == 0 && g.astep % 2 == 0, XFMM_ERR_UNSUPPORTED, "translation rows must be 16-byte aligned");
-  const dim3 grid((g.M + TG_BM - 1) / TG_BM, (g.N + TG_BN - 1) / TG_BN);
+  const int mt = (g.M + TG_BM - 1) / TG_BM, nt = (g.N + TG_BN - 1) / TG_BN;
+  // the scratch was sized for another rank, if the operators were computed again since: fewer parts then
+  const int64_t room = g.scratch ? (g.scratch_len - SPLIT_HEAD) / ((int64_t)mt * nt * TG_BM * TG_BN) : 0;
+  const int kz = (int)std::max<int64_t>(1, std::min<int64_t>(tgd_parts(g.M, g.N, g.K), room));
+  const dim3 grid(mt, nt, kz);
   constexpr size_t smem = tgd_smem<TA>();
   const bool a16 = (g.astep * (int64_t)sizeof(TA)) % 16 == 0;
   auto go = [&](auto kern) {
     XCUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<grid, TG_NT, smem, s>>>(g.M, g.N, g.K, A, g.aoff, B, g.ldb, g.alpha, C, g.coff, g.accumulate);
+    kern<<<grid, TG_NT, smem, s>>>(g.M, g.N, g.K, A, g.aoff, B, g.ldb, g.alpha, C, g.coff, g.accumulate,
+                                   g.scratch);
   };
   if (a16) go(k_tgemm_f64<TA, TC, 16>);
   else go(k_tgemm_f64<TA, TC, 8>);
   XLAUNCH();
+}
+// K parts of a tensor-core GEMM for levels with few row tiles (two CTAs per SM, about two waves), at least 8
+// steps each; only where C is accumulated into
+static int tc_parts(int M, int N, int K) {
+  const int tiles = ((M + TC_BM - 1) / TC_BM) * ((N + TC_BN - 1) / TC_BN), steps = (K + TC_BK - 1) / TC_BK;
+  if (M <= 0 || N <= 0) return 1;
+  const int want = (XFMM_TC_KSPLIT_CTAS + tiles - 1) / tiles;
+  return std::max(1, std::min(std::min(want, steps / 8), XFMM_TC_KSPLIT_MAX));
+}
+// the scratch (in doubles) a split tgemm_tc of M x N x K needs, 0 when it does not split
+int64_t tgemm_tc_scratch(int M, int N, int K, int accumulate) {
+  const int kz = accumulate ? tc_parts(M, N, K) : 1;
+  return kz > 1 ? ((int64_t)kz * M * ((N + TC_BN - 1) / TC_BN * TC_BN) + 1) / 2 : 0;
 }
 template <class TC>
 void tgemm_tc(const TGemm& g, const float* A, const float* Bth, const float* Btl, int64_t ldbt, TC* C,
@@ -561,19 +650,10 @@ void tgemm_tc(const TGemm& g, const float* A, const float* Bth, const float* Btl
   if (g.M <= 0 || g.N <= 0) return;
   XREQUIRE(g.status && g.astep % 2 == 0 && ldbt % TC_BK == 0, XFMM_ERR_UNSUPPORTED,
            "tensor-core translation: status flag and aligned rows required");
-  // K split over blockIdx.z for levels with few row tiles (two CTAs per SM, about two waves), in parts
-  // of at least 8 steps; only where C is accumulated into (the parts are added with atomics)
   const int mt = (g.M + TC_BM - 1) / TC_BM, nt = (g.N + TC_BN - 1) / TC_BN, nsteps = (g.K + TC_BK - 1) / TC_BK;
-  int kz = 1;
-  if (g.accumulate) {
-    const int want = (XFMM_TC_KSPLIT_CTAS + mt * nt - 1) / (mt * nt);
-    kz = std::max(1, std::min(std::min(want, nsteps / 8), XFMM_TC_KSPLIT_MAX));
-  }
-  if (kz > 1) {
-    // the parts meet in an FP64 scratch ([M][N], zero between uses), then one pass adds it into C
-    XREQUIRE(g.scratch && g.scratch_len >= (int64_t)g.M * g.N, XFMM_ERR_UNSUPPORTED,
-             "split tensor-core translation: scratch too small");
-  }
+  const int kz = g.accumulate ? tc_parts(g.M, g.N, g.K) : 1;
+  XREQUIRE(kz == 1 || (g.scratch && g.scratch_len >= tgemm_tc_scratch(g.M, g.N, g.K, 1)), XFMM_ERR_UNSUPPORTED,
+           "split tensor-core translation: scratch too small");
   const dim3 grid(mt, nt, kz);
   // In place, three CTAs share an SM; measured faster except for short K (fewer than 32 steps) with many
   // column tiles (the Laplace L2L: 0.86 ms with the raw buffers, 1.06 ms in place), which keeps the raw
@@ -588,17 +668,10 @@ void tgemm_tc(const TGemm& g, const float* A, const float* Bth, const float* Btl
   else ip ? go(k_tgemm_tc<TC, 8, true>, TC_SMEM_IP) : go(k_tgemm_tc<TC, 8, false>, TC_SMEM_RAW);
   XLAUNCH();
   if (kz > 1) {
-    k_tc_finish<TC><<<tg_blocks((int64_t)g.M * g.N), 256, 0, s>>>(g.M, g.N, g.scratch, C, g.coff, g.accumulate);
+    k_tc_finish<TC><<<tg_blocks((int64_t)g.M * g.N), 256, 0, s>>>(
+        g.M, g.N, nt * TC_BN, kz, reinterpret_cast<const float*>(g.scratch), g.alpha, C, g.coff, g.accumulate);
     XLAUNCH();
   }
-}
-// the FP64 scratch (doubles) a split tgemm_tc of M x N needs, 0 when it does not split
-int64_t tgemm_tc_scratch(int M, int N, int K, int accumulate) {
-  const int mt = (M + TC_BM - 1) / TC_BM, nt = (N + TC_BN - 1) / TC_BN, nsteps = (K + TC_BK - 1) / TC_BK;
-  if (!accumulate || M <= 0 || N <= 0) return 0;
-  const int want = (XFMM_TC_KSPLIT_CTAS + mt * nt - 1) / (mt * nt);
-  const int kz = std::max(1, std::min(std::min(want, nsteps / 8), XFMM_TC_KSPLIT_MAX));
-  return kz > 1 ? (int64_t)M * N : 0;
 }
 template void tgemm_tc<float>(const TGemm&, const float*, const float*, const float*, int64_t, float*, cudaStream_t);
 template void tgemm_tc<double>(const TGemm&, const float*, const float*, const float*, int64_t, double*, cudaStream_t);
