@@ -82,7 +82,7 @@ __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
 // order, so the result does not depend on the order of arrival.  FP64: the part that finishes last (a
 // counter per tile; no part waits for another) adds the tile's parts and writes the rows; the counters
 // stand at the front of the scratch and are zero between uses.  Tensor-core GEMM: a pass over the rows
-// (k_tc_finish), since its wider tiles take many parts (the last of up to 18 parts adding 128 x 64 sums
+// (k_tc_finish; its parts stand behind the counters too), since its wider tiles take many parts (the last of up to 18 parts adding 128 x 64 sums
 // alone measured 0.71 ms for the M2M of a 300k Plummer set against 0.22 with FP64 atomics).
 constexpr int SPLIT_COUNTERS = 4096;  // tiles a split GEMM may have
 constexpr int64_t SPLIT_HEAD = SPLIT_COUNTERS * sizeof(unsigned) / sizeof(double);  // in doubles
@@ -493,7 +493,8 @@ __global__ void __launch_bounds__(TC_NT, IP ? 3 : 2)
     // a part of a split K: its FP32 sums to [z][row][column], added by k_tc_finish
     const int r = m0 + 32 * w + lane, ld = gridDim.y * TC_BN;
     if (r < M) {
-      float4* o = reinterpret_cast<float4*>(reinterpret_cast<float*>(scratch) + ((int64_t)blockIdx.z * M + r) * ld + n0);
+      float4* o = reinterpret_cast<float4*>(reinterpret_cast<float*>(scratch + SPLIT_HEAD) +
+                                          ((int64_t)blockIdx.z * M + r) * ld + n0);
 #pragma unroll
       for (int j = 0; j < TC_BN; j += 4) o[j / 4] = make_float4(run[j], run[j + 1], run[j + 2], run[j + 3]);
     }
@@ -642,7 +643,7 @@ static int tc_parts(int M, int N, int K) {
 // the scratch (in doubles) a split tgemm_tc of M x N x K needs, 0 when it does not split
 int64_t tgemm_tc_scratch(int M, int N, int K, int accumulate) {
   const int kz = accumulate ? tc_parts(M, N, K) : 1;
-  return kz > 1 ? ((int64_t)kz * M * ((N + TC_BN - 1) / TC_BN * TC_BN) + 1) / 2 : 0;
+  return kz > 1 ? SPLIT_HEAD + ((int64_t)kz * M * ((N + TC_BN - 1) / TC_BN * TC_BN) + 1) / 2 : 0;
 }
 template <class TC>
 void tgemm_tc(const TGemm& g, const float* A, const float* Bth, const float* Btl, int64_t ldbt, TC* C,
@@ -669,7 +670,7 @@ void tgemm_tc(const TGemm& g, const float* A, const float* Bth, const float* Btl
   XLAUNCH();
   if (kz > 1) {
     k_tc_finish<TC><<<tg_blocks((int64_t)g.M * g.N), 256, 0, s>>>(
-        g.M, g.N, nt * TC_BN, kz, reinterpret_cast<const float*>(g.scratch), g.alpha, C, g.coff, g.accumulate);
+        g.M, g.N, nt * TC_BN, kz, reinterpret_cast<const float*>(g.scratch + SPLIT_HEAD), g.alpha, C, g.coff, g.accumulate);
     XLAUNCH();
   }
 }
