@@ -71,6 +71,29 @@ void host_surface_base(int p, std::vector<double>& c) {
   for (int i = 0; i < (n / 2) * 3; i++) c[3 * cnt + i] = -c[i];
 }
 
+// The surface points of order p line by line: 4 p - 4 lines along x (j over z = -1, then z = +1; then z interior
+// over y = -1, then y = +1), 2 (p - 2) lines along y without their ends (z interior over x = -1, then x = +1).
+// perm[position] = surface index; grid: the p coordinates of one axis, ascending.
+void host_surface_lines(int p, const std::vector<double>& base, std::vector<int>& perm, std::vector<double>& grid) {
+  grid.resize(p);
+  for (int i = 0; i < p; i++) grid[i] = (2.0 * i - p + 1) / (p - 1);
+  std::vector<int> at((size_t)p * p * p, -1);
+  auto cell = [&](int i, int j, int l) -> int& { return at[((size_t)l * p + j) * p + i]; };
+  auto index = [&](double v) { return (int)std::lround(0.5 * (v + 1.0) * (p - 1)); };
+  for (size_t k = 0; k < base.size() / 3; k++)
+    cell(index(base[3 * k]), index(base[3 * k + 1]), index(base[3 * k + 2])) = (int)k;
+  perm.clear();
+  for (int l : {0, p - 1})
+    for (int j = 0; j < p; j++)
+      for (int i = 0; i < p; i++) perm.push_back(cell(i, j, l));
+  for (int j : {0, p - 1})
+    for (int l = 1; l < p - 1; l++)
+      for (int i = 0; i < p; i++) perm.push_back(cell(i, j, l));
+  for (int i : {0, p - 1})
+    for (int l = 1; l < p - 1; l++)
+      for (int j = 1; j < p - 1; j++) perm.push_back(cell(i, j, l));
+}
+
 namespace {
 
 // geometry.h:55-62
@@ -403,6 +426,12 @@ void precompute(Fmm& f, int depth, cudaStream_t s) {
   // geometry tables shared by all levels
   host_surface_base(p, f.h_surf_base);
   f.surf_base.upload(f.h_surf_base, s);
+  std::vector<int> perm;
+  std::vector<double> line_grid;
+  host_surface_lines(p, f.h_surf_base, perm, line_grid);
+  f.surf_perm.upload(perm, s);
+  f.surf_grid.upload(line_grid, s);
+  XCUDA(cudaStreamSynchronize(s));
   std::vector<int> mup = host_surf2conv(p, true), mdn = host_surf2conv(p, false);
   f.map_up.upload(mup, s);
   f.map_dn.upload(mdn, s);

@@ -190,6 +190,8 @@ struct Fmm {
   int pre_depth = -1;
   std::vector<LevelOps> ops;          // 1 (Laplace) or depth+1 (per-level kernels)
   DBuf<double> surf_base;             // [nsurf][3] unit surface (geometry.h:21-54 before scaling)
+  DBuf<int> surf_perm;                // surface points line by line along x, then y (host_surface_lines)
+  DBuf<double> surf_grid;             // [p] grid coordinates of the unit surface along one axis
   DBuf<int> map_up, map_dn;           // surface index -> conv-grid index (geometry.h:101-134)
   DBuf<int> conv_to_surf_up;          // conv-grid index -> surface index or -1
   DBuf<double> dft_tw;                // [n1] (cos, sin)(2 pi m / n1): factors of the M2L transforms
@@ -207,6 +209,7 @@ void m2l_setup(Fmm& fmm, Tree& t, cudaStream_t s);
 // precompute.cu
 void precompute(Fmm& fmm, int depth, cudaStream_t s);
 void host_surface_base(int p, std::vector<double>& out);
+void host_surface_lines(int p, const std::vector<double>& base, std::vector<int>& perm, std::vector<double>& grid);
 // evaluate.cu
 void m2l_fragments(LevelOps& op, const double* T64, int nfreq, cudaStream_t s);
 void set_charges(Fmm& fmm, Tree& t, const double* q, bool on_device, cudaStream_t s);
