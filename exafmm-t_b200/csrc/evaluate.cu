@@ -500,8 +500,11 @@ void order_dispatch(int p, F&& fn) {
     default: throw Error(XFMM_ERR_UNSUPPORTED, "expansion order p must be in [2, 16]");
   }
 }
-// Leaves below which FAR_PARTS / NEAR_PARTS warps share one: about four times the warps resident at once.
-constexpr int SPLIT_LEAVES = 4 * 148 * 24;
+// Leaves below which several warps share one (FAR_PARTS, NEAR_PARTS, the surfaces of P2M and P2L): 64 per SM, two
+// to three times the warps resident at once.  Near field: 1.5k leaves (Plummer 20k, FP64) 0.49 -> 0.15 ms, 8.4k
+// (Plummer 300k, mixed) 0.62 -> 0.29, 4.6k even leaves (Helmholtz 200k) 0.77 -> 0.70; with 14k (Yukawa
+// sphere 300k) sharing cost more than it evened out, 0.305 -> 0.340.
+constexpr int SPLIT_LEAVES = 148 * 64;
 
 // ================================================================ near field (P2P)
 // Warp per target leaf.  The sources of the leaf's P2P list form one continuous stream that is
@@ -512,6 +515,11 @@ constexpr int SPLIT_LEAVES = 4 * 148 * 24;
 //   T <  32 : G lanes per target (G = 32 / 2^ceil(log2 T)), each taking every G-th source of a
 //             chunk, partial sums combined with shuffles at the end.
 // FP32 chunk sums are accumulated in FP64.
+// A system of few leaves would leave the chip idle behind its longest leaves: NEAR_PARTS warps then share a
+// leaf, part k taking every NEAR_PARTS-th chunk from the k-th, and the parts' FP64 sums are added in order.
+// How many parts a leaf has is fixed by its system's leaf count (NearArgs::parts), and a kernel that has
+// one warp per leaf takes the parts one after another, so the results do not depend on the kernel.
+constexpr int NEAR_PARTS = 4;
 struct NearArgs {
   const int *eval_leafs, *leafs, *nsrcs, *ntrgs;
   int n_eval;
@@ -521,6 +529,7 @@ struct NearArgs {
   const double* src_qim;
   double* out;
   double k_re, k_im;
+  int parts;  // 1 or NEAR_PARTS
 };
 
 template <class R> struct Stage4;
@@ -536,8 +545,10 @@ struct NearSmem {
   int seg_pre[NEAR_SEG + 1];
 };
 
-template <int KER, class R, int TPL>
-__device__ __forceinline__ void near_leaf(const NearArgs& a, int node, int lane, NearSmem<R>& sm) {
+// PARTS 1: the whole leaf, or its parts one after another (a.parts); NEAR_PARTS: part `part` of a leaf shared by
+// the warps of the CTA, all of which call this
+template <int KER, class R, int TPL, int PARTS = 1>
+__device__ __forceinline__ void near_leaf(const NearArgs& a, int node, int lane, NearSmem<R>& sm, int part = 0) {
   using G = Green<KER, R>;
   using Q = typename G::Q;
   using A = typename Acc64<Q>::type;
@@ -557,6 +568,8 @@ __device__ __forceinline__ void near_leaf(const NearArgs& a, int node, int lane,
   for (int t0 = 0; t0 < T; t0 += 32 * TPL) {
     R tx[TPL], ty[TPL], tz[TPL], lx[TPL], ly[TPL], lz[TPL];
     A P[TPL], GX[TPL], GY[TPL], GZ[TPL];
+    const int np = a.parts, k0 = PARTS > 1 ? part : 0, k1 = PARTS > 1 ? part + 1 : np;
+    A SP[TPL], SX[TPL], SY[TPL], SZ[TPL];  // sums of the parts before
 #pragma unroll
     for (int u = 0; u < TPL; u++) {
       const int t = t0 + tl + 32 * u;
@@ -573,20 +586,22 @@ __device__ __forceinline__ void near_leaf(const NearArgs& a, int node, int lane,
       lx[u] = (R)(dx - (double)tx[u]);
       ly[u] = (R)(dy - (double)ty[u]);
       lz[u] = (R)(dz - (double)tz[u]);
-      P[u] = GX[u] = GY[u] = GZ[u] = A();
     }
+    for (int k = k0; k < k1; k++) {
+#pragma unroll
+    for (int u = 0; u < TPL; u++) P[u] = GX[u] = GY[u] = GZ[u] = A();
     for (int64_t eb = e0; eb < e1; eb += NEAR_SEG) {
       // segment table of this batch: begin offsets and an inclusive prefix of counts
       const int nseg = (int)(e1 - eb < NEAR_SEG ? e1 - eb : NEAR_SEG);
       __syncwarp();
       int carry = 0;
-      for (int k0 = 0; k0 < nseg; k0 += 32) {
-        const int k = k0 + lane;
+      for (int q0 = 0; q0 < nseg; q0 += 32) {
+        const int q = q0 + lane;
         int cnt = 0;
-        if (k < nseg) {
-          const int sn = a.p2p[eb + k];
+        if (q < nseg) {
+          const int sn = a.p2p[eb + q];
           cnt = a.nsrcs[sn];
-          sm.seg_beg[k] = a.sbeg[sn];
+          sm.seg_beg[q] = a.sbeg[sn];
         }
         int incl = cnt;
 #pragma unroll
@@ -594,14 +609,14 @@ __device__ __forceinline__ void near_leaf(const NearArgs& a, int node, int lane,
           const int v = __shfl_up_sync(0xffffffffu, incl, o);
           if (lane >= o) incl += v;
         }
-        if (k < nseg) sm.seg_pre[k + 1] = carry + incl;
+        if (q < nseg) sm.seg_pre[q + 1] = carry + incl;
         carry += __shfl_sync(0xffffffffu, incl, 31);
       }
       if (lane == 0) sm.seg_pre[0] = 0;
       __syncwarp();
       const int total = carry;
       int seg = 0;  // per-lane cursor into the segment table
-      for (int p0 = 0; p0 < total; p0 += 32) {
+      for (int p0 = 32 * k; p0 < total; p0 += 32 * np) {
         const int pos = p0 + lane;
         __syncwarp();
         if (pos < total) {
@@ -654,6 +669,48 @@ __device__ __forceinline__ void near_leaf(const NearArgs& a, int node, int lane,
           acc64(GZ[u], gz[u]);
         }
       }
+    }
+    if (PARTS == 1 && np > 1) {
+#pragma unroll
+      for (int u = 0; u < TPL; u++) {
+        if (k > k0) {
+          P[u] = vadd(SP[u], P[u]);
+          GX[u] = vadd(SX[u], GX[u]);
+          GY[u] = vadd(SY[u], GY[u]);
+          GZ[u] = vadd(SZ[u], GZ[u]);
+        }
+        SP[u] = P[u];
+        SX[u] = GX[u];
+        SY[u] = GY[u];
+        SZ[u] = GZ[u];
+      }
+    }
+    }
+    if constexpr (PARTS > 1) {
+      __shared__ A red[PARTS - 1][4 * TPL][32];
+      if (part > 0) {
+#pragma unroll
+        for (int u = 0; u < TPL; u++) {
+          red[part - 1][4 * u][lane] = P[u];
+          red[part - 1][4 * u + 1][lane] = GX[u];
+          red[part - 1][4 * u + 2][lane] = GY[u];
+          red[part - 1][4 * u + 3][lane] = GZ[u];
+        }
+      }
+      __syncthreads();
+      if (part == 0) {
+#pragma unroll
+        for (int q = 0; q < PARTS - 1; q++)
+#pragma unroll
+          for (int u = 0; u < TPL; u++) {
+            P[u] = vadd(P[u], red[q][4 * u][lane]);
+            GX[u] = vadd(GX[u], red[q][4 * u + 1][lane]);
+            GY[u] = vadd(GY[u], red[q][4 * u + 2][lane]);
+            GZ[u] = vadd(GZ[u], red[q][4 * u + 3][lane]);
+          }
+      }
+      __syncthreads();
+      if (part > 0) continue;  // the next block of targets
     }
     if (TPL == 1) {
       for (int o = 1; o < G2; o <<= 1) {
@@ -718,8 +775,8 @@ struct NearSmemF2 {
 
 __device__ __forceinline__ float2 dup2(float a) { return make_float2(a, a); }
 
-template <int TPL>
-__device__ __forceinline__ void near_leaf_lap_f2(const NearArgs& a, int node, int lane, NearSmemF2& sm) {
+template <int TPL, int PARTS = 1>  // PARTS as in near_leaf (PARTS 1: the whole leaf in one pass)
+__device__ __forceinline__ void near_leaf_lap_f2(const NearArgs& a, int node, int lane, NearSmemF2& sm, int part = 0) {
   const int T = a.ntrgs[node];
   const int64_t tb = a.tbeg[node];
   const int64_t e0 = a.p2p_off[node], e1 = a.p2p_off[node + 1];
@@ -769,7 +826,7 @@ __device__ __forceinline__ void near_leaf_lap_f2(const NearArgs& a, int node, in
       __syncwarp();
       const int total = carry;
       int seg = 0;
-      for (int p0 = 0; p0 < total; p0 += NEAR_CH) {
+      for (int p0 = NEAR_CH * part; p0 < total; p0 += NEAR_CH * PARTS) {
         __syncwarp();
 #pragma unroll
         for (int h = 0; h < NEAR_CH / 32; h++) {
@@ -828,6 +885,32 @@ __device__ __forceinline__ void near_leaf_lap_f2(const NearArgs& a, int node, in
         }
       }
     }
+    if constexpr (PARTS > 1) {
+      __shared__ double red[PARTS - 1][4 * TPL][32];
+      if (part > 0) {
+#pragma unroll
+        for (int u = 0; u < TPL; u++) {
+          red[part - 1][4 * u][lane] = P[u];
+          red[part - 1][4 * u + 1][lane] = GX[u];
+          red[part - 1][4 * u + 2][lane] = GY[u];
+          red[part - 1][4 * u + 3][lane] = GZ[u];
+        }
+      }
+      __syncthreads();
+      if (part == 0) {
+#pragma unroll
+        for (int q = 0; q < PARTS - 1; q++)
+#pragma unroll
+          for (int u = 0; u < TPL; u++) {
+            P[u] += red[q][4 * u][lane];
+            GX[u] += red[q][4 * u + 1][lane];
+            GY[u] += red[q][4 * u + 2][lane];
+            GZ[u] += red[q][4 * u + 3][lane];
+          }
+      }
+      __syncthreads();
+      if (part > 0) continue;  // the next block of targets
+    }
     if (TPL == 1) {
       for (int o = 1; o < G2; o <<= 1) {
         P[0] += __shfl_xor_sync(0xffffffffu, P[0], o);
@@ -866,6 +949,15 @@ __global__ void __launch_bounds__(128, XFMM_NEARF2_MINB) k_near_lap_f2(NearArgs 
   if (T <= 32) near_leaf_lap_f2<1>(a, node, lane, sm[wid]);
   else if (T <= 64 || XFMM_NEARF2_TPL == 2) near_leaf_lap_f2<2>(a, node, lane, sm[wid]);
   else near_leaf_lap_f2<XFMM_NEARF2_TPL>(a, node, lane, sm[wid]);
+}
+
+// the same with the CTA's warps sharing a leaf (few leaves)
+__global__ void __launch_bounds__(32 * NEAR_PARTS, XFMM_NEARF2_MINB) k_near_lap_f2_parts(NearArgs a) {
+  __shared__ NearSmemF2 sm[NEAR_PARTS];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int node = a.leafs[a.eval_leafs[blockIdx.x]];
+  if (a.ntrgs[node] <= 32) near_leaf_lap_f2<1, NEAR_PARTS>(a, node, lane, sm[wid], wid);
+  else near_leaf_lap_f2<2, NEAR_PARTS>(a, node, lane, sm[wid], wid);
 }
 
 // The near field's close pairs (k_near_lap_f2): every (target, source) of a leaf's U list whose FP32
@@ -989,6 +1081,16 @@ __global__ void __launch_bounds__(128, XFMM_NEAR_MINB) k_near(NearArgs a) {
   }
 }
 
+// the same with the CTA's warps sharing a leaf (few leaves)
+template <int KER, class R>
+__global__ void __launch_bounds__(32 * NEAR_PARTS, XFMM_NEAR_MINB) k_near_parts(NearArgs a) {
+  __shared__ NearSmem<R> sm[NEAR_PARTS];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int node = a.leafs[a.eval_leafs[blockIdx.x]];
+  if (sizeof(R) == 4 && a.ntrgs[node] > 32) near_leaf<KER, R, (sizeof(R) == 4 ? 2 : 1), NEAR_PARTS>(a, node, lane, sm[wid], wid);
+  else near_leaf<KER, R, 1, NEAR_PARTS>(a, node, lane, sm[wid], wid);
+}
+
 // ================================================================ P2M check potentials and P2L
 // Potential at `n` surface points (base * b around centre cn) from body range(s); warp per node.
 // The Laplace operators are scale-invariant: computed for root radius pre_r0, they serve a tree of root
@@ -1016,6 +1118,15 @@ struct SurfPotArgs {
   double scale;        // 1 / (4 pi) x op_scale(f, t): the Green's function constant and the operators' r0 scale
 };
 
+// The points [k0, k1) of a surface of n that blockIdx.y takes: with few nodes several warps share one, each a
+// run of whole 32-point rows (the points are independent: the sums do not depend on the split).
+__device__ __forceinline__ void surf_range(int n, int& k0, int& k1) {
+  const int per = ((n + (int)gridDim.y - 1) / (int)gridDim.y + 31) & ~31;
+  k0 = min(n, (int)blockIdx.y * per);
+  k1 = min(n, k0 + per);
+}
+inline dim3 surf_grid_of(int count) { return dim3(nblk(count, 4), count < SPLIT_LEAVES ? 4 : 1); }
+
 template <int KER, class R>
 __global__ void __launch_bounds__(128) k_surf_pot(SurfPotArgs a) {
   using G = Green<KER, R>;
@@ -1031,6 +1142,9 @@ __global__ void __launch_bounds__(128) k_surf_pot(SurfPotArgs a) {
   const double4 c = a.center[node];
   const double b = a.alpha * c.w;
   const int n = a.nsurf;
+  int kb, ke;
+  surf_range(n, kb, ke);
+  if (kb >= ke) return;
   Q* out = (Q*)a.out + (int64_t)(a.out_by_node ? node : w) * n;
   const bool p2l = a.out_by_node;
   const int64_t e0 = p2l ? a.p2l_off[node] : 0, e1 = p2l ? a.p2l_off[node + 1] : 1;
@@ -1047,7 +1161,7 @@ __global__ void __launch_bounds__(128) k_surf_pot(SurfPotArgs a) {
         s_q[wid][lane] = load_charge<Q>(sv, a.src_qim, sb + j0 + lane);
       }
       __syncwarp();
-      for (int k = lane; k < n; k += 32) {
+      for (int k = kb + lane; k < ke; k += 32) {
         const R px = (R)(a.surf_base[3 * k] * b), py = (R)(a.surf_base[3 * k + 1] * b),
                 pz = (R)(a.surf_base[3 * k + 2] * b);
         Q acc = vzero<Q>();
@@ -1082,6 +1196,9 @@ __global__ void __launch_bounds__(128) k_surf_pot_lap_f2(SurfPotArgs a) {
   const double4 c = a.center[node];
   const double b = a.alpha * c.w;
   const int n = a.nsurf, ns = a.nsrcs[node];
+  int kb, ke;
+  surf_range(n, kb, ke);
+  if (kb >= ke) return;
   const int64_t sb = a.sbeg[node];
   float* out = (float*)a.out + (int64_t)w * n;
   const float2 M1 = make_float2(-1.f, -1.f);
@@ -1106,8 +1223,8 @@ __global__ void __launch_bounds__(128) k_surf_pot_lap_f2(SurfPotArgs a) {
     }
     __syncwarp();
     const int npair = (min(64, max(ns - j0, 0)) + 1) >> 1;
-    for (int k0 = 0; k0 < n; k0 += 32 * SP_KB) {
-      const int nk = min(SP_KB, (n - k0 + 31) >> 5);  // slots of this block holding points (warp-uniform)
+    for (int k0 = kb; k0 < ke; k0 += 32 * SP_KB) {
+      const int nk = min(SP_KB, (ke - k0 + 31) >> 5);  // slots of this block holding points (warp-uniform)
       float2 px[SP_KB], py[SP_KB], pz[SP_KB], acc[SP_KB];
 #pragma unroll
       for (int i = 0; i < SP_KB; i++) {
@@ -1134,7 +1251,7 @@ __global__ void __launch_bounds__(128) k_surf_pot_lap_f2(SurfPotArgs a) {
 #pragma unroll
       for (int i = 0; i < SP_KB; i++) {
         const int k = k0 + lane + 32 * i;
-        if (k < n) {
+        if (k < ke) {
           const float o = (acc[i].x + acc[i].y) * (float)a.scale;
           out[k] = first ? o : out[k] + o;
         }
@@ -3080,9 +3197,9 @@ struct Engine {
                       t.src4.p,   t.src_qim.p, f.surf_base.p, n,      2.95,      ws.chk.p, 0,         f.k_re, f.k_im,
                       INV4PI * op_scale(f, t)};
         if constexpr (KER == K_LAPLACE && sizeof(R) == 4)
-          k_surf_pot_lap_f2<<<nblk(t.nleafs, 4), 128, 0, s>>>(a);
+          k_surf_pot_lap_f2<<<surf_grid_of(t.nleafs), 128, 0, s>>>(a);
         else
-          k_surf_pot<KER, R><<<nblk(t.nleafs, 4), 128, 0, s>>>(a);
+          k_surf_pot<KER, R><<<surf_grid_of(t.nleafs), 128, 0, s>>>(a);
         XLAUNCH();
         ws.launches++;
       }
@@ -3369,7 +3486,7 @@ struct Engine {
   static NearArgs near_args(Fmm& f, Tree& t, Workspace& ws) {
     return NearArgs{t.eval_leafs.p, t.leafs.p, t.nsrcs.p,   t.ntrgs.p, t.n_eval_leafs, t.sbeg.p, t.tbeg.p,
                     t.p2p_off.p,    t.p2p.p,   t.center.p,  t.src4.p,  t.trg4.p,       t.src_qim.p, ws.out.p,
-                    f.k_re,         f.k_im};
+                    f.k_re,         f.k_im,    t.n_eval_leafs < SPLIT_LEAVES ? NEAR_PARTS : 1};
   }
 
   // phases: DOWN_PRE (P2L, M2L, L2L, L2P check-to-equivalent), DOWN_NEAR (P2P), DOWN_FAR (M2P + L2P
@@ -3381,7 +3498,8 @@ struct Engine {
       NearArgs na = near_args(f, t, ws);
       if constexpr (KER == K_LAPLACE && sizeof(R) == 4) {
         if (ws.n_close < 0) find_close_pairs(ws, na, t.n_eval_leafs, s);
-        k_near_lap_f2<<<nblk(t.n_eval_leafs, 4), 128, 0, s>>>(na);
+        if (na.parts > 1) k_near_lap_f2_parts<<<t.n_eval_leafs, 32 * NEAR_PARTS, 0, s>>>(na);
+        else k_near_lap_f2<<<nblk(t.n_eval_leafs, 4), 128, 0, s>>>(na);
         XLAUNCH();
         ws.launches++;
         if (ws.n_close > 0) {
@@ -3390,7 +3508,8 @@ struct Engine {
           ws.launches++;
         }
       } else {
-        k_near<KER, R><<<nblk(t.n_eval_leafs, 4), 128, 0, s>>>(na);
+        if (na.parts > 1) k_near_parts<KER, R><<<t.n_eval_leafs, 32 * NEAR_PARTS, 0, s>>>(na);
+        else k_near<KER, R><<<nblk(t.n_eval_leafs, 4), 128, 0, s>>>(na);
         XLAUNCH();
         ws.launches++;
       }
@@ -3426,7 +3545,7 @@ struct Engine {
       SurfPotArgs a{t.p2l_nodes.p, t.n_p2l_nodes, t.nsrcs.p,     t.p2l.p, t.level.p, t.sbeg.p, t.p2l_off.p, t.center.p,
                     t.src4.p,      t.src_qim.p,   f.surf_base.p, n,       1.05,      ws.dn.p,  1,           f.k_re,
                     f.k_im,        INV4PI * op_scale(f, t)};
-      k_surf_pot<KER, R><<<nblk(t.n_p2l_nodes, 4), 128, 0, s>>>(a);
+      k_surf_pot<KER, R><<<surf_grid_of(t.n_p2l_nodes), 128, 0, s>>>(a);
       XLAUNCH();
       ws.launches++;
     }

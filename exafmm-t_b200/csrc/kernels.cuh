@@ -124,7 +124,7 @@ template <class R, int NS> struct Green<K_HELMHOLTZ, R, NS> {
     const R r = r2 * invr;
     R sn, cs;
     sincos_any(k_re * r, &sn, &cs);
-    const R e = exp_any(-k_im * r) * invr;
+    const R e = k_im == R(0) ? invr : exp_any(-k_im * r) * invr;  // a real wavenumber needs no exponential
     const R gr = e * cs, gi = e * sn;
     acc.x += q.x * gr - q.y * gi;
     acc.y += q.x * gi + q.y * gr;
@@ -137,7 +137,7 @@ template <class R, int NS> struct Green<K_HELMHOLTZ, R, NS> {
     const R r = r2 * invr;
     R sn, cs;
     sincos_any(k_re * r, &sn, &cs);
-    const R e = exp_any(-k_im * r) * invr;
+    const R e = k_im == R(0) ? invr : exp_any(-k_im * r) * invr;  // a real wavenumber needs no exponential
     const R gr = e * cs, gi = e * sn;
     const R pr = q.x * gr - q.y * gi, pi = q.x * gi + q.y * gr;
     p.x += pr;
