@@ -1309,90 +1309,103 @@ void transpose(const CT* in, CT* out, int64_t R, int64_t C, cudaStream_t s) {
 // The FP64 path's form runs on the FP64 tensor cores (k_hadamard_d64), the mixed path's on the FP16 tensor
 // cores with split operands (k_hadamard_h below).
 
-// Hadamard product of the FP64 path on the FP64 tensor cores (DMMA, mma.sync m8n8k4 f64), dense form for
-// every target: per frequency, D[target][16] = A[target][26 x 16] B[26 x 16][16] as in k_hadamard_h,
-// accumulated in FP64 by the tensor core across the positions.  A warp owns HAD64_TW tiles of 8 targets;
-// per (tile, position) eight DMMAs (4 reduction steps x 2 output halves) add the position's products to the
-// tile's accumulators.  The reduction index of step c is input real 4 t + c, so that a lane (g, t) supplies
-// the reals 4 t .. 4 t + 3 of its target g's source spectrum (32 contiguous bytes) and receives the output
-// component 4 h + t (re, im) of target g.  A position none of a tile's 8 targets occupies is skipped (warp
-// ballot); sources are loaded one position ahead.
-constexpr int HAD64_NT = 256, HAD64_TW = 2;
+// Hadamard product of the FP64 path on the FP64 tensor cores (DMMA, mma.sync m8n8k4 f64), for every target.
+// A complex product needs three real ones (Gauss): with a = source, b = operator,
+//   k1 = (a.re + a.im) b.re,  k2 = a.re (b.im - b.re),  k3 = a.im (b.re + b.im),  a b = (k1 - k3) + i (k1 + k2),
+// and the three sums run over the positions and source components before they are combined: per frequency
+// three real GEMMs D_i[target][8] = A_i[target][26 x 8] B_i[26 x 8][8], six DMMAs per 8 targets and position
+// (two 4-wide reduction steps) where the 2 x 2 real form takes eight.  The FP64 tensor pipe bounds it (16 cycles per
+// DMMA and SM quadrant, measured: the same 64 FMA per SM and clock as the FP64 lanes): 1M bodies, p = 8:
+// 5.47 -> 3.83 ms (100k: 0.76 -> 0.57; Helmholtz 50k: 0.95 -> 0.69).
+// A warp owns HAD64_TW tiles of 8 targets.  Lane (g, t) supplies components 2 t, 2 t + 1 of its target g's
+// source spectrum, 32 contiguous bytes in one load (a row's quad reads a whole 128-byte line), step c taking
+// component 2 t + c, and receives the target components 2 t, 2 t + 1.  A position none of a tile's 8 targets
+// occupies is skipped (warp ballot); a tile's next spectra are loaded as soon as its products are issued.
+// The operator's B fragments are built once per table (k_m2l_fragments64) and copied per CTA.
+constexpr int HAD64_NT = 256, HAD64_TW = 4;
 constexpr int HAD64_TT = (HAD64_NT / 32) * 8 * HAD64_TW;  // targets per CTA
-constexpr size_t HAD64_SMEM = (size_t)26 * 4 * 2 * 32 * sizeof(double);
+constexpr int HAD64_B = 26 * 6 * 32;                      // B fragments (doubles) per frequency
+constexpr size_t HAD64_SMEM = (size_t)HAD64_B * sizeof(double);
 
 __device__ __forceinline__ void dmma_884(double (&d)[2], double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
                : "+d"(d[0]), "+d"(d[1])
                : "d"(a), "d"(b));
 }
+// frag[(f * 26 + ipos) * 6 * 32 + (2 i + c) * 32 + lane] = B_i[component 2 t + c][component g] of the block
+// of position ipos, i = 0, 1, 2: b.re, b.im - b.re, b.re + b.im.  One warp per block.
+__global__ void k_m2l_fragments64(const double2* __restrict__ T, int nfreq, double* __restrict__ frag) {
+  const int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  if (w >= 26ll * nfreq) return;
+  const int f = (int)(w / 26), ipos = (int)(w % 26);
+  const double2* blk = T + ((int64_t)ipos * nfreq + f) * 64;
+  double* o = frag + w * 6 * 32 + lane;
+#pragma unroll
+  for (int c = 0; c < 2; c++) {
+    const double2 m = blk[(2 * t + c) * 8 + g];
+    o[c * 32] = m.x;
+    o[(2 + c) * 32] = m.y - m.x;
+    o[(4 + c) * 32] = m.x + m.y;
+  }
+}
+__device__ __forceinline__ double4 ldg_double4(const double* p) {  // 32-byte aligned
+  double4 v;
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+  return v;
+}
 
 // tab: [26][ld] compact source index of target k at each position (-1: empty or padding); rows: [ld]
 // output row of target k (-1: padding); ld a multiple of HAD64_TT
 __global__ void __launch_bounds__(HAD64_NT, 2)
-    k_hadamard_d64(const double2* __restrict__ T, const double2* __restrict__ in, double2* __restrict__ out,
-                   const int* __restrict__ tab, int ld, const int* __restrict__ rows, int nsrc, int ntrg, int nfreq) {
-  // sB[((ipos * 4 + c) * 2 + h) * 32 + lane] = B[input real 4 t + c][output real 8 h + g] for that lane
+    k_hadamard_d64(const double* __restrict__ frag, const double2* __restrict__ in, double2* __restrict__ out,
+                   const int* __restrict__ tab, int ld, const int* __restrict__ rows, int nsrc, int ntrg) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double* sB = reinterpret_cast<double*>(smem_raw);
+  const double* sB = reinterpret_cast<const double*>(smem_raw);
   const int f = blockIdx.y, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  for (int e = tid; e < 26 * 4 * 2 * 32; e += HAD64_NT) {
-    const int ln = e & 31, h = (e >> 5) & 1, c = (e >> 6) & 3, ipos = e >> 8;
-    const int gg = ln >> 2, tt = ln & 3;
-    const int sc = 2 * tt + (c >> 1), ri = c & 1;      // input real 4 tt + c: component sc, re / im
-    const int o = 8 * h + gg, tc = o >> 1, ro = o & 1;  // output real o: component tc, re / im
-    const double2 m = T[((int64_t)ipos * nfreq + f) * 64 + sc * 8 + tc];
-    // output re <- (Re m, -Im m) . (in re, in im); output im <- (Im m, Re m)
-    sB[e] = ro == 0 ? (ri == 0 ? m.x : -m.y) : (ri == 0 ? m.y : m.x);
+  {
+    const uint32_t b0 = tc5::smem_u32(smem_raw);
+    const double* src = frag + (int64_t)f * HAD64_B;
+    for (int e = tid; e < HAD64_B / 2; e += HAD64_NT) tc5::cp_async16(b0 + 16 * e, src + 2 * e, 16u);
+    tc5::cp_async_commit();
   }
-  __syncthreads();
   const int g = lane >> 2, t = lane & 3;
-  const double2* inf = in + (int64_t)f * nsrc * 8 + 2 * t;  // components 2 t, 2 t + 1: reals 4 t .. 4 t + 3
+  const double* inf = reinterpret_cast<const double*>(in + (int64_t)f * nsrc * 8) + 4 * t;
   auto load4 = [&](int sidx) {
-    if (sidx < 0) return make_double4(0.0, 0.0, 0.0, 0.0);
-    const double2 u = __ldg(inf + (int64_t)sidx * 8), v = __ldg(inf + (int64_t)sidx * 8 + 1);
-    return make_double4(u.x, u.y, v.x, v.y);
+    return sidx >= 0 ? ldg_double4(inf + (int64_t)sidx * 16) : make_double4(0.0, 0.0, 0.0, 0.0);
   };
   const int base = blockIdx.x * HAD64_TT + wid * 8 * HAD64_TW + g;  // this lane's target in tile j: base + 8 j
-  double acc[HAD64_TW][2][2];
+  double acc[HAD64_TW][3][2];
   int src[HAD64_TW], srcn[HAD64_TW];
   double4 x[HAD64_TW];
 #pragma unroll
   for (int j = 0; j < HAD64_TW; j++) {
 #pragma unroll
-    for (int h = 0; h < 2; h++) acc[j][h][0] = acc[j][h][1] = 0.0;
+    for (int i = 0; i < 3; i++) acc[j][i][0] = acc[j][i][1] = 0.0;
     src[j] = tab[base + 8 * j];
     srcn[j] = tab[ld + base + 8 * j];
-    x[j] = load4(src[j]);
   }
+#pragma unroll
+  for (int j = 0; j < HAD64_TW; j++) x[j] = load4(src[j]);
+  tc5::cp_async_wait<0>();
+  __syncthreads();
   for (int ipos = 0; ipos < 26; ipos++) {
-    // next position's source pieces, and the position after's source indices
-    double4 xn[HAD64_TW];
-    int srcnn[HAD64_TW];
+    double b[6];
+#pragma unroll
+    for (int i = 0; i < 6; i++) b[i] = sB[(ipos * 6 + i) * 32 + lane];
 #pragma unroll
     for (int j = 0; j < HAD64_TW; j++) {
-      xn[j] = ipos + 1 < 26 ? load4(srcn[j]) : make_double4(0.0, 0.0, 0.0, 0.0);
-      srcnn[j] = ipos + 2 < 26 ? tab[(ipos + 2) * ld + base + 8 * j] : -1;
-    }
-    double b[4][2];
-#pragma unroll
-    for (int c = 0; c < 4; c++)
-#pragma unroll
-      for (int h = 0; h < 2; h++) b[c][h] = sB[((ipos * 4 + c) * 2 + h) * 32 + lane];
-#pragma unroll
-    for (int j = 0; j < HAD64_TW; j++) {
-      if (__ballot_sync(0xffffffffu, src[j] >= 0) == 0u) continue;  // no target of the tile here
-      const double a[4] = {x[j].x, x[j].y, x[j].z, x[j].w};
-#pragma unroll
-      for (int c = 0; c < 4; c++)
-#pragma unroll
-        for (int h = 0; h < 2; h++) dmma_884(acc[j][h], a[c], b[c][h]);
-    }
-#pragma unroll
-    for (int j = 0; j < HAD64_TW; j++) {
+      if (__ballot_sync(0xffffffffu, src[j] >= 0) != 0u) {  // a target of the tile has a source here
+        dmma_884(acc[j][0], x[j].x + x[j].y, b[0]);
+        dmma_884(acc[j][1], x[j].x, b[2]);
+        dmma_884(acc[j][2], x[j].y, b[4]);
+        dmma_884(acc[j][0], x[j].z + x[j].w, b[1]);
+        dmma_884(acc[j][1], x[j].z, b[3]);
+        dmma_884(acc[j][2], x[j].w, b[5]);
+      }
       src[j] = srcn[j];
-      srcn[j] = srcnn[j];
-      x[j] = xn[j];
+      x[j] = load4(src[j]);  // the next position's spectra, the index of the one after
+      srcn[j] = ipos + 2 < 26 ? tab[(ipos + 2) * ld + base + 8 * j] : -1;
     }
   }
   double2* of = out + (int64_t)f * ntrg * 8;
@@ -1401,7 +1414,8 @@ __global__ void __launch_bounds__(HAD64_NT, 2)
     const int row = rows[base + 8 * j];
     if (row < 0) continue;
 #pragma unroll
-    for (int h = 0; h < 2; h++) of[(int64_t)row * 8 + 4 * h + t] = make_double2(acc[j][h][0], acc[j][h][1]);
+    for (int i = 0; i < 2; i++)
+      of[(int64_t)row * 8 + 2 * t + i] = make_double2(acc[j][0][i] - acc[j][2][i], acc[j][0][i] + acc[j][1][i]);
   }
 }
 
@@ -3376,8 +3390,8 @@ struct Engine {
               ws.had64_attr = true;
             }
             k_hadamard_d64<<<dim3(ws.hadd_ld[g] / HAD64_TT, nfreq), HAD64_NT, HAD64_SMEM, s>>>(
-                (const CT*)f.ops[tab_level].m2l_T.p, spec, (CT*)ws.specA.p, ws.hadd_tab.p + ws.hadd_tab0[g], ws.hadd_ld[g],
-                ws.hadd_row.p + ws.hadd_row0[g], ns, nt, nfreq);
+                (const double*)f.ops[tab_level].m2l_frag.p, spec, (CT*)ws.specA.p, ws.hadd_tab.p + ws.hadd_tab0[g], ws.hadd_ld[g],
+                ws.hadd_row.p + ws.hadd_row0[g], ns, nt);
             XLAUNCH();
             ws.launches++;
           }
@@ -3635,7 +3649,13 @@ void check_ready(const Fmm& f, const Tree& t) {
 }  // namespace
 
 // ================================================================ public (internal API)
-void m2l_fragments(LevelOps& op, const double* T64, int nfreq, cudaStream_t s) {
+void m2l_fragments(LevelOps& op, const double* T64, int nfreq, bool mixed, cudaStream_t s) {
+  if (!mixed) {
+    op.m2l_frag.alloc((size_t)nfreq * HAD64_B * sizeof(double));
+    k_m2l_fragments64<<<nblk(26ll * nfreq * 32), 256, 0, s>>>((const double2*)T64, nfreq, (double*)op.m2l_frag.p);
+    XLAUNCH();
+    return;
+  }
   op.m2l_frag.alloc((size_t)nfreq * HADH_FB * sizeof(uint4));
   op.m2l_binv.alloc((size_t)nfreq * 32);
   k_m2l_fragments<<<nblk(26ll * nfreq * 32), 256, 0, s>>>((const double2*)T64, nfreq, (uint4*)op.m2l_frag.p,

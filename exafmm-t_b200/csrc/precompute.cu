@@ -613,13 +613,7 @@ void precompute(Fmm& f, int depth, cudaStream_t s) {
         if (named) dat.m2l[ti] = T64.download(s);
       }
       LevelOps& op = f.ops[l];
-      const int64_t cnt = 26ll * nfreq * 64 * 2;
-      if (single) {
-        m2l_fragments(op, (const double*)T64.p, nfreq, s);
-      } else {
-        op.m2l_T.alloc(cnt * sizeof(double));
-        XCUDA(cudaMemcpyAsync(op.m2l_T.p, T64.p, cnt * sizeof(double), cudaMemcpyDeviceToDevice, s));
-      }
+      m2l_fragments(op, (const double*)T64.p, nfreq, single, s);
     }
     XCUDA(cudaStreamSynchronize(s));
     if (plan) cufftDestroy(plan);

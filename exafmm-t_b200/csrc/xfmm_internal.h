@@ -164,9 +164,8 @@ struct LevelOps {
   DBuf<char> l2p_B1f;  // FP32 copy of l2p_B1 (mixed path, real kernels: the L2P first factor runs in FP32)
   DBuf<char> m2m_B;    // [8n][n]     B[c*n+k][j] = M2M[c][j][k], M2M[c] = (V S+)(U^H K_c)
   DBuf<char> l2l_B;    // [n][8n]     B[k][c*n+j] = M2M[c][k][j] (L2L = M2M^T)
-  // M2L tables, entry [s*8+t] of [26][nfreq][64] complex (fmm_scale_invariant.h:549-551): FP64, or for the
-  // mixed path the Hadamard's FP16 head/tail fragments per frequency (m2l_fragments)
-  DBuf<char> m2l_T;
+  // M2L tables ([26][nfreq][64] complex, entry [s*8+t]; fmm_scale_invariant.h:549-551) as the Hadamard's
+  // fragments per frequency: FP64, or FP16 head / tail for the mixed path (m2l_fragments)
   DBuf<char> m2l_frag;
   DBuf<float> m2l_binv;  // mixed: [nfreq][32], undoes the exponent of each block
   int rank = 0;        // singular values kept by the pinv threshold: B1 columns / B2 rows beyond are zero
@@ -211,7 +210,7 @@ void precompute(Fmm& fmm, int depth, cudaStream_t s);
 void host_surface_base(int p, std::vector<double>& out);
 void host_surface_lines(int p, const std::vector<double>& base, std::vector<int>& perm, std::vector<double>& grid);
 // evaluate.cu
-void m2l_fragments(LevelOps& op, const double* T64, int nfreq, cudaStream_t s);
+void m2l_fragments(LevelOps& op, const double* T64, int nfreq, bool mixed, cudaStream_t s);
 void set_charges(Fmm& fmm, Tree& t, const double* q, bool on_device, cudaStream_t s);
 void clear_values(Fmm& fmm, Tree& t, cudaStream_t s);
 void upward_pass(Fmm& fmm, Tree& t, cudaStream_t s);
