@@ -10,6 +10,11 @@
 #include "xfmm_internal.h"
 
 struct xfmm_fmm {
+  // declared first, so that the operators' memory is released before the hold
+  struct Hold {
+    Hold() { xfmm::pool_hold(); }
+    ~Hold() { xfmm::pool_unhold(); }
+  } hold;
   xfmm::Fmm f;
 };
 struct xfmm_tree {
@@ -102,7 +107,10 @@ xfmm_status xfmm_fmm_set_operator_file(xfmm_fmm* fmm, const char* filename) {
 }
 
 xfmm_status xfmm_fmm_free(xfmm_fmm* fmm) {
-  return guarded([&] { delete fmm; });
+  return guarded([&] {
+    xfmm::PoolQuiet quiet;
+    delete fmm;
+  });
 }
 
 xfmm_status xfmm_fmm_info(const xfmm_fmm* fmm, int64_t* i6, double* d4) {
@@ -144,7 +152,10 @@ xfmm_status xfmm_build_tree(xfmm_fmm* fmm, const double* src_xyz, int64_t nsrc, 
 }
 
 xfmm_status xfmm_tree_free(xfmm_tree* tree) {
-  return guarded([&] { delete tree; });
+  return guarded([&] {
+    xfmm::PoolQuiet quiet;
+    delete tree;
+  });
 }
 
 xfmm_status xfmm_build_list(xfmm_fmm* fmm, xfmm_tree* tree, void* stream) {

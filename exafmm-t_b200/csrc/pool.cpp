@@ -1,0 +1,128 @@
+// pool.cpp -- kept device memory blocks (declared in xfmm_internal.h).
+#include <cuda_runtime.h>
+
+#include <map>
+#include <mutex>
+#include <vector>
+
+#include "xfmm_internal.h"
+
+namespace xfmm {
+namespace {
+
+constexpr size_t POOL_KEEP = (size_t)2 << 30;       // bytes kept per device
+constexpr size_t POOL_MAX_BLOCK = (size_t)512 << 20;  // larger blocks go back to the device at once
+
+struct Kept {
+  std::multimap<size_t, void*> blocks;  // by capacity
+  size_t bytes = 0;
+};
+struct Pool {
+  std::mutex m;
+  std::map<int, Kept> dev;
+  std::map<void*, int> owner;  // device of every block handed out
+  int holds = 0;
+};
+// never destroyed: handles may be freed while the process exits
+Pool& pool() {
+  static Pool* p = new Pool();
+  return *p;
+}
+thread_local int t_quiet = 0;
+thread_local bool t_waited = false;
+
+// capacities in steps of an eighth of a power of two, so that blocks of nearly equal sizes serve each other
+size_t round_up(size_t b) {
+  size_t step = 512;
+  while (step * 16 < b) step *= 2;
+  return (b + step - 1) / step * step;
+}
+void give_back(Kept& k) {
+  for (auto& b : k.blocks) cudaFree(b.second);
+  k.blocks.clear();
+  k.bytes = 0;
+}
+}  // namespace
+
+void* pool_alloc(size_t bytes, size_t* capacity) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+  const size_t want = round_up(bytes);
+  Pool& P = pool();
+  std::lock_guard<std::mutex> lock(P.m);
+  Kept& k = P.dev[dev];
+  auto it = k.blocks.lower_bound(want);
+  if (it != k.blocks.end() && it->first <= want + want / 4) {
+    void* p = it->second;
+    *capacity = it->first;
+    k.bytes -= it->first;
+    k.blocks.erase(it);
+    P.owner[p] = dev;
+    return p;
+  }
+  void* p = nullptr;
+  if (cudaMalloc(&p, want) != cudaSuccess) {
+    cudaGetLastError();
+    give_back(k);
+    if (cudaMalloc(&p, want) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+  }
+  *capacity = want;
+  P.owner[p] = dev;
+  return p;
+}
+
+void pool_release(void* p, size_t capacity) noexcept {
+  Pool& P = pool();
+  int dev = -1, cur = -1;
+  bool keep = false;
+  {
+    std::lock_guard<std::mutex> lock(P.m);
+    auto it = P.owner.find(p);
+    if (it != P.owner.end()) {
+      dev = it->second;
+      P.owner.erase(it);
+    }
+    keep = P.holds > 0 && capacity <= POOL_MAX_BLOCK;
+  }
+  if (keep && cudaGetDevice(&cur) == cudaSuccess && cur == dev) {
+    // no work in flight may still use the block (cudaFree waits in the same way)
+    bool idle = t_quiet > 0 && t_waited;
+    if (!idle) {
+      idle = cudaDeviceSynchronize() == cudaSuccess;
+      t_waited = idle;
+    }
+    if (idle) {
+      std::lock_guard<std::mutex> lock(P.m);
+      Kept& k = P.dev[dev];
+      if (P.holds > 0 && k.bytes + capacity <= POOL_KEEP) {
+        k.blocks.emplace(capacity, p);
+        k.bytes += capacity;
+        return;
+      }
+    }
+  }
+  cudaFree(p);
+}
+
+void pool_hold() {
+  std::lock_guard<std::mutex> lock(pool().m);
+  pool().holds++;
+}
+void pool_unhold() noexcept {
+  Pool& P = pool();
+  std::lock_guard<std::mutex> lock(P.m);
+  if (--P.holds == 0)
+    for (auto& d : P.dev) give_back(d.second);
+}
+
+PoolQuiet::PoolQuiet() noexcept {
+  if (t_quiet++ == 0) t_waited = false;
+}
+PoolQuiet::~PoolQuiet() {
+  if (--t_quiet == 0) t_waited = false;
+}
+
+}  // namespace xfmm

@@ -35,40 +35,60 @@ struct Error : std::exception {
   } while (0)
 #define XLAUNCH() XCUDA(cudaGetLastError())
 
+// Device memory of the buffers below (pool.cpp).  A cudaMalloc or cudaFree takes 50 to 100 us, and a set-up at new
+// positions makes about a hundred of each: blocks that are released while an Fmm handle lives are kept for
+// the next allocations, at most POOL_KEEP bytes per device; the kept blocks go back to the device when the last
+// Fmm handle is freed, and whenever an allocation fails.  As with cudaFree, a release waits for the device
+// (every stream of it), so a kept block has no work left that could touch it; a PoolQuiet scope waits once
+// for all releases made inside it.  Any thread may allocate and release.
+void* pool_alloc(size_t bytes, size_t* capacity);  // null (and the CUDA error) on failure
+void pool_release(void* p, size_t capacity) noexcept;
+void pool_hold();            // an Fmm handle was created
+void pool_unhold() noexcept;  // ... was freed
+struct PoolQuiet {
+  PoolQuiet() noexcept;
+  ~PoolQuiet();
+  PoolQuiet(const PoolQuiet&) = delete;
+  PoolQuiet& operator=(const PoolQuiet&) = delete;
+};
+
 // Owning device buffer (move-only).
 template <class T>
 struct DBuf {
   T* p = nullptr;
-  size_t n = 0;
+  size_t n = 0, cap = 0;  // elements; bytes of the block
   DBuf() = default;
   explicit DBuf(size_t count) { alloc(count); }
   DBuf(const DBuf&) = delete;
   DBuf& operator=(const DBuf&) = delete;
-  DBuf(DBuf&& o) noexcept : p(o.p), n(o.n) { o.p = nullptr; o.n = 0; }
+  DBuf(DBuf&& o) noexcept : p(o.p), n(o.n), cap(o.cap) { o.p = nullptr; o.n = o.cap = 0; }
   DBuf& operator=(DBuf&& o) noexcept {
     if (this != &o) {
       release();
       p = o.p;
       n = o.n;
+      cap = o.cap;
       o.p = nullptr;
-      o.n = 0;
+      o.n = o.cap = 0;
     }
     return *this;
   }
   ~DBuf() { release(); }
   void alloc(size_t count) {
     release();
+    if (!count) return;
+    p = static_cast<T*>(pool_alloc(count * sizeof(T), &cap));
+    if (!p) XCUDA(cudaErrorMemoryAllocation);
     n = count;
-    if (count) XCUDA(cudaMalloc(&p, count * sizeof(T)));
   }
   // grow-only reallocation (contents not preserved)
   void reserve(size_t count) {
     if (count > n) alloc(count);
   }
   void release() {
-    if (p) cudaFree(p);
+    if (p) pool_release(p, cap);
     p = nullptr;
-    n = 0;
+    n = cap = 0;
   }
   size_t bytes() const { return n * sizeof(T); }
   void upload(const T* h, size_t count, cudaStream_t s) {
