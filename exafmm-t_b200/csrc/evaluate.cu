@@ -117,39 +117,35 @@ struct EvalArgs {
   const void* eq;  // working values [nleafs][nsurf]
   double* out;     // tree order, 4 values per target (complex: interleaved)
   double k_re, k_im;
-  int do_near, do_far, accumulate, hilo;
 };
 
 constexpr int EVAL_WARPS = 4;
 
-// R: arithmetic of the pair interactions; W: value type of the upward equivalent densities (M2P
-// sources).  The downward equivalent densities (L2P sources) are FP64 (the pinv output).
+// Far field (M2P + L2P) of the modified Helmholtz and Helmholtz kernels, in FP64, added to the near field's
+// values.  W: value type of the upward equivalent densities (M2P sources); the downward equivalent
+// densities (L2P sources) are FP64 (the pinv output).  A leaf by one warp (PARTS 1) or, with few leaves, by
+// the CTA's PARTS warps, each taking every PARTS-th chunk of 32 surface points, their sums added in order.
 #ifndef XFMM_FAR_NS32
 #define XFMM_FAR_NS32 1  // Newton steps of the FP64 far field when the working precision is FP32
 #endif
-template <int KER, class R, class W>
+template <int KER, class W, int PARTS>
 __global__ void __launch_bounds__(32 * EVAL_WARPS) k_eval(EvalArgs a) {
   // with an FP32 working precision (W), one Newton step on the FP64 reciprocal square root (~2^-44)
-  using G = Green<KER, R, std::is_same<typename Base<W>::type, float>::value ? XFMM_FAR_NS32 : 2>;
+  using G = Green<KER, double, std::is_same<typename Base<W>::type, float>::value ? XFMM_FAR_NS32 : 2>;
   using Q = typename G::Q;
-  using A = typename Acc64<Q>::type;
-  using V4 = typename R4<R>::type;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int w = blockIdx.x * EVAL_WARPS + wid;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, part = PARTS > 1 ? wid : 0;
+  const int w = PARTS > 1 ? (int)blockIdx.x : blockIdx.x * EVAL_WARPS + wid;
   if (w >= a.n_eval) return;
-  __shared__ V4 s_xyz[EVAL_WARPS][32];
-  __shared__ V4 s_lo[EVAL_WARPS][32];  // FP32: low parts of the leaf-relative coordinates
+  __shared__ double4 s_xyz[EVAL_WARPS][32];
   __shared__ Q s_q[EVAL_WARPS][32];
-  constexpr bool HILO = sizeof(R) == 4;
-  const G g{(R)a.k_re, (R)a.k_im};
+  const G g{a.k_re, a.k_im};
   const int pos = a.eval_leafs[w];
   const int node = a.leafs[pos];
-  const int T = a.ntrgs[node];
+  const int T = a.ntrgs[node], n = a.nsurf;
   const int64_t tb = a.tbeg[node];
   const double4 c = a.center[node];
-  using Q64 = typename Acc64<Q>::type;
   const W* upv = (const W*)a.up;
-  const Q64* eqv = (const Q64*)a.eq;
+  const Q* eqv = (const Q*)a.eq;
   for (int t0 = 0, Tc = 0; t0 < T; t0 += Tc) {
     // blocks of 32 targets, the last 17..32 as 16 + the rest, so that the split of the sources over
     // 2..32 lanes per target keeps the lanes busy
@@ -158,111 +154,81 @@ __global__ void __launch_bounds__(32 * EVAL_WARPS) k_eval(EvalArgs a) {
     while (G2 * 2 * Tc <= 32) G2 *= 2;
     const int tl = lane / G2, sub = lane % G2;
     const bool active = tl < Tc;
-    // leaf-relative target coordinates; in FP32 as hi + lo so that differences keep ~FP32
-    // relative accuracy of the separation itself (not of the leaf size)
-    R tx = 0, ty = 0, tz = 0, lx = 0, ly = 0, lz = 0;
+    double tx = 0, ty = 0, tz = 0;
     if (active) {
       const double4 t = a.trg4[tb + t0 + tl];
-      const double dx = t.x - c.x, dy = t.y - c.y, dz = t.z - c.z;
-      tx = (R)dx;
-      ty = (R)dy;
-      tz = (R)dz;
-      lx = (R)(dx - (double)tx);
-      ly = (R)(dy - (double)ty);
-      lz = (R)(dz - (double)tz);
+      tx = t.x - c.x;
+      ty = t.y - c.y;
+      tz = t.z - c.z;
     }
-    A P, GX, GY, GZ;
-    P = GX = GY = GZ = A();
-    // one staged chunk of <= 32 sources: lanes accumulate their share, then FP64 accumulation
-    auto consume = [&](int cnt) {
-      __syncwarp();
-      Q p = vzero<Q>(), gx = vzero<Q>(), gy = vzero<Q>(), gz = vzero<Q>();
-      if (active) {
-        if (HILO && a.hilo) {
-          for (int j = sub; j < cnt; j += G2) {
-            const V4 s = s_xyz[wid][j], sl = s_lo[wid][j];
-            g.grad((tx - s.x) + (lx - sl.x), (ty - s.y) + (ly - sl.y), (tz - s.z) + (lz - sl.z), s_q[wid][j], p, gx,
-                   gy, gz);
-          }
-        } else {
-          for (int j = sub; j < cnt; j += G2) {
-            const V4 s = s_xyz[wid][j];
-            g.grad(tx - s.x, ty - s.y, tz - s.z, s_q[wid][j], p, gx, gy, gz);
-          }
-        }
-      }
-      acc64(P, p);
-      acc64(GX, gx);
-      acc64(GY, gy);
-      acc64(GZ, gz);
-      __syncwarp();
-    };
-    if (a.do_near) {
-      for (int64_t e = a.p2p_off[node]; e < a.p2p_off[node + 1]; e++) {
-        const int s = a.p2p[e];
-        const int ns = a.nsrcs[s];
-        const int64_t sb = a.sbeg[s];
-        for (int j0 = 0; j0 < ns; j0 += 32) {
-          const int cnt = min(32, ns - j0);
-          if (lane < cnt) {
-            const double4 sv = a.src4[sb + j0 + lane];
-            const double dx = sv.x - c.x, dy = sv.y - c.y, dz = sv.z - c.z;
-            const R hx = (R)dx, hy = (R)dy, hz = (R)dz;
-            s_xyz[wid][lane] = V4{hx, hy, hz, (R)0};
-            s_lo[wid][lane] = V4{(R)(dx - (double)hx), (R)(dy - (double)hy), (R)(dz - (double)hz), (R)0};
-            s_q[wid][lane] = load_charge<Q>(sv, a.src_qim, sb + j0 + lane);
-          }
-          consume(cnt);
-        }
-      }
-    }
-    if (a.do_far) {
-      const int n = a.nsurf;
-      // M2P: W-list nodes' upward equivalent surfaces (1.05 box, fmm_base.h:103-121)
-      for (int64_t e = a.m2p_off[node]; e < a.m2p_off[node + 1]; e++) {
-        const int s = a.m2p[e];
-        const double4 cs = a.center[s];
-        const double b = 1.05 * cs.w;
-        for (int j0 = 0; j0 < n; j0 += 32) {
-          const int cnt = min(32, n - j0);
-          if (lane < cnt) {
-            const int k = j0 + lane;
-            s_xyz[wid][lane] = V4{(R)(cs.x + a.surf_base[3 * k] * b - c.x), (R)(cs.y + a.surf_base[3 * k + 1] * b - c.y),
-                                  (R)(cs.z + a.surf_base[3 * k + 2] * b - c.z), (R)0};
-            s_lo[wid][lane] = V4{(R)0, (R)0, (R)0, (R)0};
-            s_q[wid][lane] = cvt<Q>(upv[(int64_t)s * n + k]);
-          }
-          consume(cnt);
-        }
-      }
-      // L2P: own downward equivalent surface (2.95 box, fmm_scale_invariant.h:221-228)
-      const double b = 2.95 * c.w;
+    Q P = vzero<Q>(), GX = vzero<Q>(), GY = vzero<Q>(), GZ = vzero<Q>();
+    int chunk = 0;
+    // one surface of half size b at offset (ox, oy, oz) from the leaf's centre: den(k) its densities
+    auto surface = [&](double ox, double oy, double oz, double b, auto&& den) {
       for (int j0 = 0; j0 < n; j0 += 32) {
-        const int cnt = min(32, n - j0);
+        if (PARTS > 1 && (chunk++) % PARTS != part) continue;
+        const int cnt = min(32, n - j0), k = j0 + lane;
+        __syncwarp();
         if (lane < cnt) {
-          const int k = j0 + lane;
-          s_xyz[wid][lane] = V4{(R)(a.surf_base[3 * k] * b), (R)(a.surf_base[3 * k + 1] * b),
-                                (R)(a.surf_base[3 * k + 2] * b), (R)0};
-          s_lo[wid][lane] = V4{(R)0, (R)0, (R)0, (R)0};
-          s_q[wid][lane] = cvt<Q>(eqv[(int64_t)pos * n + k]);
+          s_xyz[wid][lane] = make_double4(ox + a.surf_base[3 * k] * b, oy + a.surf_base[3 * k + 1] * b,
+                                          oz + a.surf_base[3 * k + 2] * b, 0.0);
+          s_q[wid][lane] = den(k);
         }
-        consume(cnt);
+        __syncwarp();
+        if (!active) continue;
+        Q p = vzero<Q>(), gx = vzero<Q>(), gy = vzero<Q>(), gz = vzero<Q>();  // the chunk's sums
+        for (int j = sub; j < cnt; j += G2) {
+          const double4 s = s_xyz[wid][j];
+          g.grad(tx - s.x, ty - s.y, tz - s.z, s_q[wid][j], p, gx, gy, gz);
+        }
+        P = vadd(P, p);
+        GX = vadd(GX, gx);
+        GY = vadd(GY, gy);
+        GZ = vadd(GZ, gz);
       }
+    };
+    // M2P: W-list nodes' upward equivalent surfaces (1.05 box, fmm_base.h:103-121)
+    for (int64_t e = a.m2p_off[node]; e < a.m2p_off[node + 1]; e++) {
+      const int s = a.m2p[e];
+      const double4 cs = a.center[s];
+      surface(cs.x - c.x, cs.y - c.y, cs.z - c.z, 1.05 * cs.w, [&](int k) { return cvt<Q>(upv[(int64_t)s * n + k]); });
     }
+    // L2P: own downward equivalent surface (2.95 box, fmm_scale_invariant.h:221-228)
+    surface(0.0, 0.0, 0.0, 2.95 * c.w, [&](int k) { return eqv[(int64_t)pos * n + k]; });
     for (int o = 1; o < G2; o <<= 1) {
       P = vadd(P, shfl_x(P, o));
       GX = vadd(GX, shfl_x(GX, o));
       GY = vadd(GY, shfl_x(GY, o));
       GZ = vadd(GZ, shfl_x(GZ, o));
     }
-    if (active && sub == 0) {
+    if constexpr (PARTS > 1) {
+      __shared__ Q red[PARTS - 1][4][32];
+      if (part > 0) {
+        red[part - 1][0][lane] = P;
+        red[part - 1][1][lane] = GX;
+        red[part - 1][2][lane] = GY;
+        red[part - 1][3][lane] = GZ;
+      }
+      __syncthreads();
+      if (part == 0) {
+#pragma unroll
+        for (int k = 0; k < PARTS - 1; k++) {
+          P = vadd(P, red[k][0][lane]);
+          GX = vadd(GX, red[k][1][lane]);
+          GY = vadd(GY, red[k][2][lane]);
+          GZ = vadd(GZ, red[k][3][lane]);
+        }
+      }
+      __syncthreads();
+    }
+    if (active && sub == 0 && part == 0) {
       const int stride = (KER == K_HELMHOLTZ) ? 8 : 4;
       double* o = a.out + (tb + t0 + tl) * stride;
       const int vs = stride / 4;
-      put_out(o, P, INV4PI, a.accumulate);
-      put_out(o + vs, GX, INV4PI, a.accumulate);
-      put_out(o + 2 * vs, GY, INV4PI, a.accumulate);
-      put_out(o + 3 * vs, GZ, INV4PI, a.accumulate);
+      put_out(o, P, INV4PI, 1);
+      put_out(o + vs, GX, INV4PI, 1);
+      put_out(o + 2 * vs, GY, INV4PI, 1);
+      put_out(o + 3 * vs, GZ, INV4PI, 1);
     }
   }
 }
@@ -3528,14 +3494,11 @@ struct Engine {
 
   // the far field (M2P + L2P evaluation), added to the near field's values
   static EvalArgs far_args(Fmm& f, Tree& t, Workspace& ws) {
-    EvalArgs a{t.eval_leafs.p, t.leafs.p, t.nsrcs.p,   t.ntrgs.p, t.level.p, t.n_eval_leafs, t.sbeg.p,
+    return EvalArgs{t.eval_leafs.p, t.leafs.p, t.nsrcs.p,   t.ntrgs.p, t.level.p, t.n_eval_leafs, t.sbeg.p,
                t.tbeg.p,       t.center.p, t.src4.p,   t.trg4.p,  t.src_qim.p, t.p2p_off.p,  t.m2p_off.p,
                t.p2p.p,        t.m2p.p,   f.surf_base.p, f.surf_perm.p, f.surf_grid.p, f.nsurf, ws.up.p,
                ws.eq.p,        ws.out.p,
-               f.k_re,         f.k_im,    1,           1,         0,         1};
-    a.do_near = 0;
-    a.accumulate = 1;
-    return a;
+               f.k_re,         f.k_im};
   }
 
   static NearArgs near_args(Fmm& f, Tree& t, Workspace& ws) {
@@ -3583,7 +3546,8 @@ struct Engine {
             k_far_lap<W, PP, 1><<<blocks, 32 * EVAL_WARPS, smem, s>>>(a);
         });
       } else {
-        k_eval<KER, double, W><<<blocks, 32 * EVAL_WARPS, 0, s>>>(a);
+        if (t.n_eval_leafs < SPLIT_LEAVES) k_eval<KER, W, EVAL_WARPS><<<t.n_eval_leafs, 32 * EVAL_WARPS, 0, s>>>(a);
+        else k_eval<KER, W, 1><<<blocks, 32 * EVAL_WARPS, 0, s>>>(a);
       }
       XLAUNCH();
       ws.launches++;
