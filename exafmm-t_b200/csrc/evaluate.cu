@@ -468,8 +468,8 @@ void order_dispatch(int p, F&& fn) {
 }
 // Leaves below which several warps share one (FAR_PARTS, NEAR_PARTS, the surfaces of P2M and P2L): 64 per SM, two
 // to three times the warps resident at once.  Near field: 1.5k leaves (Plummer 20k, FP64) 0.49 -> 0.15 ms, 8.4k
-// (Plummer 300k, mixed) 0.62 -> 0.29, 4.6k even leaves (Helmholtz 200k) 0.77 -> 0.70; with 14k (Yukawa
-// sphere 300k) sharing cost more than it evened out, 0.305 -> 0.340.
+// (Plummer 300k, mixed) 0.62 -> 0.29, 4.6k even leaves (Helmholtz 200k) 0.77 -> 0.70, 4.1k even leaves
+// (Laplace 100k, FP64) 0.21 -> 0.20: the gain is gone where every SM has several rounds of leaves.
 constexpr int SPLIT_LEAVES = 148 * 64;
 
 // ================================================================ near field (P2P)
@@ -511,8 +511,9 @@ struct NearSmem {
   int seg_pre[NEAR_SEG + 1];
 };
 
-// PARTS 1: the whole leaf, or its parts one after another (a.parts); NEAR_PARTS: part `part` of a leaf shared by
-// the warps of the CTA, all of which call this
+// PARTS 0: the whole leaf in one pass (systems of one part); 1: its parts one after another (a.parts; the sums kept
+// beside the running ones cost registers: Yukawa sphere 300k 0.305 -> 0.340 ms); NEAR_PARTS: part `part` of a
+// leaf shared by the warps of the CTA, all of which call this
 template <int KER, class R, int TPL, int PARTS = 1>
 __device__ __forceinline__ void near_leaf(const NearArgs& a, int node, int lane, NearSmem<R>& sm, int part = 0) {
   using G = Green<KER, R>;
@@ -534,7 +535,7 @@ __device__ __forceinline__ void near_leaf(const NearArgs& a, int node, int lane,
   for (int t0 = 0; t0 < T; t0 += 32 * TPL) {
     R tx[TPL], ty[TPL], tz[TPL], lx[TPL], ly[TPL], lz[TPL];
     A P[TPL], GX[TPL], GY[TPL], GZ[TPL];
-    const int np = a.parts, k0 = PARTS > 1 ? part : 0, k1 = PARTS > 1 ? part + 1 : np;
+    const int np = PARTS == 1 ? a.parts : PARTS > 1 ? PARTS : 1, k0 = PARTS > 1 ? part : 0, k1 = PARTS > 1 ? part + 1 : np;
     A SP[TPL], SX[TPL], SY[TPL], SZ[TPL];  // sums of the parts before
 #pragma unroll
     for (int u = 0; u < TPL; u++) {
@@ -1037,13 +1038,13 @@ __global__ void __launch_bounds__(128, XFMM_NEAR_MINB) k_near(NearArgs a) {
   const int node = a.leafs[a.eval_leafs[w]];
   const int T = a.ntrgs[node];
   if constexpr (sizeof(R) == 4) {
-    if (T <= 32 || XFMM_NEAR_MAXTPL == 1) near_leaf<KER, R, 1>(a, node, lane, sm[wid]);
-    else if (T <= 64 || XFMM_NEAR_MAXTPL == 2) near_leaf<KER, R, (XFMM_NEAR_MAXTPL >= 2 ? 2 : 1)>(a, node, lane, sm[wid]);
-    else if (T <= 96 || XFMM_NEAR_MAXTPL == 3) near_leaf<KER, R, (XFMM_NEAR_MAXTPL >= 3 ? 3 : 1)>(a, node, lane, sm[wid]);
-    else near_leaf<KER, R, (XFMM_NEAR_MAXTPL >= 4 ? 4 : 1)>(a, node, lane, sm[wid]);
+    if (T <= 32 || XFMM_NEAR_MAXTPL == 1) near_leaf<KER, R, 1, 0>(a, node, lane, sm[wid]);
+    else if (T <= 64 || XFMM_NEAR_MAXTPL == 2) near_leaf<KER, R, (XFMM_NEAR_MAXTPL >= 2 ? 2 : 1), 0>(a, node, lane, sm[wid]);
+    else if (T <= 96 || XFMM_NEAR_MAXTPL == 3) near_leaf<KER, R, (XFMM_NEAR_MAXTPL >= 3 ? 3 : 1), 0>(a, node, lane, sm[wid]);
+    else near_leaf<KER, R, (XFMM_NEAR_MAXTPL >= 4 ? 4 : 1), 0>(a, node, lane, sm[wid]);
   } else {
     // FP64: one target per lane keeps occupancy up (two per lane: 134 registers, 27.6 -> 31.3 ms at 4M)
-    near_leaf<KER, R, 1>(a, node, lane, sm[wid]);
+    near_leaf<KER, R, 1, 0>(a, node, lane, sm[wid]);
   }
 }
 
