@@ -1390,14 +1390,17 @@ __global__ void __launch_bounds__(HAD64_NT, 2)
 // frequency-major, (frequency f, node, child c) at [(f * nrows + node) * 8 + c]: a CTA (one frequency)
 // reads its sources from one block of the spectra and writes its rows contiguously.
 //
-// The mixed path's spectra are stored split: a real x of source node s is the pair of FP16 values
-// h = fp16(2^e x), t = fp16(2^e x - h), with one exponent e per source node (all its children and
-// frequencies), so that 22 bits of x survive as long as |x| is within 2^-17 of the node's bound and the
-// absolute error stays below 2^-39 of that bound elsewhere.  A split spectrum has the size of the FP32
-// one, the products need no conversion (the operator's blocks are split the same way, one exponent per
-// position and frequency), and an FP16 MMA does twice the work of a TF32 one in the same 8 cycles
-// (measured: m16n8k16 f16 and m16n8k8 tf32 both 8.0 cycles per warp and SM quadrant) with the same
-// 11-bit significands.  A child's complex value is the 8 bytes {h.re, h.im, t.re, t.im}.
+// The mixed path's spectra are stored split: a real x of a child's spectrum is the pair of FP16 values
+// h = fp16(2^e x), t = fp16(2^e x - h): 22 bits of x within 2^-17 of the top (2^15), an absolute error below
+// 2^-39 of it elsewhere.  Every spectrum value of a child is at most the sum of its densities' magnitudes,
+// its bound.  A source node has one exponent e, set by its strongest child; a child whose bound is more than
+// 2^-18 below goes to the next window of the node, with the exponent e + 18, and so on, so that every child
+// keeps an error below 2^-21 of its own bound however strong its siblings are (a screened kernel shows a
+// weak source: the strong one's field is gone where its own targets are).  A split spectrum has the size of
+// the FP32 one, the products need no conversion (the operator's blocks are split the same way,
+// k_m2l_fragments), and an FP16 MMA does twice the work of a TF32 one in the same 8 cycles (measured:
+// m16n8k16 f16 and m16n8k8 tf32 both 8.0 cycles per warp and SM quadrant) with the same 11-bit significands.
+// A child's complex value is the 8 bytes {h.re, h.im, t.re, t.im}.
 using SplitC = uint2;
 __device__ __forceinline__ uint32_t h2_bits(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
 __device__ __forceinline__ float2 h2_float2(uint32_t u) { return __half22float2(*reinterpret_cast<__half2*>(&u)); }
@@ -1415,11 +1418,21 @@ __device__ __forceinline__ int split_code(float bound) {
   if (!(e & 1)) e -= 1;
   return (127 - e) >> 1;
 }
-__device__ __forceinline__ float split_scale(int code) { return __uint_as_float((uint32_t)(254 - 2 * code) << 23); }
+constexpr int SPLIT_WIN = 9;   // steps of 2 bits between the windows of a node's children and of the operator's pairs
+constexpr int SPLIT_PASS = 10;  // steps that one pass over a tile covers: 2^-18 from its strongest source to its weakest
+constexpr int SPLIT_DEEP = 0x100, SPLIT_ZERO = 0x200;  // beside a source's code: a child beyond window 0; no values
+__device__ __forceinline__ float pow2f(int e) { return e >= -126 ? __uint_as_float((uint32_t)(127 + e) << 23) : 0.f; }
+__device__ __forceinline__ float split_scale(int code, int w) { return pow2f(127 - 2 * (code - SPLIT_WIN * w)); }
+// the window of a child with bound c of a node with bound b, whose scale is still a float
+__device__ __forceinline__ int split_window(float c, float b, int code) {
+  if (!(c > 0.f)) return 0;
+  const int below = (int)(__float_as_uint(b) >> 23) - (int)(__float_as_uint(c) >> 23);
+  return min(max(0, below) / (2 * SPLIT_WIN), (code - 1) / SPLIT_WIN);
+}
 // Packed sources: the source row in the low 25 bits (2^25 sources would need 206 GB of spectra at the lowest
 // order) and 7 bits of exponent: in the opt-in tcgen05 form's table the source's code (written by
 // k_pack_sources after every forward transform), in a tile's slot list the source's distance from the tile's
-// common exponent (k_tile_codes).  SPLIT_NONE: no source.
+// largest code in steps (k_tile_codes).  SPLIT_NONE: no source.
 constexpr int SPLIT_ROW_BITS = 25;
 constexpr uint32_t SPLIT_ROW_MASK = (1u << SPLIT_ROW_BITS) - 1;
 constexpr uint32_t SPLIT_NONE = 0xffffffffu;
@@ -1428,7 +1441,7 @@ __device__ __forceinline__ float split_inv_code(int code) { return __uint_as_flo
 __global__ void k_pack_sources(const int* __restrict__ in, int64_t n, const int* __restrict__ scode,
                                uint32_t* __restrict__ out) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    out[i] = in[i] >= 0 ? (uint32_t)in[i] | ((uint32_t)scode[in[i]] << SPLIT_ROW_BITS) : SPLIT_NONE;
+    out[i] = in[i] >= 0 ? (uint32_t)in[i] | ((uint32_t)(scode[in[i]] & 0x7f) << SPLIT_ROW_BITS) : SPLIT_NONE;
 }
 
 // opt-in tcgen05 form (k_hadamard_dc): occupied positions that make a target dense, dense targets a group
@@ -1447,7 +1460,7 @@ constexpr int HADC_TT = 512;  // padding of its source table
 //
 // A CTA owns a tile of up to 512 targets at one frequency.  The tile's distinct sources (up to 1016, about
 // twice the targets of a spatially compact tile, each used by up to 26 of them) are brought into shared
-// memory once, on a common exponent, and every A fragment is read from there with ldmatrix, whose lanes
+// memory once, on the exponent of the strongest, and every A fragment is read from there with ldmatrix, whose lanes
 // address the rows of a fragment freely: a gather without register moves at 8 shared-memory cycles per 16
 // targets and position.  Measured, Hadamard stage: 1M bodies, p = 10: 2.95 ms (the same products gathered
 // row by row from L1 at 14 cycles per 16 targets: 4.03; the TF32 form with per-use conversions before it:
@@ -1457,6 +1470,10 @@ constexpr int HADC_TT = 512;  // padding of its source table
 // targets at one relative position have 8 different octants, so their 64-byte rows (four 16-byte chunks,
 // swizzled by (slot / 2) % 4) fall on different banks; empty positions read one of 8 zero slots, chosen to
 // stay off the banks of the other rows.
+// A tile whose children lie within 2^-18 of its strongest has one pass: all tiles of cubes, Plummer spheres and
+// surfaces of up to 4M bodies with charges in (-1, 1) (2 to 9 steps of 2 bits).  Otherwise pass w takes the
+// children 10 w .. 10 w + 9 steps below, the others at zero, over the same accumulators: weak sources keep their 22
+// bits.  The same for the windows of the operator.
 // Tiles with at most 256, 128 or 64 targets split the 26 positions over 2, 4 or 8 warps per 64 targets.
 // Bounds per 64 targets and position and SM (cycles): MMAs 24 x 8 / 4 = 48; shared memory 32 (A) + 8 (B).
 // At 1M, p = 8 the tensor pipe is 54% and the shared-memory pipe 64% busy: 16 warps per SM hide the rest of
@@ -1469,6 +1486,7 @@ constexpr int HADH_B = 26 * 2 * 32;              // B fragments (uint4) in share
 constexpr int HADH_FB = HADH_B / 2;              // and as stored
 constexpr size_t HADH_SMEM = (size_t)HADH_SLOTS * 64 + (size_t)HADH_B * 16 + 32 * sizeof(float);
 static_assert(2 * (HADH_SMEM + 1024) <= 228 * 1024, "two CTAs per SM");
+constexpr uint32_t TILE_DEEP = 1u << 31;
 struct HadTile {
   int nslots;   // slots used (a multiple of 8, the zero slots included)
   int groups;   // 1, 2, 4 or 8 groups of 64 targets
@@ -1482,6 +1500,8 @@ struct HadSys {
   const HadTile* tiles;
   const uint32_t* slots;  // packed source of each slot (k_tile_codes)
   const float* tinv;      // per tile: undoes its exponent
+  const uint32_t* tpass;  // per tile: bit w: pass w has sources; TILE_DEEP: children beyond window 0
+  const uint8_t* win;     // window of every source's children
   const uint2* tab;
   const int* rows;
   int nsrc, ntrg;
@@ -1511,49 +1531,72 @@ __device__ __forceinline__ void tf32_split(float x, uint32_t& h, uint32_t& t) {
 // FP64 values: for every (position, output half h, lane) of a warp the four registers {b0 head, b1 head,
 // b0 tail, b1 tail}, scaled by the block's exponent; b0 / b1 are the factors of source components t / t + 4
 // and half h the target components 4 h .. 4 h + 3 (t = lane % 4).  Stored are the lanes of even g = lane / 4
-// (real outputs: (Re, -Im) of a factor), at frag[f * HADH_FB + (ipos * 2 + h) * 16 + 4 (g / 2) + t]; those of
-// g + 1 (imaginary outputs: (Im, Re)) are the same values swapped (hadh_odd).  inv[f * 32 + ipos] undoes the
-// exponent.  One warp per block.
-__global__ void k_m2l_fragments(const double2* __restrict__ T, int nfreq, uint4* __restrict__ frag,
-                                float* __restrict__ inv) {
+// (real outputs: (Re, -Im) of a factor), at frag[(v * nfreq + f) * HADH_FB + (ipos * 2 + h) * 16 + 4 (g / 2) + t];
+// those of g + 1 (imaginary outputs: (Im, Re)) are the same values swapped (hadh_odd).
+// inv[(v * nfreq + f) * 32 + ipos] undoes the exponent.  One warp per block.
+// v: the operator's window.  The factors of a screened kernel's child pairs differ by e^(-k (distance)): a
+// pair whose largest factor over the frequencies (k_pair_max) is more than 2^-18 below the largest of its
+// position goes to the next window, with an exponent of its own, as the sources' children do; pwin[ipos * 64 + pair]
+// is the pair's window.  One window for Laplace and for Helmholtz with a real wavenumber; modified Helmholtz takes a
+// second from k (box size) of about 4.6 on.
+__global__ void __launch_bounds__(256)
+    k_pair_max(const double2* __restrict__ T, int nfreq, unsigned* __restrict__ pmax) {
+  const int pair = threadIdx.x & 63, ipos = blockIdx.y;
+  float m = 0.f;
+  for (int f = blockIdx.x * 4 + (threadIdx.x >> 6); f < nfreq; f += gridDim.x * 4) {
+    const double2 q = T[((int64_t)ipos * nfreq + f) * 64 + pair];
+    m = fmaxf(m, (float)fmax(fabs(q.x), fabs(q.y)));
+  }
+  atomicMax(pmax + ipos * 64 + pair, __float_as_uint(m));
+}
+__global__ void k_m2l_fragments(const double2* __restrict__ T, int nfreq, const uint8_t* __restrict__ pwin,
+                                uint4* __restrict__ frag, float* __restrict__ inv) {
   const int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, win = blockIdx.y;
   if (w >= 26ll * nfreq) return;
   const int f = (int)(w / 26), ipos = (int)(w % 26);
   const double2* blk = T + ((int64_t)ipos * nfreq + f) * 64;
-  const double2 u = blk[lane], v = blk[32 + lane];
+  auto entry = [&](int pair) { return pwin[ipos * 64 + pair] == win ? blk[pair] : make_double2(0.0, 0.0); };
+  const double2 u = entry(lane), v = entry(32 + lane);
   float m = (float)fmax(fmax(fabs(u.x), fabs(u.y)), fmax(fabs(v.x), fabs(v.y)));
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
   const int code = split_code(m);
-  const double sc = (double)split_scale(code);
+  const double sc = (double)split_scale(code, 0);
   const int h = lane >> 4, tc = 4 * h + ((lane >> 2) & 3), t = lane & 3;
   uint32_t hd[2], tl[2];
 #pragma unroll
   for (int c = 0; c < 2; c++) {
-    const double2 q = blk[(t + 4 * c) * 8 + tc];
+    const double2 q = entry((t + 4 * c) * 8 + tc);
     const double re = q.x * sc, im = -q.y * sc;
     const __half2 hh = __halves2half2(__double2half(re), __double2half(im));
     const float2 hf = __half22float2(hh);
     hd[c] = h2_bits(hh);
     tl[c] = h2_bits(__halves2half2(__double2half(re - hf.x), __double2half(im - hf.y)));
   }
-  frag[(int64_t)f * HADH_FB + ipos * 32 + lane] = make_uint4(hd[0], hd[1], tl[0], tl[1]);
-  if (lane == 0) inv[(int64_t)f * 32 + ipos] = split_inv_code(code);
+  const int64_t row = (int64_t)win * nfreq + f;
+  frag[row * HADH_FB + ipos * 32 + lane] = make_uint4(hd[0], hd[1], tl[0], tl[1]);
+  if (lane == 0) inv[row * 32 + ipos] = split_inv_code(code);
 }
 // the registers of lane g + 1 from those of an even g: (Re, -Im) -> (Im, Re) in every half pair
 __device__ __forceinline__ uint4 hadh_odd(const uint4& e) {
   auto sw = [](uint32_t v) { return __byte_perm(v, v, 0x1032) ^ 0x8000u; };
   return make_uint4(sw(e.x), sw(e.y), sw(e.z), sw(e.w));
 }
-// After a forward transform, per tile (one CTA each): the largest exponent code of its sources, the common
-// exponent, and the slot list packed with every source's distance d from it (SPLIT_NONE: no source).
+// After a forward transform, per tile (one CTA each): the largest exponent code of its sources, whose exponent is
+// the tile's, the slot list packed with every source's distance d from it (SPLIT_NONE: no source, or one
+// without values), and the passes that the tile needs.
 __global__ void __launch_bounds__(256)
     k_tile_codes(const HadTile* __restrict__ tiles, const int* __restrict__ slots, const int* __restrict__ scode,
-                 uint32_t* __restrict__ pslots, float* __restrict__ tinv) {
+                 const uint8_t* __restrict__ win, uint32_t* __restrict__ pslots, float* __restrict__ tinv,
+                 uint32_t* __restrict__ tpass) {
   __shared__ int smax;
+  __shared__ uint32_t spass;
   const HadTile T = tiles[blockIdx.x];
-  if (threadIdx.x == 0) smax = 1;
+  if (threadIdx.x == 0) {
+    smax = 1;
+    spass = 1u;
+  }
   __syncthreads();
   int src[(HADH_SLOTS + 255) / 256], code[(HADH_SLOTS + 255) / 256], kmax = 1;
 #pragma unroll
@@ -1561,18 +1604,33 @@ __global__ void __launch_bounds__(256)
     const int q = threadIdx.x + 256 * i;
     src[i] = q < T.nslots ? slots[T.slot0 + q] : -1;
     code[i] = src[i] >= 0 ? scode[src[i]] : 0;
-    kmax = max(kmax, code[i]);
+    if (code[i] & SPLIT_ZERO) src[i] = -1;
+    if (src[i] >= 0) kmax = max(kmax, code[i] & 0x7f);
   }
   atomicMax(&smax, __reduce_max_sync(0xffffffffu, kmax));
   __syncthreads();
   kmax = smax;
+  uint32_t pass = 0u;
 #pragma unroll
   for (int i = 0; i < (HADH_SLOTS + 255) / 256; i++) {
-    const int q = threadIdx.x + 256 * i;
+    const int q = threadIdx.x + 256 * i, d = kmax - (code[i] & 0x7f);
     if (q < T.nslots)
-      pslots[T.slot0 + q] = src[i] >= 0 ? (uint32_t)src[i] | (uint32_t)(kmax - code[i]) << SPLIT_ROW_BITS : SPLIT_NONE;
+      pslots[T.slot0 + q] = src[i] >= 0 ? (uint32_t)src[i] | (uint32_t)d << SPLIT_ROW_BITS : SPLIT_NONE;
+    if (src[i] < 0) continue;
+    if (code[i] & SPLIT_DEEP) {
+      pass |= TILE_DEEP;
+      for (int c = 0; c < 8; c++) pass |= 1u << ((d + SPLIT_WIN * win[(int64_t)src[i] * 8 + c]) / SPLIT_PASS);
+    } else {
+      pass |= 1u << (d / SPLIT_PASS);
+    }
   }
-  if (threadIdx.x == 0) tinv[blockIdx.x] = split_inv_code(kmax);
+  pass = __reduce_or_sync(0xffffffffu, pass);
+  if ((threadIdx.x & 31) == 0) atomicOr(&spass, pass);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    tinv[blockIdx.x] = split_inv_code(kmax);
+    tpass[blockIdx.x] = spass;
+  }
 }
 
 __device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t (&r)[4]) {
@@ -1584,11 +1642,11 @@ __device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t (&r)[4]) {
 // Table entry of a slot: 4 slot + swizzle; chunk c of the slot is at 16 (entry ^ c).
 __host__ __device__ __forceinline__ uint32_t hadh_entry(int slot) { return (uint32_t)(4 * slot + ((slot >> 1) & 3)); }
 
-// one tile at frequency f; its first tile also stores the CTA's B fragments and block scales (frag, binv: those
-// of f) into shared memory
+// one tile at frequency f; with `fill` it also brings the frequency's B fragments and block scales (frag, binv: those
+// of f; bstride frequencies between the operator's nbw windows) into shared memory
 __device__ __forceinline__ void hadh_tile(const HadSys& S, int tile, int f, unsigned char* sA, uint4* sB, float* sInv,
-                                          const uint4* __restrict__ frag, const float* __restrict__ binv, bool first,
-                                          int tid) {
+                                          const uint4* __restrict__ frag, const float* __restrict__ binv, int nbw,
+                                          int bstride, bool fill, int tid) {
   const HadTile T = S.tiles[tile];
   const int lane = tid & 31, wid = tid >> 5;
   // ---- the tile's sources: four threads per slot, 16 bytes each
@@ -1597,43 +1655,14 @@ __device__ __forceinline__ void hadh_tile(const HadSys& S, int tile, int f, unsi
   constexpr int QS = HADH_NT / 4, NB = (HADH_SLOTS + QS - 1) / QS;  // slots per round; rounds, all in flight
   const int c = tid & 3;
   constexpr int NF = (HADH_FB + HADH_NT - 1) / HADH_NT;
-  uint4 fb[NF];
-  if (first) {
-#pragma unroll
-    for (int i = 0; i < NF; i++) fb[i] = __ldg(frag + min(tid + HADH_NT * i, HADH_FB - 1));
-  }
-  uint32_t src[NB];
-#pragma unroll
-  for (int i = 0; i < NB; i++) {
-    const int q = (tid >> 2) + QS * i;
-    src[i] = q < T.nslots ? slots[q] : SPLIT_NONE;
-  }
-  uint4 v[NB];
-#pragma unroll
-  for (int i = 0; i < NB; i++) {
-    const uint32_t e = src[i];
-    v[i] = e != SPLIT_NONE ? __ldg(inf + (int64_t)(e & SPLIT_ROW_MASK) * 4 + c) : make_uint4(0u, 0u, 0u, 0u);
-  }
-#pragma unroll
-  for (int i = 0; i < NB; i++) {
-    const int q = (tid >> 2) + QS * i;
-    if (q >= T.nslots) break;
-    const int d = (int)(src[i] >> SPLIT_ROW_BITS);  // 2^(-2 d) brings the source to the common exponent
-    uint4 w = v[i];
-    if (d > 0) {
-      const __half2 m = __float2half2_rn(__uint_as_float((uint32_t)max(0, 127 - 2 * d) << 23));
-      w.x = h2_bits(__hmul2(*reinterpret_cast<__half2*>(&w.x), m));
-      w.y = h2_bits(__hmul2(*reinterpret_cast<__half2*>(&w.y), m));
-      w.z = h2_bits(__hmul2(*reinterpret_cast<__half2*>(&w.z), m));
-      w.w = h2_bits(__hmul2(*reinterpret_cast<__half2*>(&w.w), m));
-    }
-    // global pieces are children 2c, 2c + 1 as {head, tail, head, tail}; shared chunks are heads of
-    // children 0-3 and 4-7, then tails
+  // global pieces are children 2c, 2c + 1 as {head, tail, head, tail}; shared chunks are heads of
+  // children 0-3 and 4-7, then tails
+  auto store_a = [&](int q, const uint4& w) {
     const uint32_t e = hadh_entry(q);
     *reinterpret_cast<uint2*>(sA + 16 * (e ^ (c >> 1)) + 8 * (c & 1)) = make_uint2(w.x, w.z);
     *reinterpret_cast<uint2*>(sA + 16 * (e ^ (2 + (c >> 1))) + 8 * (c & 1)) = make_uint2(w.y, w.w);
-  }
-  if (first) {
+  };
+  auto store_b = [&](const uint4 (&fb)[NF], const float* bi) {
 #pragma unroll
     for (int i = 0; i < NF; i++) {
       const int e = tid + HADH_NT * i, ln = e & 15;  // stored lane 4 (g / 2) + t
@@ -1642,9 +1671,65 @@ __device__ __forceinline__ void hadh_tile(const HadSys& S, int tile, int f, unsi
       o[0] = fb[i];
       o[4] = hadh_odd(fb[i]);
     }
-    if (tid < 26) sInv[tid] = binv[tid];
+    if (tid < 26) sInv[tid] = bi[tid];
+  };
+  auto load_b = [&](const uint4* fr, uint4 (&fb)[NF]) {
+#pragma unroll
+    for (int i = 0; i < NF; i++) fb[i] = __ldg(fr + min(tid + HADH_NT * i, HADH_FB - 1));
+  };
+  auto scaled = [](uint32_t v, int d) {  // times 2^(-2 d), 0 <= d < 12: exact but for the subnormal range
+    const __half2 m = __float2half2_rn(__uint_as_float((uint32_t)(127 - 2 * d) << 23));
+    return h2_bits(__hmul2(*reinterpret_cast<__half2*>(&v), m));
+  };
+  // the children of pass w alone
+  auto load_pass = [&](int w) {
+    for (int q = tid >> 2; q < T.nslots; q += QS) {
+      const uint32_t e = slots[q];
+      uint4 v = make_uint4(0u, 0u, 0u, 0u);
+      if (e != SPLIT_NONE) {
+        const int64_t row = e & SPLIT_ROW_MASK;
+        const uchar2 cw = reinterpret_cast<const uchar2*>(S.win)[row * 4 + c];
+        const int d = (int)(e >> SPLIT_ROW_BITS) - SPLIT_PASS * w, d0 = d + SPLIT_WIN * cw.x, d1 = d + SPLIT_WIN * cw.y;
+        const uint4 u = __ldg(inf + row * 4 + c);
+        if (d0 >= 0 && d0 < SPLIT_PASS) v.x = scaled(u.x, d0), v.y = scaled(u.y, d0);
+        if (d1 >= 0 && d1 < SPLIT_PASS) v.z = scaled(u.z, d1), v.w = scaled(u.w, d1);
+      }
+      store_a(q, v);
+    }
+  };
+  uint4 fb[NF];
+  if (fill) load_b(frag, fb);
+  uint32_t todo = S.tpass[tile];  // the passes left, the open one included
+  if (todo == 1u) {
+    uint32_t src[NB];
+#pragma unroll
+    for (int i = 0; i < NB; i++) {
+      const int q = (tid >> 2) + QS * i;
+      src[i] = q < T.nslots ? slots[q] : SPLIT_NONE;
+    }
+    uint4 v[NB];
+#pragma unroll
+    for (int i = 0; i < NB; i++) {
+      const uint32_t e = src[i];
+      v[i] = e != SPLIT_NONE ? __ldg(inf + (int64_t)(e & SPLIT_ROW_MASK) * 4 + c) : make_uint4(0u, 0u, 0u, 0u);
+    }
+#pragma unroll
+    for (int i = 0; i < NB; i++) {
+      const int q = (tid >> 2) + QS * i;
+      if (q >= T.nslots) break;
+      const int d = src[i] != SPLIT_NONE ? (int)(src[i] >> SPLIT_ROW_BITS) : 0;
+      uint4 w = v[i];
+      if (d > 0) w = make_uint4(scaled(w.x, d), scaled(w.y, d), scaled(w.z, d), scaled(w.w, d));
+      store_a(q, w);
+    }
+  } else {
+    todo &= ~TILE_DEEP;
+    load_pass(__ffs(todo) - 1);
   }
+  if (fill) store_b(fb, binv);
   __syncthreads();
+  float pscale = 1.f;  // of the open pass
+  int bw = 0;          // the open window of the operator
   // ---- products: group gr of 64 targets, positions ps, ps + np, ...
   const int gr = wid % T.groups, ps = wid / T.groups, np = (HADH_NT / 32) / T.groups;
   const int g = lane >> 2, t = lane & 3;
@@ -1659,6 +1744,7 @@ __device__ __forceinline__ void hadh_tile(const HadSys& S, int tile, int f, unsi
     for (int h = 0; h < 2; h++)
 #pragma unroll
       for (int i = 0; i < 4; i++) acc[j][h][i] = 0.f;
+  for (;;) {
   // table entries two positions ahead
   uint2 e0 = __ldg(tab + ps * pstep), e1 = __ldg(tab + min(ps + np, 25) * pstep);
   for (int ipos = ps; ipos < 26; ipos += np) {
@@ -1666,7 +1752,7 @@ __device__ __forceinline__ void hadh_tile(const HadSys& S, int tile, int f, unsi
     e0 = e1;
     e1 = __ldg(tab + min(ipos + 2 * np, 25) * pstep);
     const uint4 b[2] = {sB[(ipos * 2) * 32 + lane], sB[(ipos * 2 + 1) * 32 + lane]};
-    const float ib = sInv[ipos];
+    const float ib = sInv[ipos] * pscale;
 #pragma unroll
     for (int jp = 0; jp < 4; jp += 2) {
       uint32_t xh[2][4], xt[2][4];
@@ -1697,6 +1783,24 @@ __device__ __forceinline__ void hadh_tile(const HadSys& S, int tile, int f, unsi
 #pragma unroll
           for (int i = 0; i < 4; i++) acc[jp + jj][h][i] = fmaf(d[jj][h][i], ib, acc[jp + jj][h][i]);
     }
+  }
+  // ---- the next window of the operator, then the next pass over the sources
+  if (++bw == nbw) {
+    bw = 0;
+    todo &= todo - 1u;
+    if (todo == 0u) break;
+  }
+  __syncthreads();
+  if (nbw > 1) {
+    load_b(frag + (int64_t)bw * bstride * HADH_FB, fb);
+    store_b(fb, binv + (int64_t)bw * bstride * 32);
+  }
+  if (bw == 0) {
+    const int w = __ffs(todo) - 1;
+    load_pass(w);
+    pscale = pow2f(-2 * SPLIT_PASS * w);
+  }
+  __syncthreads();
   }
   // ---- the position parts of a group, added in order by its first warp
   if (np > 1) {
@@ -1743,22 +1847,23 @@ __device__ __forceinline__ void hadh_tile(const HadSys& S, int tile, int f, unsi
 
 // tiles [blockIdx.x * tpc, ...) at frequency blockIdx.y share one copy of the frequency's B fragments
 __global__ void __launch_bounds__(HADH_NT, 2)
-    k_hadamard_h(const uint4* __restrict__ frag, const float* __restrict__ binv, HadSys S, int ntiles, int tpc) {
+    k_hadamard_h(const uint4* __restrict__ frag, const float* __restrict__ binv, int nbw, HadSys S, int ntiles, int tpc) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   uint4* sB = reinterpret_cast<uint4*>(smem_raw + (size_t)HADH_SLOTS * 64);
   float* sInv = reinterpret_cast<float*>(sB + HADH_B);
   const int f = blockIdx.y, tid = threadIdx.x;
   const int te = min(ntiles, ((int)blockIdx.x + 1) * tpc);
   for (int k = blockIdx.x * tpc; k < te; k++) {
-    hadh_tile(S, k, f, smem_raw, sB, sInv, frag + (int64_t)f * HADH_FB, binv + f * 32, k == (int)blockIdx.x * tpc, tid);
+    hadh_tile(S, k, f, smem_raw, sB, sInv, frag + (int64_t)f * HADH_FB, binv + f * 32, nbw, gridDim.y,
+              nbw > 1 || k == (int)blockIdx.x * tpc, tid);
     if (k + 1 < te) __syncthreads();
   }
 }
 // the same over the tiles of many systems that share one operator table (a batch of Laplace systems):
 // tiles[k] = (system, its tile)
 __global__ void __launch_bounds__(HADH_NT, 2)
-    k_hadamard_h_batch(const uint4* __restrict__ frag, const float* __restrict__ binv, const HadSys* __restrict__ sys,
-                       const int2* __restrict__ tiles, int ntiles, int tpc) {
+    k_hadamard_h_batch(const uint4* __restrict__ frag, const float* __restrict__ binv, int nbw,
+                       const HadSys* __restrict__ sys, const int2* __restrict__ tiles, int ntiles, int tpc) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   uint4* sB = reinterpret_cast<uint4*>(smem_raw + (size_t)HADH_SLOTS * 64);
   float* sInv = reinterpret_cast<float*>(sB + HADH_B);
@@ -1766,8 +1871,8 @@ __global__ void __launch_bounds__(HADH_NT, 2)
   const int te = min(ntiles, ((int)blockIdx.x + 1) * tpc);
   for (int k = blockIdx.x * tpc; k < te; k++) {
     const int2 tl = tiles[k];
-    hadh_tile(sys[tl.x], tl.y, f, smem_raw, sB, sInv, frag + (int64_t)f * HADH_FB, binv + f * 32,
-              k == (int)blockIdx.x * tpc, tid);
+    hadh_tile(sys[tl.x], tl.y, f, smem_raw, sB, sInv, frag + (int64_t)f * HADH_FB, binv + f * 32, nbw, gridDim.y,
+              nbw > 1 || k == (int)blockIdx.x * tpc, tid);
     if (k + 1 < te) __syncthreads();
   }
 }
@@ -1820,15 +1925,20 @@ __host__ __device__ __forceinline__ uint32_t hadc_boff(int n, int c) {
 // btab[f] (HADC_BBYTES per frequency): factor m(sc, tc) of position ipos (head + tail of the stored
 // fragments) -> the real 2 x 2 block (outputs 2 tc, 2 tc + 1; inputs 2 sc, 2 sc + 1) =
 // [[Re m, -Im m], [Im m, Re m]], TF32 head then tail
-__global__ void k_hadc_btab(const uint4* __restrict__ frag, const float* __restrict__ binv, int nfreq,
+__global__ void k_hadc_btab(const uint4* __restrict__ frag, const float* __restrict__ binv, int nbw, int nfreq,
                             unsigned char* __restrict__ btab) {
   const int64_t total = (int64_t)nfreq * 26 * 64;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     const int f = (int)(e / (26 * 64)), ipos = (int)(e / 64 % 26), sc = (int)(e >> 3 & 7), tc = (int)(e & 7);
-    const uint4 q = frag[(int64_t)f * HADH_FB + (ipos * 2 + (tc >> 2)) * 16 + 4 * (tc & 3) + (sc & 3)];
-    const float2 hd = h2_float2(sc < 4 ? q.x : q.y), tl = h2_float2(sc < 4 ? q.z : q.w);
-    const float bi = binv[f * 32 + ipos];
-    const float2 m = make_float2((hd.x + tl.x) * bi, -(hd.y + tl.y) * bi);
+    float2 m = make_float2(0.f, 0.f);
+    for (int w = 0; w < nbw; w++) {  // the factor stands in one of the operator's windows, zeros in the others
+      const int64_t row = (int64_t)w * nfreq + f;
+      const uint4 q = frag[row * HADH_FB + (ipos * 2 + (tc >> 2)) * 16 + 4 * (tc & 3) + (sc & 3)];
+      const float2 hd = h2_float2(sc < 4 ? q.x : q.y), tl = h2_float2(sc < 4 ? q.z : q.w);
+      const float bi = binv[row * 32 + ipos];
+      m.x += (hd.x + tl.x) * bi;
+      m.y -= (hd.y + tl.y) * bi;
+    }
     const float v[4] = {m.x, -m.y, m.y, m.x};
     unsigned char* blk = btab + (int64_t)f * HADC_BBYTES + ipos * 2048;
 #pragma unroll
@@ -1848,8 +1958,8 @@ __device__ __forceinline__ bool hadc_wait(uint32_t mbar, uint32_t parity) {
 
 __global__ void __launch_bounds__(HADC_NT, 2)
     k_hadamard_dc(const unsigned char* __restrict__ btab, const SplitC* __restrict__ in, float2* __restrict__ out,
-                  const uint32_t* __restrict__ tab, int ld, const int* __restrict__ rows, int nsrc, int ntrg, int nfreq,
-                  int* __restrict__ status) {
+                  const uint8_t* __restrict__ win, const uint32_t* __restrict__ tab, int ld, const int* __restrict__ rows,
+                  int nsrc, int ntrg, int nfreq, int* __restrict__ status) {
   using namespace tc5;
   extern __shared__ __align__(16) unsigned char smem_raw[];  // B blocks of the current frequency, gather ring
   __shared__ __align__(8) uint64_t mbar[2 * HADC_S + 2];       // full[S], done[S], B half 0, B half 1
@@ -1992,11 +2102,14 @@ __global__ void __launch_bounds__(HADC_NT, 2)
         const uint4* sl = reinterpret_cast<const uint4*>(smem_raw + HADC_BBYTES + (size_t)(gi % HADC_R) * (128 * 64)) +
                            (wid * 4) * 32 + lane;
 #pragma unroll
-        for (int i = 0; i < 4; i++) {  // head + tail, exponent undone: children 2 q and 2 q + 1
+        for (int i = 0; i < 4; i++) {  // head + tail, exponents undone: children 2 q and 2 q + 1
           const uint4 v = sl[i * 32];
-          const float sc = split_inv(__shfl_sync(0xffffffffu, entg, g + 8 * i));
+          const uint32_t e = __shfl_sync(0xffffffffu, entg, g + 8 * i);
+          uchar2 cw = make_uchar2(0, 0);
+          if (e != SPLIT_NONE) cw = reinterpret_cast<const uchar2*>(win)[(int64_t)(e & SPLIT_ROW_MASK) * 4 + q];
+          const float s0 = split_inv(e) * pow2f(-2 * SPLIT_WIN * cw.x), s1 = split_inv(e) * pow2f(-2 * SPLIT_WIN * cw.y);
           const float2 h0 = h2_float2(v.x), t0 = h2_float2(v.y), h1 = h2_float2(v.z), t1 = h2_float2(v.w);
-          x[i] = make_float4((h0.x + t0.x) * sc, (h0.y + t0.y) * sc, (h1.x + t1.x) * sc, (h1.y + t1.y) * sc);
+          x[i] = make_float4((h0.x + t0.x) * s0, (h0.y + t0.y) * s0, (h1.x + t1.x) * s1, (h1.y + t1.y) * s1);
         }
       }
       if (gi >= HADC_S) {  // the stage's previous position is done: take its products, then reuse it
@@ -2097,12 +2210,12 @@ template <> struct Spec<double> {
 };
 __device__ __forceinline__ float abs1(float v) { return fabsf(v); }
 __device__ __forceinline__ float abs1(float2 v) { return fabsf(v.x) + fabsf(v.y); }
-// The scale of source node s (children at node0 .. node0 + 7): every spectrum value of a child is at most
-// the sum of its densities' magnitudes.  One warp per child; red: 8 floats of shared memory.  Called by a
-// whole CTA of 256 threads; writes the source's exponent code for k_pack_sources.
+// The scales of source node s (children at node0 .. node0 + 7).  One warp per child; red: 8 floats of shared memory;
+// csc: the children's scales, ready after the caller's next barrier.  Called by a whole CTA of 256 threads;
+// writes the source's exponent code and its children's windows.
 template <class W>
-__device__ __forceinline__ float source_scale(const W* __restrict__ up, int64_t node0, int nsurf, float* red,
-                                              int* __restrict__ scode) {
+__device__ __forceinline__ void source_scales(const W* __restrict__ up, int64_t node0, int nsurf, float* red, float* csc,
+                                              int* __restrict__ scode, uint8_t* __restrict__ win) {
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const W* u = up + (node0 + wid) * nsurf;
   float m = 0.f;
@@ -2111,12 +2224,16 @@ __device__ __forceinline__ float source_scale(const W* __restrict__ up, int64_t 
   for (int o = 16; o > 0; o >>= 1) m += __shfl_xor_sync(0xffffffffu, m, o);
   if (lane == 0) red[wid] = m;
   __syncthreads();
-  float b = red[0];
+  if (threadIdx.x < 8) {
+    float b = red[0];
 #pragma unroll
-  for (int c = 1; c < 8; c++) b = fmaxf(b, red[c]);
-  const int code = split_code(b);
-  if (threadIdx.x == 0) *scode = code;
-  return split_scale(code);
+    for (int c = 1; c < 8; c++) b = fmaxf(b, red[c]);
+    const int code = split_code(b), w = split_window(red[lane], b, code);
+    csc[lane] = split_scale(code, w);
+    win[lane] = (uint8_t)w;
+    const bool deep = __any_sync(0xffu, w > 0);
+    if (lane == 0) *scode = code | (deep ? SPLIT_DEEP : 0) | (b == 0.f ? SPLIT_ZERO : 0);
+  }
 }
 // DFT factors as compile-time constants: where the loops unroll, an index (j k mod N) is known to the compiler and the
 // factor becomes an operand of the multiply-add instead of a shared-memory load or a register.  cos and
@@ -2172,17 +2289,17 @@ __device__ __forceinline__ void wfma(CT& acc, const CT& a, const CT& w) {
   }
 }
 
-// The cuFFT path (orders beyond the DFT kernels): each source's exponent code ...
+// The cuFFT path (orders beyond the DFT kernels): each source's exponent code and windows ...
 template <class W>
 __global__ void __launch_bounds__(256)
     k_source_codes(const int* __restrict__ src, const int* __restrict__ child0, const W* __restrict__ up, int nsurf,
-                   int* __restrict__ scode) {
-  __shared__ float red[8];
-  source_scale(up, (int64_t)child0[src[blockIdx.x]], nsurf, red, scode + blockIdx.x);
+                   int* __restrict__ scode, uint8_t* __restrict__ win) {
+  __shared__ float red[8], csc[8];
+  source_scales(up, (int64_t)child0[src[blockIdx.x]], nsurf, red, csc, scode + blockIdx.x, win + 8ll * blockIdx.x);
 }
 // ... and its spectra, rows (source, child) x nfreq, into the split layout [f][source][child]
 __global__ void k_transpose_split(const float2* __restrict__ in, SplitC* __restrict__ out, int ns, int nfreq,
-                                  const int* __restrict__ scode) {
+                                  const int* __restrict__ scode, const uint8_t* __restrict__ win) {
   __shared__ float2 tile[32][33];
   const int64_t r0 = (int64_t)blockIdx.y * 32, c0 = (int64_t)blockIdx.x * 32, nr = (int64_t)ns * 8;
   for (int i = threadIdx.y; i < 32; i += 8) {
@@ -2193,7 +2310,7 @@ __global__ void k_transpose_split(const float2* __restrict__ in, SplitC* __restr
   for (int i = threadIdx.y; i < 32; i += 8) {
     const int64_t c = c0 + i, r = r0 + threadIdx.x;
     if (r >= nr || c >= nfreq) continue;
-    const float sc = split_scale(scode[r >> 3]);
+    const float sc = split_scale(scode[r >> 3] & 0x7f, win[r]);
     const float2 v = tile[threadIdx.x][i];
     out[c * nr + r] = split16(v.x * sc, v.y * sc);
   }
@@ -2373,7 +2490,8 @@ template <class R, int P>
 __global__ void __launch_bounds__(FT_NT, FtcFwdMinB<R>::v)
     k_m2l_fwd_c(const int* __restrict__ src, int ns, const int* __restrict__ child0,
                 const typename C2<R>::type* __restrict__ up, int nsurf, const int* __restrict__ conv2surf,
-                const double* __restrict__ tw, typename Spec<R>::type* __restrict__ spec, int* __restrict__ scode) {
+                const double* __restrict__ tw, typename Spec<R>::type* __restrict__ spec, int* __restrict__ scode,
+                uint8_t* __restrict__ win) {
   using CT = typename C2<R>::type;
   constexpr int N = 2 * P, CPB = FtcCpb<R>::v, KS = 2 * FTC_JS;
   const int s = blockIdx.x, ch0 = blockIdx.y * CPB, tid = threadIdx.x;
@@ -2388,10 +2506,10 @@ __global__ void __launch_bounds__(FT_NT, FtcFwdMinB<R>::v)
     sidx[e] = conv2surf[(c * N + b) * N + a];
   }
   const int64_t node0 = (int64_t)child0[src[s]] + ch0;
-  float sc = 1.f;  // the node's power-of-two scale
+  __shared__ float csc[8];  // the children's power-of-two scales (mixed)
   if constexpr (sizeof(R) == 4) {
     __shared__ float red[8];
-    sc = source_scale(up, node0, nsurf, red, scode + s);
+    source_scales(up, node0, nsurf, red, csc, scode + s, win + 8ll * s);
   }
   const int64_t fstride = (int64_t)N * N * ns * 8;
   for (int j0 = 0; j0 < P; j0 += FTC_JS) {
@@ -2438,7 +2556,7 @@ __global__ void __launch_bounds__(FT_NT, FtcFwdMinB<R>::v)
 #pragma unroll
       for (int c = 0; c < P; c++) x[c] = sB[((c * N + kb) * CPB + ch) * KS + sl];
       auto* o = spec + ((int64_t)(kb * N + ka) * ns + s) * 8 + ch0 + ch;
-      ftc_dft_p<P>(x, ConstW<CT, N, -1>(), [&](int kc, CT v) { o[kc * fstride] = Spec<R>::make(v, sc); });
+      ftc_dft_p<P>(x, ConstW<CT, N, -1>(), [&](int kc, CT v) { o[kc * fstride] = Spec<R>::make(v, csc[ch]); });
     }
   }
 }
@@ -2572,7 +2690,7 @@ template <class R, int P>
 __global__ void __launch_bounds__(FT_NT, FtrMinB<R>::v)
     k_m2l_fwd_r(const int* __restrict__ src, int ns, const int* __restrict__ child0, const R* __restrict__ up,
                 int nsurf, const int* __restrict__ conv2surf, const double* __restrict__ tw,
-                typename Spec<R>::type* __restrict__ spec, int* __restrict__ scode) {
+                typename Spec<R>::type* __restrict__ spec, int* __restrict__ scode, uint8_t* __restrict__ win) {
   using CT = typename C2<R>::type;
   constexpr int N = 2 * P, H = P + 1, CPB = FtCpb<R>::v, KS = FTR_KS;
   const int s = blockIdx.x, ch0 = blockIdx.y * CPB, tid = threadIdx.x;
@@ -2587,10 +2705,10 @@ __global__ void __launch_bounds__(FT_NT, FtrMinB<R>::v)
     sidx[e] = conv2surf[(c * N + b) * N + a];
   }
   const int64_t node0 = (int64_t)child0[src[s]] + ch0;
-  float sc = 1.f;  // the node's power-of-two scale
+  __shared__ float csc[8];  // the children's power-of-two scales (mixed)
   if constexpr (sizeof(R) == 4) {
     __shared__ float red[8];
-    sc = source_scale(up, node0, nsurf, red, scode + s);
+    source_scales(up, node0, nsurf, red, csc, scode + s, win + 8ll * s);
   }
   const int64_t fstride = (int64_t)N * H * ns * 8;  // kc -> kc + 1
   for (int k0 = 0; k0 < H; k0 += KS) {
@@ -2639,7 +2757,7 @@ __global__ void __launch_bounds__(FT_NT, FtrMinB<R>::v)
 #pragma unroll
       for (int c = 0; c < P; c++) x[c] = sB[((c * N + kb) * CPB + ch) * KS + sl];
       auto* o = spec + ((int64_t)(kb * H + ka) * ns + s) * 8 + ch0 + ch;
-      ftc_dft_p<P>(x, ConstW<CT, N, -1>(), [&](int kc, CT v) { o[kc * fstride] = Spec<R>::make(v, sc); });
+      ftc_dft_p<P>(x, ConstW<CT, N, -1>(), [&](int kc, CT v) { o[kc * fstride] = Spec<R>::make(v, csc[ch]); });
     }
   }
 }
@@ -2800,11 +2918,12 @@ struct Workspace {
   // Hadamard tiling: per group, tiles of TT targets; CSR over (tile, ipos) of (local target, source)
   std::vector<int> had_tile0;  // first tile of each group (ngroups + 1)
   // mixed path: tiles of k_hadamard_h (per group [had_tile0[g], had_tile0[g + 1])), their source slots,
-  // tables and output rows; scode: every source's exponent code of the last forward transform (one group at
-  // a time)
+  // tables and output rows; scode, swin: every source's exponent code and its children's windows of the last
+  // forward transform (one group at a time)
   DBuf<HadTile> hadh_tile;
   DBuf<int> hadh_slots, hadh_rows, scode;
-  DBuf<uint32_t> hadh_pslots;  // k_tile_codes
+  DBuf<uint8_t> swin;
+  DBuf<uint32_t> hadh_pslots, hadh_tpass;  // k_tile_codes
   DBuf<float> hadh_tinv;
   DBuf<uint2> hadh_tab;
   // FP64, and the dense targets of the tcgen05 form: per group a [26][ld] source table and ld output rows
@@ -2974,6 +3093,7 @@ Workspace& workspace(Fmm& f, Tree& t, cudaStream_t s) {
   if (f.mixed()) {
     XREQUIRE(maxn < (int)SPLIT_ROW_MASK, XFMM_ERR_UNSUPPORTED, "too many M2L sources");
     W.scode.alloc(maxn);
+    W.swin.alloc((size_t)maxn * 8);
   }
   int dims[3] = {f.n1, f.n1, f.n1};
   cufftType tf = cplx ? (f.mixed() ? CUFFT_C2C : CUFFT_Z2Z) : (f.mixed() ? CUFFT_R2C : CUFFT_D2Z);
@@ -3113,6 +3233,7 @@ Workspace& workspace(Fmm& f, Tree& t, cudaStream_t s) {
       W.hadh_tab.upload(tab, s);
       W.hadh_pslots.alloc(slots.size());
       W.hadh_tinv.alloc(tiles.size());
+      W.hadh_tpass.alloc(tiles.size());
     }
     if (!dtab.empty()) {
       W.hadd_tab.upload(dtab, s);
@@ -3297,7 +3418,8 @@ struct Engine {
                 ws.ft_fwd_smem = smem;
               }
               k_m2l_fwd_r<R, PP><<<dim3(ns, 8 / FtCpb<R>::v), FT_NT, smem, s>>>(
-                  src, ns, t.child0.p, (const R*)ws.up.p, n, f.conv_to_surf_up.p, f.dft_tw.p, spec, ws.scode.p);
+                  src, ns, t.child0.p, (const R*)ws.up.p, n, f.conv_to_surf_up.p, f.dft_tw.p, spec, ws.scode.p,
+                  ws.swin.p);
             });
             XLAUNCH();
             ws.launches++;
@@ -3311,7 +3433,8 @@ struct Engine {
               ws.ft_fwd_smem = smem;
             }
             k_m2l_fwd_c<R, PP><<<dim3(ns, 8 / FtcCpb<R>::v), FT_NT, smem, s>>>(
-                src, ns, t.child0.p, (const CT*)ws.up.p, n, f.conv_to_surf_up.p, f.dft_tw.p, spec, ws.scode.p);
+                src, ns, t.child0.p, (const CT*)ws.up.p, n, f.conv_to_surf_up.p, f.dft_tw.p, spec, ws.scode.p,
+                  ws.swin.p);
           });
           XLAUNCH();
           ws.launches++;
@@ -3325,11 +3448,12 @@ struct Engine {
           exec_fwd(ws.fwd[g], ws.grid.p, ws.specA.p);
           ws.launches++;
           if constexpr (sizeof(R) == 4) {  // -> [f][s][c], split
-            k_source_codes<W><<<ns, 256, 0, s>>>(src, t.child0.p, (const W*)ws.up.p, n, ws.scode.p);
+            k_source_codes<W><<<ns, 256, 0, s>>>(src, t.child0.p, (const W*)ws.up.p, n, ws.scode.p, ws.swin.p);
             XLAUNCH();
             const dim3 grid((nfreq + 31) / 32, ((int64_t)ns * 8 + 31) / 32);
             XREQUIRE(grid.y < 65536, XFMM_ERR_UNSUPPORTED, "transpose too tall");
-            k_transpose_split<<<grid, dim3(32, 8), 0, s>>>((const float2*)ws.specA.p, spec, ns, nfreq, ws.scode.p);
+            k_transpose_split<<<grid, dim3(32, 8), 0, s>>>((const float2*)ws.specA.p, spec, ns, nfreq, ws.scode.p,
+                                                         ws.swin.p);
             XLAUNCH();
             ws.launches++;
           } else {
@@ -3338,7 +3462,8 @@ struct Engine {
         }
         if (const int nht = ws.had_tile0[g + 1] - ws.had_tile0[g]; sizeof(R) == 4 && nht > 0) {
           k_tile_codes<<<nht, 256, 0, s>>>(ws.hadh_tile.p + ws.had_tile0[g], ws.hadh_slots.p, ws.scode.p,
-                                           ws.hadh_pslots.p, ws.hadh_tinv.p + ws.had_tile0[g]);
+                                           ws.swin.p, ws.hadh_pslots.p, ws.hadh_tinv.p + ws.had_tile0[g],
+                                           ws.hadh_tpass.p + ws.had_tile0[g]);
           XLAUNCH();
           ws.launches++;
         }
@@ -3365,7 +3490,7 @@ struct Engine {
             const HadSys S = had_sys(ws, g, ns, nt);
             const LevelOps& op = f.ops[tab_level];
             k_hadamard_h<<<dim3((ntiles + tpc - 1) / tpc, nfreq), HADH_NT, HADH_SMEM, s>>>(
-                (const uint4*)op.m2l_frag.p, op.m2l_binv.p, S, ntiles, tpc);
+                (const uint4*)op.m2l_frag.p, op.m2l_binv.p, op.m2l_windows, S, ntiles, tpc);
             XLAUNCH();
             ws.launches++;
           }
@@ -3378,14 +3503,14 @@ struct Engine {
             if (ws.hadc_btab_T != (const void*)op.m2l_frag.p || ws.hadc_btab_nf != nfreq) {  // B blocks in the MMA layout
               ws.hadc_btab.reserve((size_t)nfreq * HADC_BBYTES);
               k_hadc_btab<<<std::min<int64_t>(nblk((int64_t)nfreq * 26 * 64), 148 * 16), 256, 0, s>>>(
-                  (const uint4*)op.m2l_frag.p, op.m2l_binv.p, nfreq, ws.hadc_btab.p);
+                  (const uint4*)op.m2l_frag.p, op.m2l_binv.p, op.m2l_windows, nfreq, ws.hadc_btab.p);
               XLAUNCH();
               ws.launches++;
               ws.hadc_btab_T = op.m2l_frag.p;
               ws.hadc_btab_nf = nfreq;
             }
             k_hadamard_dc<<<dim3(ws.hadd_ld[g] / 128, (nfreq + HADC_FPB - 1) / HADC_FPB), HADC_NT, HADC_SMEM, s>>>(
-                ws.hadc_btab.p, spec, (CT*)ws.specA.p, ws.hadd_tabp.p + ws.hadd_tab0[g], ws.hadd_ld[g],
+                ws.hadc_btab.p, spec, (CT*)ws.specA.p, ws.swin.p, ws.hadd_tabp.p + ws.hadd_tab0[g], ws.hadd_ld[g],
                 ws.hadd_row.p + ws.hadd_row0[g], ns, nt, nfreq, ws.status.p);
             XLAUNCH();
             ws.launches++;
@@ -3489,6 +3614,7 @@ struct Engine {
   static HadSys had_sys(Workspace& ws, int g, int ns, int nt) {
     return HadSys{(const SplitC*)ws.specB.p,           (float2*)ws.specA.p, ws.hadh_tile.p + ws.had_tile0[g],
                   ws.hadh_pslots.p,                    ws.hadh_tinv.p + ws.had_tile0[g],
+                  ws.hadh_tpass.p + ws.had_tile0[g],   ws.swin.p,
                   ws.hadh_tab.p,                       ws.hadh_rows.p,      ns,
                   nt};
   }
@@ -3662,11 +3788,31 @@ void m2l_fragments(LevelOps& op, const double* T64, int nfreq, bool mixed, cudaS
     XLAUNCH();
     return;
   }
-  op.m2l_frag.alloc((size_t)nfreq * HADH_FB * sizeof(uint4));
-  op.m2l_binv.alloc((size_t)nfreq * 32);
-  k_m2l_fragments<<<nblk(26ll * nfreq * 32), 256, 0, s>>>((const double2*)T64, nfreq, (uint4*)op.m2l_frag.p,
-                                                          op.m2l_binv.p);
+  // every child pair's window (k_m2l_fragments)
+  DBuf<unsigned> pmax(26 * 64);
+  XCUDA(cudaMemsetAsync(pmax.p, 0, pmax.bytes(), s));
+  k_pair_max<<<dim3(std::min((nfreq + 3) / 4, 64), 26), 256, 0, s>>>((const double2*)T64, nfreq, pmax.p);
   XLAUNCH();
+  const std::vector<unsigned> hm = pmax.download(s);  // the bits of floats >= 0
+  std::vector<uint8_t> hw(26 * 64, 255);              // 255: no factors, or below the FP32 range
+  op.m2l_windows = 1;
+  for (int i = 0; i < 26; i++) {
+    const int top = (int)(*std::max_element(hm.begin() + 64 * i, hm.begin() + 64 * (i + 1)) >> 23);
+    for (int k = 64 * i; k < 64 * (i + 1); k++) {
+      const int x = (int)(hm[k] >> 23);
+      if (x == 0) continue;
+      hw[k] = (uint8_t)((top - x) / (2 * SPLIT_WIN));
+      op.m2l_windows = std::max(op.m2l_windows, (int)hw[k] + 1);
+    }
+  }
+  DBuf<uint8_t> pwin;
+  pwin.upload(hw, s);
+  op.m2l_frag.alloc((size_t)op.m2l_windows * nfreq * HADH_FB * sizeof(uint4));
+  op.m2l_binv.alloc((size_t)op.m2l_windows * nfreq * 32);
+  k_m2l_fragments<<<dim3(nblk(26ll * nfreq * 32), op.m2l_windows), 256, 0, s>>>(
+      (const double2*)T64, nfreq, pwin.p, (uint4*)op.m2l_frag.p, op.m2l_binv.p);
+  XLAUNCH();
+  XCUDA(cudaStreamSynchronize(s));  // pwin is released here
 }
 void set_charges(Fmm& f, Tree& t, const double* q, bool on_device, cudaStream_t s) {
   const int64_t n = t.nsrc;
@@ -4119,7 +4265,8 @@ void batch_evaluate(Batch* b, const double* const* charges, double* const* outs,
     if (b->nhtiles > 0) {
       const int tpc = std::max(1, b->had_tpc);
       k_hadamard_h_batch<<<dim3((b->nhtiles + tpc - 1) / tpc, b->had_nfreq), HADH_NT, HADH_SMEM, s>>>(
-          (const uint4*)b->had_op->m2l_frag.p, b->had_op->m2l_binv.p, b->hsys.p, b->htiles.p, b->nhtiles, tpc);
+          (const uint4*)b->had_op->m2l_frag.p, b->had_op->m2l_binv.p, b->had_op->m2l_windows, b->hsys.p, b->htiles.p,
+          b->nhtiles, tpc);
       XLAUNCH();
     }
     per_system(2 * E, 0, M2L_BWD, false);

@@ -187,7 +187,8 @@ struct LevelOps {
   // M2L tables ([26][nfreq][64] complex, entry [s*8+t]; fmm_scale_invariant.h:549-551) as the Hadamard's
   // fragments per frequency: FP64, or FP16 head / tail for the mixed path (m2l_fragments)
   DBuf<char> m2l_frag;
-  DBuf<float> m2l_binv;  // mixed: [nfreq][32], undoes the exponent of each block
+  DBuf<float> m2l_binv;  // mixed: [window][nfreq][32], undoes the exponent of each block
+  int m2l_windows = 1;   // mixed: windows of the factors' exponents (k_m2l_fragments)
   int rank = 0;        // singular values kept by the pinv threshold: B1 columns / B2 rows beyond are zero
   // the same operators in the form the translation GEMMs (translate.cu) read: real [K][N] row-major, a
   // complex operator expanded to [2K][2N] (expand_operator); FP64 for the pinv factors and the FP64
