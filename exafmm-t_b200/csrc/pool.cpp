@@ -44,9 +44,10 @@ void give_back(Kept& k) {
 }
 }  // namespace
 
-void* pool_alloc(size_t bytes, size_t* capacity) {
+cudaError_t pool_alloc(size_t bytes, void** out, size_t* capacity) {
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+  cudaError_t err = cudaGetDevice(&dev);
+  if (err != cudaSuccess) return err;
   const size_t want = round_up(bytes);
   Pool& P = pool();
   std::lock_guard<std::mutex> lock(P.m);
@@ -58,20 +59,24 @@ void* pool_alloc(size_t bytes, size_t* capacity) {
     k.bytes -= it->first;
     k.blocks.erase(it);
     P.owner[p] = dev;
-    return p;
+    *out = p;
+    return cudaSuccess;
   }
   void* p = nullptr;
-  if (cudaMalloc(&p, want) != cudaSuccess) {
+  err = cudaMalloc(&p, want);
+  if (err == cudaErrorMemoryAllocation) {
     cudaGetLastError();
     give_back(k);
-    if (cudaMalloc(&p, want) != cudaSuccess) {
-      cudaGetLastError();
-      return nullptr;
-    }
+    err = cudaMalloc(&p, want);
+  }
+  if (err != cudaSuccess) {
+    cudaGetLastError();
+    return err;
   }
   *capacity = want;
   P.owner[p] = dev;
-  return p;
+  *out = p;
+  return cudaSuccess;
 }
 
 void pool_release(void* p, size_t capacity) noexcept {

@@ -41,7 +41,7 @@ struct Error : std::exception {
 // Fmm handle is freed, and whenever an allocation fails.  As with cudaFree, a release waits for the device
 // (every stream of it), so a kept block has no work left that could touch it; a PoolQuiet scope waits once
 // for all releases made inside it.  Any thread may allocate and release.
-void* pool_alloc(size_t bytes, size_t* capacity);  // null (and the CUDA error) on failure
+cudaError_t pool_alloc(size_t bytes, void** p, size_t* capacity);
 void pool_release(void* p, size_t capacity) noexcept;
 void pool_hold();            // an Fmm handle was created
 void pool_unhold() noexcept;  // ... was freed
@@ -77,8 +77,9 @@ struct DBuf {
   void alloc(size_t count) {
     release();
     if (!count) return;
-    p = static_cast<T*>(pool_alloc(count * sizeof(T), &cap));
-    if (!p) XCUDA(cudaErrorMemoryAllocation);
+    void* block = nullptr;
+    XCUDA(pool_alloc(count * sizeof(T), &block, &cap));
+    p = static_cast<T*>(block);
     n = count;
   }
   // grow-only reallocation (contents not preserved)

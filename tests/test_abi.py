@@ -46,6 +46,23 @@ def test_status_without_gpu_is_an_error_not_a_crash():
         raise AssertionError("setup without a GPU must fail loudly")
 
 
+def test_missing_device_is_a_cuda_error_not_out_of_memory():
+    import numpy as np
+    import pytest
+    import exafmm.laplace as L
+    from exafmm import _lib
+    torch = pytest.importorskip("torch")
+    if torch.cuda.is_available():
+        pytest.skip("needs a machine without a device")
+    x, q, out = np.random.default_rng(0).random((50, 3)), np.ones(50), np.zeros((50, 4))
+    f = L.LaplaceFmm(4, 32)
+    with pytest.raises(_lib.FmmError) as e:
+        L.setup(L.init_sources(x, q), L.init_targets(x), f)
+    assert e.value.code == 3  # XFMM_ERR_CUDA
+    p = [a.ctypes.data_as(_lib.vp) for a in (x, q, x, out)]
+    assert _lib.lib().xfmm_gradient_p2p(0, 0.0, 0.0, 0, p[0], 50, p[1], p[2], 50, p[3], 0, None) == 3
+
+
 def test_argument_errors():
     import numpy as np
     import exafmm.laplace as L
