@@ -31,12 +31,6 @@ Pool& pool() {
 thread_local int t_quiet = 0;
 thread_local bool t_waited = false;
 
-// capacities in steps of an eighth of a power of two, so that blocks of nearly equal sizes serve each other
-size_t round_up(size_t b) {
-  size_t step = 512;
-  while (step * 16 < b) step *= 2;
-  return (b + step - 1) / step * step;
-}
 void give_back(Kept& k) {
   for (auto& b : k.blocks) cudaFree(b.second);
   k.blocks.clear();
@@ -44,11 +38,20 @@ void give_back(Kept& k) {
 }
 }  // namespace
 
+// Capacities in steps of an eighth of a power of two, so that blocks of nearly equal sizes serve each other; the
+// exact size for blocks that are never kept (spectra of tens of GB would grow by GBs).
+size_t pool_capacity(size_t b) {
+  size_t step = 512;
+  while (step * 16 < b) step *= 2;
+  const size_t r = (b + step - 1) / step * step;
+  return r <= POOL_MAX_BLOCK ? r : b;
+}
+
 cudaError_t pool_alloc(size_t bytes, void** out, size_t* capacity) {
   int dev = 0;
   cudaError_t err = cudaGetDevice(&dev);
   if (err != cudaSuccess) return err;
-  const size_t want = round_up(bytes);
+  const size_t want = pool_capacity(bytes);
   Pool& P = pool();
   std::lock_guard<std::mutex> lock(P.m);
   Kept& k = P.dev[dev];

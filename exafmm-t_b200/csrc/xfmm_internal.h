@@ -42,6 +42,7 @@ struct Error : std::exception {
 // (every stream of it), so a kept block has no work left that could touch it; a PoolQuiet scope waits once
 // for all releases made inside it.  Any thread may allocate and release.
 cudaError_t pool_alloc(size_t bytes, void** p, size_t* capacity);
+size_t pool_capacity(size_t bytes);  // of the block that an allocation takes
 void pool_release(void* p, size_t capacity) noexcept;
 void pool_hold();            // an Fmm handle was created
 void pool_unhold() noexcept;  // ... was freed
