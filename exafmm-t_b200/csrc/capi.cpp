@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -108,7 +109,8 @@ xfmm_status xfmm_fmm_set_operator_file(xfmm_fmm* fmm, const char* filename) {
 
 xfmm_status xfmm_fmm_free(xfmm_fmm* fmm) {
   return guarded([&] {
-    xfmm::PoolQuiet quiet;
+    if (!fmm) return;
+    xfmm::FreeScope free(fmm->f.uses);
     delete fmm;
   });
 }
@@ -137,23 +139,20 @@ xfmm_status xfmm_build_tree(xfmm_fmm* fmm, const double* src_xyz, int64_t nsrc, 
       check_finite_host(src_xyz, 3 * (size_t)nsrc, "source coordinates");
       check_finite_host(trg_xyz, 3 * (size_t)ntrg, "target coordinates");
     }
-    auto* h = new xfmm_tree();
-    try {
-      h->t.nsrc = nsrc;
-      h->t.ntrg = ntrg;
-      DevIn s(src_xyz, 3 * (size_t)nsrc, on_device, S(stream)), t(trg_xyz, 3 * (size_t)ntrg, on_device, S(stream));
-      xfmm::build_tree(fmm->f, h->t, s.p, t.p, nonadaptive_depth, S(stream));
-    } catch (...) {
-      delete h;
-      throw;
-    }
-    *out = h;
+    std::unique_ptr<xfmm_tree> h(new xfmm_tree());
+    xfmm::UseScope use(S(stream), {&fmm->f.uses, &h->t.uses});
+    h->t.nsrc = nsrc;
+    h->t.ntrg = ntrg;
+    DevIn s(src_xyz, 3 * (size_t)nsrc, on_device, S(stream)), t(trg_xyz, 3 * (size_t)ntrg, on_device, S(stream));
+    xfmm::build_tree(fmm->f, h->t, s.p, t.p, nonadaptive_depth, S(stream));
+    *out = h.release();
   });
 }
 
 xfmm_status xfmm_tree_free(xfmm_tree* tree) {
   return guarded([&] {
-    xfmm::PoolQuiet quiet;
+    if (!tree) return;
+    xfmm::FreeScope free(tree->t.uses);
     delete tree;
   });
 }
@@ -161,6 +160,7 @@ xfmm_status xfmm_tree_free(xfmm_tree* tree) {
 xfmm_status xfmm_build_list(xfmm_fmm* fmm, xfmm_tree* tree, void* stream) {
   return guarded([&] {
     XREQUIRE(fmm && tree, XFMM_ERR_ARG, "null argument");
+    xfmm::UseScope use(S(stream), {&fmm->f.uses, &tree->t.uses});
     xfmm::build_lists(fmm->f, tree->t, S(stream));
   });
 }
@@ -168,6 +168,7 @@ xfmm_status xfmm_build_list(xfmm_fmm* fmm, xfmm_tree* tree, void* stream) {
 xfmm_status xfmm_m2l_setup(xfmm_fmm* fmm, xfmm_tree* tree, void* stream) {
   return guarded([&] {
     XREQUIRE(fmm && tree, XFMM_ERR_ARG, "null argument");
+    xfmm::UseScope use(S(stream), {&fmm->f.uses, &tree->t.uses});
     xfmm::m2l_setup(fmm->f, tree->t, S(stream));
   });
 }
@@ -175,6 +176,7 @@ xfmm_status xfmm_m2l_setup(xfmm_fmm* fmm, xfmm_tree* tree, void* stream) {
 xfmm_status xfmm_precompute(xfmm_fmm* fmm, xfmm_tree* tree, void* stream) {
   return guarded([&] {
     XREQUIRE(fmm && tree, XFMM_ERR_ARG, "null argument");
+    xfmm::UseScope use(S(stream), {&fmm->f.uses, &tree->t.uses});
     xfmm::Fmm& f = fmm->f;
     XREQUIRE(tree->t.r0 > 0, XFMM_ERR_STATE, "precompute before build_tree");
     f.r0 = tree->t.r0;
@@ -191,6 +193,7 @@ xfmm_status xfmm_precompute(xfmm_fmm* fmm, xfmm_tree* tree, void* stream) {
 xfmm_status xfmm_set_charges(xfmm_fmm* fmm, xfmm_tree* tree, const double* q, int on_device, void* stream) {
   return guarded([&] {
     XREQUIRE(fmm && tree && q, XFMM_ERR_ARG, "null argument");
+    xfmm::UseScope use(S(stream), {&fmm->f.uses, &tree->t.uses});
     xfmm::set_charges(fmm->f, tree->t, q, on_device != 0, S(stream));
   });
 }
@@ -198,6 +201,7 @@ xfmm_status xfmm_set_charges(xfmm_fmm* fmm, xfmm_tree* tree, const double* q, in
 xfmm_status xfmm_clear_values(xfmm_fmm* fmm, xfmm_tree* tree, void* stream) {
   return guarded([&] {
     XREQUIRE(fmm && tree, XFMM_ERR_ARG, "null argument");
+    xfmm::UseScope use(S(stream), {&fmm->f.uses, &tree->t.uses});
     xfmm::clear_values(fmm->f, tree->t, S(stream));
   });
 }
@@ -205,6 +209,7 @@ xfmm_status xfmm_clear_values(xfmm_fmm* fmm, xfmm_tree* tree, void* stream) {
 xfmm_status xfmm_upward_pass(xfmm_fmm* fmm, xfmm_tree* tree, void* stream) {
   return guarded([&] {
     XREQUIRE(fmm && tree, XFMM_ERR_ARG, "null argument");
+    xfmm::UseScope use(S(stream), {&fmm->f.uses, &tree->t.uses});
     xfmm::upward_pass(fmm->f, tree->t, S(stream));
   });
 }
@@ -212,6 +217,7 @@ xfmm_status xfmm_upward_pass(xfmm_fmm* fmm, xfmm_tree* tree, void* stream) {
 xfmm_status xfmm_downward_pass(xfmm_fmm* fmm, xfmm_tree* tree, void* stream) {
   return guarded([&] {
     XREQUIRE(fmm && tree, XFMM_ERR_ARG, "null argument");
+    xfmm::UseScope use(S(stream), {&fmm->f.uses, &tree->t.uses});
     xfmm::downward_pass(fmm->f, tree->t, S(stream));
   });
 }
@@ -219,6 +225,7 @@ xfmm_status xfmm_downward_pass(xfmm_fmm* fmm, xfmm_tree* tree, void* stream) {
 xfmm_status xfmm_get_values(xfmm_fmm* fmm, xfmm_tree* tree, double* out, int on_device, void* stream) {
   return guarded([&] {
     XREQUIRE(fmm && tree && out, XFMM_ERR_ARG, "null argument");
+    xfmm::UseScope use(S(stream), {&fmm->f.uses, &tree->t.uses});
     const size_t n = (size_t)tree->t.ntrg * 4 * (fmm->f.is_complex() ? 2 : 1);
     if (on_device) {
       xfmm::get_values(fmm->f, tree->t, out, S(stream));
@@ -235,6 +242,7 @@ xfmm_status xfmm_get_values(xfmm_fmm* fmm, xfmm_tree* tree, double* out, int on_
 xfmm_status xfmm_evaluate(xfmm_fmm* fmm, xfmm_tree* tree, double* out, int on_device, void* stream) {
   return guarded([&] {
     XREQUIRE(fmm && tree && out, XFMM_ERR_ARG, "null argument");
+    xfmm::UseScope use(S(stream), {&fmm->f.uses, &tree->t.uses});
     xfmm::clear_values(fmm->f, tree->t, S(stream));
     xfmm::upward_pass(fmm->f, tree->t, S(stream));
     xfmm::downward_pass(fmm->f, tree->t, S(stream));
@@ -344,6 +352,9 @@ xfmm_status xfmm_batch_create(xfmm_fmm* const* fmms, xfmm_tree* const* trees, in
       f[k] = &fmms[k]->f;
       t[k] = &trees[k]->t;
     }
+    std::vector<xfmm::Uses*> u;
+    for (int k = 0; k < n; k++) u.insert(u.end(), {&f[k]->uses, &t[k]->uses});
+    xfmm::UseScope use(S(stream), u);
     *out = reinterpret_cast<xfmm_batch*>(xfmm::batch_create(f.data(), t.data(), n, S(stream)));
   });
 }
@@ -352,6 +363,7 @@ xfmm_status xfmm_batch_evaluate(xfmm_batch* b, const double* const* charges, dou
                                 void* stream) {
   return guarded([&] {
     XREQUIRE(b && outs, XFMM_ERR_ARG, "null argument");
+    xfmm::UseScope use(S(stream), xfmm::batch_uses(reinterpret_cast<xfmm::Batch*>(b)));
     xfmm::batch_evaluate(reinterpret_cast<xfmm::Batch*>(b), charges, outs, nstreams, S(stream));
   });
 }
@@ -385,6 +397,7 @@ xfmm_status xfmm_gradient_p2p(int kernel, double k_re, double k_im, int precisio
     XREQUIRE(src_xyz && q && trg_xyz && out, XFMM_ERR_ARG, "null argument");
     const int vs = kernel == XFMM_HELMHOLTZ ? 2 : 1;
     cudaStream_t s = S(stream);
+    xfmm::UseScope use(s, {});
     DevIn sx(src_xyz, 3 * (size_t)nsrc, on_device, s), tx(trg_xyz, 3 * (size_t)ntrg, on_device, s),
         qq(q, (size_t)nsrc * vs, on_device, s);
     xfmm::DBuf<double> tmp;
@@ -405,6 +418,7 @@ xfmm_status xfmm_gradient_p2p(int kernel, double k_re, double k_im, int precisio
 xfmm_status xfmm_verify(xfmm_fmm* fmm, xfmm_tree* tree, int sample, double* err2, void* stream) {
   return guarded([&] {
     XREQUIRE(fmm && tree && err2, XFMM_ERR_ARG, "null argument");
+    xfmm::UseScope use(S(stream), {&fmm->f.uses, &tree->t.uses});
     xfmm::verify(fmm->f, tree->t, sample, err2, S(stream));
   });
 }

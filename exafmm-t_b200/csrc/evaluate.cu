@@ -3912,6 +3912,7 @@ __global__ void k_tag_pairs(const int4* __restrict__ src, int64_t n, int sys, in
 }
 
 struct Batch {
+  Uses uses;
   std::vector<Fmm*> fmm;
   std::vector<Tree*> tree;
   int kernel = 0, precision = 0;
@@ -4147,7 +4148,17 @@ Batch* batch_create(Fmm** fmms, Tree** trees, int n, cudaStream_t s) {
   return b;
 }
 
-void batch_free(Batch* b) { delete b; }
+// The batch's own buffers were written when it was created, and its evaluates use them with the systems'.
+void batch_free(Batch* b) {
+  if (!b) return;
+  FreeScope free(b->uses);
+  delete b;
+}
+std::vector<Uses*> batch_uses(Batch* b) {
+  std::vector<Uses*> u{&b->uses};
+  for (size_t k = 0; k < b->fmm.size(); k++) u.insert(u.end(), {&b->fmm[k]->uses, &b->tree[k]->uses});
+  return u;
+}
 
 void batch_schedule(const int64_t* sizes, int n, int nstreams, int* stream_of) {
   XREQUIRE(n >= 0 && nstreams >= 1, XFMM_ERR_ARG, "batch schedule needs n >= 0 and nstreams >= 1");

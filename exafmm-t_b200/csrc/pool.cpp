@@ -1,6 +1,7 @@
-// pool.cpp -- kept device memory blocks (declared in xfmm_internal.h).
+// pool.cpp -- kept device memory blocks, and the work that uses them (declared in xfmm_internal.h).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <map>
 #include <mutex>
 #include <vector>
@@ -17,10 +18,15 @@ struct Kept {
   std::multimap<size_t, void*> blocks;  // by capacity
   size_t bytes = 0;
 };
+struct Block {
+  int dev;
+  uint64_t number;  // of its allocation, ascending
+};
 struct Pool {
   std::mutex m;
   std::map<int, Kept> dev;
-  std::map<void*, int> owner;  // device of every block handed out
+  std::map<void*, Block> owner;  // every block handed out
+  uint64_t allocations = 0;
   int holds = 0;
 };
 // never destroyed: handles may be freed while the process exits
@@ -28,8 +34,21 @@ Pool& pool() {
   static Pool* p = new Pool();
   return *p;
 }
-thread_local int t_quiet = 0;
-thread_local bool t_waited = false;
+thread_local UseScope* t_scope = nullptr;  // the API call that this thread is in
+thread_local bool t_idle = false;          // an object is being freed and its work is done
+
+// Waits that CUDA allows while another thread captures: of streams and events that take no part in a capture.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+bool capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
+  cudaGetLastError();  // the legacy stream, while a stream that waits for it captures
+  return true;
+}
 
 void give_back(Kept& k) {
   for (auto& b : k.blocks) cudaFree(b.second);
@@ -61,7 +80,7 @@ cudaError_t pool_alloc(size_t bytes, void** out, size_t* capacity) {
     *capacity = it->first;
     k.bytes -= it->first;
     k.blocks.erase(it);
-    P.owner[p] = dev;
+    P.owner[p] = Block{dev, ++P.allocations};
     *out = p;
     return cudaSuccess;
   }
@@ -77,39 +96,32 @@ cudaError_t pool_alloc(size_t bytes, void** out, size_t* capacity) {
     return err;
   }
   *capacity = want;
-  P.owner[p] = dev;
+  P.owner[p] = Block{dev, ++P.allocations};
   *out = p;
   return cudaSuccess;
 }
 
 void pool_release(void* p, size_t capacity) noexcept {
   Pool& P = pool();
-  int dev = -1, cur = -1;
+  Block b{-1, 0};
+  int cur = -1;
   bool keep = false;
   {
     std::lock_guard<std::mutex> lock(P.m);
     auto it = P.owner.find(p);
     if (it != P.owner.end()) {
-      dev = it->second;
+      b = it->second;
       P.owner.erase(it);
     }
     keep = P.holds > 0 && capacity <= POOL_MAX_BLOCK;
   }
-  if (keep && cudaGetDevice(&cur) == cudaSuccess && cur == dev) {
-    // no work in flight may still use the block (cudaFree waits in the same way)
-    bool idle = t_quiet > 0 && t_waited;
-    if (!idle) {
-      idle = cudaDeviceSynchronize() == cudaSuccess;
-      t_waited = idle;
-    }
-    if (idle) {
-      std::lock_guard<std::mutex> lock(P.m);
-      Kept& k = P.dev[dev];
-      if (P.holds > 0 && k.bytes + capacity <= POOL_KEEP) {
-        k.blocks.emplace(capacity, p);
-        k.bytes += capacity;
-        return;
-      }
+  if (keep && (t_idle || (t_scope && t_scope->idle(b.number))) && cudaGetDevice(&cur) == cudaSuccess && cur == b.dev) {
+    std::lock_guard<std::mutex> lock(P.m);
+    Kept& k = P.dev[b.dev];
+    if (P.holds > 0 && k.bytes + capacity <= POOL_KEEP) {
+      k.blocks.emplace(capacity, p);
+      k.bytes += capacity;
+      return;
     }
   }
   cudaFree(p);
@@ -126,11 +138,65 @@ void pool_unhold() noexcept {
     for (auto& d : P.dev) give_back(d.second);
 }
 
-PoolQuiet::PoolQuiet() noexcept {
-  if (t_quiet++ == 0) t_waited = false;
+bool Uses::wait() const noexcept {
+  if (captured) return false;
+  RelaxedCapture relaxed;
+  for (const auto& u : last)
+    if (cudaEventSynchronize(u.second->e) != cudaSuccess) return false;
+  return true;
 }
-PoolQuiet::~PoolQuiet() {
-  if (--t_quiet == 0) t_waited = false;
+
+UseScope::UseScope(cudaStream_t s, std::vector<Uses*> objects)
+    : s_(s), objects_(std::move(objects)), capturing_(capturing(s)), outer_(t_scope) {
+  {
+    std::lock_guard<std::mutex> lock(pool().m);
+    begin_ = pool().allocations;
+  }
+  if (capturing_)
+    for (Uses* u : objects_) u->captured = true;
+  t_scope = this;
 }
+
+UseScope::~UseScope() {
+  t_scope = outer_;
+  if (capturing_ || objects_.empty()) return;
+  try {
+    unsigned long long id = 0;
+    std::shared_ptr<Uses::Event> ev;
+    bool ok = cudaStreamGetId(s_, &id) == cudaSuccess;
+    // the stream's event of one of the objects, recorded again: all earlier work of the stream is before it
+    for (Uses* u : objects_)
+      for (auto& l : u->last)
+        if (l.first == id) ev = l.second;
+    if (ok && !ev) {
+      ev = std::make_shared<Uses::Event>();
+      ok = cudaEventCreateWithFlags(&ev->e, cudaEventDisableTiming) == cudaSuccess;
+    }
+    if (ok && cudaEventRecord(ev->e, s_) == cudaSuccess) {
+      for (Uses* u : objects_) {
+        auto it = std::find_if(u->last.begin(), u->last.end(), [&](const auto& l) { return l.first == id; });
+        if (it == u->last.end()) u->last.emplace_back(id, ev);
+        else it->second = ev;
+      }
+      return;
+    }
+    cudaGetLastError();
+  } catch (...) {
+  }
+  for (Uses* u : objects_) u->captured = true;  // nothing tells the end of this work
+}
+
+bool UseScope::idle(uint64_t allocated) const noexcept {
+  if (capturing_) return false;
+  RelaxedCapture relaxed;
+  if (cudaStreamSynchronize(s_) != cudaSuccess) return false;
+  if (allocated > begin_) return true;
+  for (const Uses* u : objects_)
+    if (!u->wait()) return false;
+  return true;
+}
+
+FreeScope::FreeScope(const Uses& u) noexcept { t_idle = u.wait(); }
+FreeScope::~FreeScope() { t_idle = false; }
 
 }  // namespace xfmm

@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstring>
+#include <memory>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -38,19 +39,56 @@ struct Error : std::exception {
 // Device memory of the buffers below (pool.cpp).  A cudaMalloc or cudaFree takes 50 to 100 us, and a set-up at new
 // positions makes about a hundred of each: blocks that are released while an Fmm handle lives are kept for
 // the next allocations, at most POOL_KEEP bytes per device; the kept blocks go back to the device when the last
-// Fmm handle is freed, and whenever an allocation fails.  As with cudaFree, a release waits for the device
-// (every stream of it), so a kept block has no work left that could touch it; a PoolQuiet scope waits once
-// for all releases made inside it.  Any thread may allocate and release.
+// Fmm handle is freed, and whenever an allocation fails.  A block is kept only once nothing in flight can
+// touch it, and any other goes to cudaFree.  Waiting for the whole device would tell, but CUDA forbids it while any
+// stream captures, and breaks that capture; so every object knows the work that used it (Uses), and a release
+// waits for that work alone.  Any thread may allocate and release.
 cudaError_t pool_alloc(size_t bytes, void** p, size_t* capacity);
 size_t pool_capacity(size_t bytes);  // of the block that an allocation takes
 void pool_release(void* p, size_t capacity) noexcept;
 void pool_hold();            // an Fmm handle was created
 void pool_unhold() noexcept;  // ... was freed
-struct PoolQuiet {
-  PoolQuiet() noexcept;
-  ~PoolQuiet();
-  PoolQuiet(const PoolQuiet&) = delete;
-  PoolQuiet& operator=(const PoolQuiet&) = delete;
+
+// The device work that used an object: per stream (by its id) an event behind the last of it, and whether some
+// was captured into a graph, which may be replayed at any time.  Like the handles, for one thread at a time.
+struct Uses {
+  struct Event {
+    cudaEvent_t e = nullptr;
+    Event() = default;
+    Event(const Event&) = delete;
+    Event& operator=(const Event&) = delete;
+    ~Event() {
+      if (e) cudaEventDestroy(e);
+    }
+  };
+  std::vector<std::pair<unsigned long long, std::shared_ptr<Event>>> last;
+  bool captured = false;
+  bool wait() const noexcept;  // waits for the work; false: some was captured, or an error
+};
+// One call of the C API: its work on stream s uses the objects; they learn of it at the end of the scope.  Blocks that
+// the scope allocated itself are idle once s is, others once the objects' earlier work is done too.
+class UseScope {
+ public:
+  UseScope(cudaStream_t s, std::vector<Uses*> objects);
+  ~UseScope();
+  UseScope(const UseScope&) = delete;
+  UseScope& operator=(const UseScope&) = delete;
+  bool idle(uint64_t allocated) const noexcept;  // waits until a block with that allocation number is idle
+
+ private:
+  cudaStream_t s_;
+  std::vector<Uses*> objects_;
+  uint64_t begin_;
+  bool capturing_;
+  UseScope* outer_;
+};
+// The freeing of an object: waits for its work, and its blocks can be kept.
+class FreeScope {
+ public:
+  explicit FreeScope(const Uses& u) noexcept;
+  ~FreeScope();
+  FreeScope(const FreeScope&) = delete;
+  FreeScope& operator=(const FreeScope&) = delete;
 };
 
 // Owning device buffer (move-only).
@@ -119,6 +157,7 @@ void release_workspace(Tree& t);
 
 // Tree + interaction lists on the device, node arrays in the reference's idx order.
 struct Tree {
+  Uses uses;
   Workspace* ws[2] = {nullptr, nullptr};  // evaluate workspace per precision
   Tree() = default;
   Tree(const Tree&) = delete;
@@ -201,6 +240,7 @@ struct LevelOps {
 };
 
 struct Fmm {
+  Uses uses;
   int kernel = 0, p = 0, ncrit = 0, precision = 0;
   double k_re = 0, k_im = 0;
   int nsurf = 0, nconv = 0, nfreq = 0, n1 = 0;
@@ -279,6 +319,7 @@ void prepare_translation_operands(const Fmm& f, LevelOps& op, cudaStream_t s);
 struct Batch;
 Batch* batch_create(Fmm** fmms, Tree** trees, int n, cudaStream_t s);
 void batch_free(Batch* b);
+std::vector<Uses*> batch_uses(Batch* b);  // of the batch and its systems
 void batch_schedule(const int64_t* sizes, int n, int nstreams, int* stream_of);
 void batch_set_tuning(Batch* b, int option, int value);
 void batch_evaluate(Batch* b, const double* const* charges, double* const* outs, int nstreams, cudaStream_t s);

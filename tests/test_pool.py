@@ -66,3 +66,58 @@ def test_threads():
     for t in threads:
         t.join()
     assert not bad
+
+
+def _tree(fmm, seed, n):
+    import exafmm.laplace as lap
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    x = torch.rand(n, 3, dtype=torch.float64, device="cuda", generator=gen)
+    q = torch.rand(n, dtype=torch.float64, device="cuda", generator=gen) - 0.5
+    return lap.setup(lap.init_sources(x, q), lap.init_targets(x), fmm)
+
+
+def test_freeing_a_tree_leaves_another_threads_capture_alone():
+    """CUDA breaks a capture when any thread waits for the whole device: a release waits for the tree's own work."""
+    import exafmm.laplace as lap
+    fmm = _fmm()
+    held = [_tree(fmm, 1, 20000)]
+    want = torch.empty(20000, 4, dtype=torch.float64, device="cuda")
+    lap.evaluate(held[0], fmm, out=want)
+    torch.cuda.synchronize()
+    a = torch.zeros(1000, device="cuda")
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, capture_error_mode="thread_local"):
+        a.add_(1)
+        t = threading.Thread(target=held.clear)
+        t.start()
+        t.join()
+        a.add_(1)
+    g.replay()
+    out = torch.empty_like(want)
+    lap.evaluate(_tree(fmm, 1, 20000), fmm, out=out)
+    torch.cuda.synchronize()
+    assert bool((a == 2).all()) and torch.equal(out, want)
+
+
+def test_blocks_of_a_tree_freed_with_work_in_flight():
+    """A tree evaluated on one stream and freed at once, the next one set up on another stream in its memory."""
+    import exafmm.laplace as lap
+    fmm = _fmm()
+    seeds, n = range(6), 60000
+    want = []
+    for s in seeds:
+        o = torch.empty(n, 4, dtype=torch.float64, device="cuda")
+        lap.evaluate(_tree(fmm, s, n), fmm, out=o)
+        torch.cuda.synchronize()
+        want.append(o)
+    streams, outs = [torch.cuda.Stream() for _ in range(2)], []
+    for s in seeds:
+        with torch.cuda.stream(streams[s % 2]):
+            outs.append(torch.empty(n, 4, dtype=torch.float64, device="cuda"))
+            tree = _tree(fmm, s, n)
+            for _ in range(3):
+                lap.evaluate(tree, fmm, out=outs[-1])
+            del tree
+    torch.cuda.synchronize()
+    for o, w in zip(outs, want):
+        assert torch.equal(o, w)
