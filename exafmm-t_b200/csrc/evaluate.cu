@@ -1393,14 +1393,15 @@ __global__ void __launch_bounds__(HAD64_NT, 2)
 // The mixed path's spectra are stored split: a real x of a child's spectrum is the pair of FP16 values
 // h = fp16(2^e x), t = fp16(2^e x - h): 22 bits of x within 2^-17 of the top (2^15), an absolute error below
 // 2^-39 of it elsewhere.  Every spectrum value of a child is at most the sum of its densities' magnitudes,
-// its bound.  A source node has one exponent e, set by its strongest child; a child whose bound is more than
-// 2^-18 below goes to the next window of the node, with the exponent e + 18, and so on, so that every child
-// keeps an error below 2^-21 of its own bound however strong its siblings are (a screened kernel shows a
-// weak source: the strong one's field is gone where its own targets are).  A split spectrum has the size of
-// the FP32 one, the products need no conversion (the operator's blocks are split the same way,
-// k_m2l_fragments), and an FP16 MMA does twice the work of a TF32 one in the same 8 cycles (measured:
-// m16n8k16 f16 and m16n8k8 tf32 both 8.0 cycles per warp and SM quadrant) with the same 11-bit significands.
-// A child's complex value is the 8 bytes {h.re, h.im, t.re, t.im}.
+// its bound.  A source node has one exponent e, set by its strongest child.  With the unscreened kernels a weak
+// child's error stays far below the FP32 rounding of its siblings' fields, which reach the same targets at a
+// comparable distance.  A screened kernel shows a weak child (the strong one's field is gone where its own targets
+// are), so there every child has its level, the steps of 2 bits by which its bound lies below the node's, and
+// those from 9 steps on the exponent e + 18, from 18 on e + 36 and so on: every child keeps an error below
+// 2^-21 of its own bound.  A split spectrum has the size of the FP32 one, the products need no conversion (the
+// operator's blocks are split the same way, k_m2l_fragments), and an FP16 MMA does twice the work of a TF32 one
+// in the same 8 cycles (measured: m16n8k16 f16 and m16n8k8 tf32 both 8.0 cycles per warp and SM quadrant) with
+// the same 11-bit significands.  A child's complex value is the 8 bytes {h.re, h.im, t.re, t.im}.
 using SplitC = uint2;
 __device__ __forceinline__ uint32_t h2_bits(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
 __device__ __forceinline__ float2 h2_float2(uint32_t u) { return __half22float2(*reinterpret_cast<__half2*>(&u)); }
@@ -1420,14 +1421,16 @@ __device__ __forceinline__ int split_code(float bound) {
 }
 constexpr int SPLIT_WIN = 9;   // steps of 2 bits between the windows of a node's children and of the operator's pairs
 constexpr int SPLIT_PASS = 10;  // steps that one pass over a tile covers: 2^-18 from its strongest source to its weakest
-constexpr int SPLIT_DEEP = 0x100, SPLIT_ZERO = 0x200;  // beside a source's code: a child beyond window 0; no values
+constexpr int SPLIT_DEEP = 0x100, SPLIT_ZERO = 0x200;  // beside a source's code: children at levels > 0; no values
 __device__ __forceinline__ float pow2f(int e) { return e >= -126 ? __uint_as_float((uint32_t)(127 + e) << 23) : 0.f; }
-__device__ __forceinline__ float split_scale(int code, int w) { return pow2f(127 - 2 * (code - SPLIT_WIN * w)); }
-// the window of a child with bound c of a node with bound b, whose scale is still a float
-__device__ __forceinline__ int split_window(float c, float b, int code) {
+__device__ __forceinline__ float split_scale(int code, int level = 0) {
+  return pow2f(127 - 2 * (code - level / SPLIT_WIN * SPLIT_WIN));
+}
+// the level of a child with bound c of a node with bound b (its scale is still a float)
+__device__ __forceinline__ int split_level(float c, float b, int code) {
   if (!(c > 0.f)) return 0;
   const int below = (int)(__float_as_uint(b) >> 23) - (int)(__float_as_uint(c) >> 23);
-  return min(max(0, below) / (2 * SPLIT_WIN), (code - 1) / SPLIT_WIN);
+  return min(max(0, below) / 2, (code - 1) / SPLIT_WIN * SPLIT_WIN + SPLIT_WIN - 1);
 }
 // Packed sources: the source row in the low 25 bits (2^25 sources would need 206 GB of spectra at the lowest
 // order) and 7 bits of exponent: in the opt-in tcgen05 form's table the source's code (written by
@@ -1470,10 +1473,10 @@ constexpr int HADC_TT = 512;  // padding of its source table
 // targets at one relative position have 8 different octants, so their 64-byte rows (four 16-byte chunks,
 // swizzled by (slot / 2) % 4) fall on different banks; empty positions read one of 8 zero slots, chosen to
 // stay off the banks of the other rows.
-// A tile whose children lie within 2^-18 of its strongest has one pass: all tiles of cubes, Plummer spheres and
-// surfaces of up to 4M bodies with charges in (-1, 1) (2 to 9 steps of 2 bits).  Otherwise pass w takes the
-// children 10 w .. 10 w + 9 steps below, the others at zero, over the same accumulators: weak sources keep their 22
-// bits.  The same for the windows of the operator.
+// A tile whose sources (screened kernels: whose children) lie within 2^-18 of the strongest has one pass: all
+// Laplace tiles of cubes, Plummer spheres and surfaces of up to 4M bodies with charges in (-1, 1), 2 to 9 steps of
+// 2 bits.  Otherwise pass w takes those 10 w .. 10 w + 9 steps below, the others at zero, over the same
+// accumulators: weak sources keep their 22 bits.  The same for the windows of the operator.
 // Tiles with at most 256, 128 or 64 targets split the 26 positions over 2, 4 or 8 warps per 64 targets.
 // Bounds per 64 targets and position and SM (cycles): MMAs 24 x 8 / 4 = 48; shared memory 32 (A) + 8 (B).
 // At 1M, p = 8 the tensor pipe is 54% and the shared-memory pipe 64% busy: 16 warps per SM hide the rest of
@@ -1500,8 +1503,8 @@ struct HadSys {
   const HadTile* tiles;
   const uint32_t* slots;  // packed source of each slot (k_tile_codes)
   const float* tinv;      // per tile: undoes its exponent
-  const uint32_t* tpass;  // per tile: bit w: pass w has sources; TILE_DEEP: children beyond window 0
-  const uint8_t* win;     // window of every source's children
+  const uint32_t* tpass;  // per tile: bit w: pass w has sources; TILE_DEEP: children with exponents of their own
+  const uint8_t* level;   // of every source's children
   const uint2* tab;
   const int* rows;
   int nsrc, ntrg;
@@ -1562,7 +1565,7 @@ __global__ void k_m2l_fragments(const double2* __restrict__ T, int nfreq, const 
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
   const int code = split_code(m);
-  const double sc = (double)split_scale(code, 0);
+  const double sc = (double)split_scale(code);
   const int h = lane >> 4, tc = 4 * h + ((lane >> 2) & 3), t = lane & 3;
   uint32_t hd[2], tl[2];
 #pragma unroll
@@ -1588,7 +1591,7 @@ __device__ __forceinline__ uint4 hadh_odd(const uint4& e) {
 // without values), and the passes that the tile needs.
 __global__ void __launch_bounds__(256)
     k_tile_codes(const HadTile* __restrict__ tiles, const int* __restrict__ slots, const int* __restrict__ scode,
-                 const uint8_t* __restrict__ win, uint32_t* __restrict__ pslots, float* __restrict__ tinv,
+                 const uint8_t* __restrict__ level, uint32_t* __restrict__ pslots, float* __restrict__ tinv,
                  uint32_t* __restrict__ tpass) {
   __shared__ int smax;
   __shared__ uint32_t spass;
@@ -1618,8 +1621,12 @@ __global__ void __launch_bounds__(256)
       pslots[T.slot0 + q] = src[i] >= 0 ? (uint32_t)src[i] | (uint32_t)d << SPLIT_ROW_BITS : SPLIT_NONE;
     if (src[i] < 0) continue;
     if (code[i] & SPLIT_DEEP) {
-      pass |= TILE_DEEP;
-      for (int c = 0; c < 8; c++) pass |= 1u << ((d + SPLIT_WIN * win[(int64_t)src[i] * 8 + c]) / SPLIT_PASS);
+#pragma unroll
+      for (int c = 0; c < 8; c++) {
+        const int l = level[(int64_t)src[i] * 8 + c];
+        pass |= 1u << ((d + l) / SPLIT_PASS);
+        if (l >= SPLIT_WIN) pass |= TILE_DEEP;
+      }
     } else {
       pass |= 1u << (d / SPLIT_PASS);
     }
@@ -1677,22 +1684,29 @@ __device__ __forceinline__ void hadh_tile(const HadSys& S, int tile, int f, unsi
 #pragma unroll
     for (int i = 0; i < NF; i++) fb[i] = __ldg(fr + min(tid + HADH_NT * i, HADH_FB - 1));
   };
-  auto scaled = [](uint32_t v, int d) {  // times 2^(-2 d), 0 <= d < 12: exact but for the subnormal range
+  auto scaled = [](uint32_t v, int d) {  // times 2^(-2 d), d < SPLIT_PASS
     const __half2 m = __float2half2_rn(__uint_as_float((uint32_t)(127 - 2 * d) << 23));
     return h2_bits(__hmul2(*reinterpret_cast<__half2*>(&v), m));
   };
-  // the children of pass w alone
+  auto moved = [](uint32_t v, int s) {  // times 2^(2 s), |s| <= 9
+    const uint32_t m = (uint32_t)(15 + s) << 10;
+    const __half2 f = __halves2half2(__ushort_as_half((unsigned short)m), __ushort_as_half((unsigned short)m));
+    return h2_bits(__hmul2(__hmul2(*reinterpret_cast<__half2*>(&v), f), f));
+  };
+  // the children of pass w alone, at the exponent 20 w above the tile's
   auto load_pass = [&](int w) {
     for (int q = tid >> 2; q < T.nslots; q += QS) {
       const uint32_t e = slots[q];
       uint4 v = make_uint4(0u, 0u, 0u, 0u);
       if (e != SPLIT_NONE) {
         const int64_t row = e & SPLIT_ROW_MASK;
-        const uchar2 cw = reinterpret_cast<const uchar2*>(S.win)[row * 4 + c];
-        const int d = (int)(e >> SPLIT_ROW_BITS) - SPLIT_PASS * w, d0 = d + SPLIT_WIN * cw.x, d1 = d + SPLIT_WIN * cw.y;
+        const uchar2 l = reinterpret_cast<const uchar2*>(S.level)[row * 4 + c];
+        const int d = (int)(e >> SPLIT_ROW_BITS);
         const uint4 u = __ldg(inf + row * 4 + c);
-        if (d0 >= 0 && d0 < SPLIT_PASS) v.x = scaled(u.x, d0), v.y = scaled(u.y, d0);
-        if (d1 >= 0 && d1 < SPLIT_PASS) v.z = scaled(u.z, d1), v.w = scaled(u.w, d1);
+        // stored 2 d + 18 (level / 9) above the tile's exponent
+        const int s0 = SPLIT_PASS * w - d - l.x / SPLIT_WIN * SPLIT_WIN, s1 = SPLIT_PASS * w - d - l.y / SPLIT_WIN * SPLIT_WIN;
+        if ((d + l.x) / SPLIT_PASS == w) v.x = moved(u.x, s0), v.y = moved(u.y, s0);
+        if ((d + l.y) / SPLIT_PASS == w) v.z = moved(u.z, s1), v.w = moved(u.w, s1);
       }
       store_a(q, v);
     }
@@ -1958,8 +1972,8 @@ __device__ __forceinline__ bool hadc_wait(uint32_t mbar, uint32_t parity) {
 
 __global__ void __launch_bounds__(HADC_NT, 2)
     k_hadamard_dc(const unsigned char* __restrict__ btab, const SplitC* __restrict__ in, float2* __restrict__ out,
-                  const uint8_t* __restrict__ win, const uint32_t* __restrict__ tab, int ld, const int* __restrict__ rows,
-                  int nsrc, int ntrg, int nfreq, int* __restrict__ status) {
+                  const uint8_t* __restrict__ level, const uint32_t* __restrict__ tab, int ld,
+                  const int* __restrict__ rows, int nsrc, int ntrg, int nfreq, int* __restrict__ status) {
   using namespace tc5;
   extern __shared__ __align__(16) unsigned char smem_raw[];  // B blocks of the current frequency, gather ring
   __shared__ __align__(8) uint64_t mbar[2 * HADC_S + 2];       // full[S], done[S], B half 0, B half 1
@@ -2105,9 +2119,10 @@ __global__ void __launch_bounds__(HADC_NT, 2)
         for (int i = 0; i < 4; i++) {  // head + tail, exponents undone: children 2 q and 2 q + 1
           const uint4 v = sl[i * 32];
           const uint32_t e = __shfl_sync(0xffffffffu, entg, g + 8 * i);
-          uchar2 cw = make_uchar2(0, 0);
-          if (e != SPLIT_NONE) cw = reinterpret_cast<const uchar2*>(win)[(int64_t)(e & SPLIT_ROW_MASK) * 4 + q];
-          const float s0 = split_inv(e) * pow2f(-2 * SPLIT_WIN * cw.x), s1 = split_inv(e) * pow2f(-2 * SPLIT_WIN * cw.y);
+          uchar2 l = make_uchar2(0, 0);
+          if (e != SPLIT_NONE) l = reinterpret_cast<const uchar2*>(level)[(int64_t)(e & SPLIT_ROW_MASK) * 4 + q];
+          const float s0 = split_inv(e) * pow2f(-2 * SPLIT_WIN * (l.x / SPLIT_WIN));
+          const float s1 = split_inv(e) * pow2f(-2 * SPLIT_WIN * (l.y / SPLIT_WIN));
           const float2 h0 = h2_float2(v.x), t0 = h2_float2(v.y), h1 = h2_float2(v.z), t1 = h2_float2(v.w);
           x[i] = make_float4((h0.x + t0.x) * s0, (h0.y + t0.y) * s0, (h1.x + t1.x) * s1, (h1.y + t1.y) * s1);
         }
@@ -2212,10 +2227,15 @@ __device__ __forceinline__ float abs1(float v) { return fabsf(v); }
 __device__ __forceinline__ float abs1(float2 v) { return fabsf(v.x) + fabsf(v.y); }
 // The scales of source node s (children at node0 .. node0 + 7).  One warp per child; red: 8 floats of shared memory;
 // csc: the children's scales, ready after the caller's next barrier.  Called by a whole CTA of 256 threads;
-// writes the source's exponent code and its children's windows.
+// writes the source's exponent code and its children's levels (all 0 unless the kernel is screened).
+struct SplitOut {
+  int* code;
+  uint8_t* level;
+  int screened;
+};
 template <class W>
 __device__ __forceinline__ void source_scales(const W* __restrict__ up, int64_t node0, int nsurf, float* red, float* csc,
-                                              int* __restrict__ scode, uint8_t* __restrict__ win) {
+                                              const SplitOut& so, int64_t s) {
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const W* u = up + (node0 + wid) * nsurf;
   float m = 0.f;
@@ -2228,11 +2248,11 @@ __device__ __forceinline__ void source_scales(const W* __restrict__ up, int64_t 
     float b = red[0];
 #pragma unroll
     for (int c = 1; c < 8; c++) b = fmaxf(b, red[c]);
-    const int code = split_code(b), w = split_window(red[lane], b, code);
-    csc[lane] = split_scale(code, w);
-    win[lane] = (uint8_t)w;
-    const bool deep = __any_sync(0xffu, w > 0);
-    if (lane == 0) *scode = code | (deep ? SPLIT_DEEP : 0) | (b == 0.f ? SPLIT_ZERO : 0);
+    const int code = split_code(b), l = so.screened ? split_level(red[lane], b, code) : 0;
+    csc[lane] = split_scale(code, l);
+    so.level[8 * s + lane] = (uint8_t)l;
+    const bool deep = __any_sync(0xffu, l > 0);
+    if (lane == 0) so.code[s] = code | (deep ? SPLIT_DEEP : 0) | (b == 0.f ? SPLIT_ZERO : 0);
   }
 }
 // DFT factors as compile-time constants: where the loops unroll, an index (j k mod N) is known to the compiler and the
@@ -2289,17 +2309,17 @@ __device__ __forceinline__ void wfma(CT& acc, const CT& a, const CT& w) {
   }
 }
 
-// The cuFFT path (orders beyond the DFT kernels): each source's exponent code and windows ...
+// The cuFFT path (orders beyond the DFT kernels): each source's exponent code and levels ...
 template <class W>
 __global__ void __launch_bounds__(256)
     k_source_codes(const int* __restrict__ src, const int* __restrict__ child0, const W* __restrict__ up, int nsurf,
-                   int* __restrict__ scode, uint8_t* __restrict__ win) {
+                   SplitOut so) {
   __shared__ float red[8], csc[8];
-  source_scales(up, (int64_t)child0[src[blockIdx.x]], nsurf, red, csc, scode + blockIdx.x, win + 8ll * blockIdx.x);
+  source_scales(up, (int64_t)child0[src[blockIdx.x]], nsurf, red, csc, so, blockIdx.x);
 }
 // ... and its spectra, rows (source, child) x nfreq, into the split layout [f][source][child]
 __global__ void k_transpose_split(const float2* __restrict__ in, SplitC* __restrict__ out, int ns, int nfreq,
-                                  const int* __restrict__ scode, const uint8_t* __restrict__ win) {
+                                  SplitOut so) {
   __shared__ float2 tile[32][33];
   const int64_t r0 = (int64_t)blockIdx.y * 32, c0 = (int64_t)blockIdx.x * 32, nr = (int64_t)ns * 8;
   for (int i = threadIdx.y; i < 32; i += 8) {
@@ -2310,7 +2330,7 @@ __global__ void k_transpose_split(const float2* __restrict__ in, SplitC* __restr
   for (int i = threadIdx.y; i < 32; i += 8) {
     const int64_t c = c0 + i, r = r0 + threadIdx.x;
     if (r >= nr || c >= nfreq) continue;
-    const float sc = split_scale(scode[r >> 3] & 0x7f, win[r]);
+    const float sc = split_scale(so.code[r >> 3] & 0x7f, so.level[r]);
     const float2 v = tile[threadIdx.x][i];
     out[c * nr + r] = split16(v.x * sc, v.y * sc);
   }
@@ -2490,8 +2510,7 @@ template <class R, int P>
 __global__ void __launch_bounds__(FT_NT, FtcFwdMinB<R>::v)
     k_m2l_fwd_c(const int* __restrict__ src, int ns, const int* __restrict__ child0,
                 const typename C2<R>::type* __restrict__ up, int nsurf, const int* __restrict__ conv2surf,
-                const double* __restrict__ tw, typename Spec<R>::type* __restrict__ spec, int* __restrict__ scode,
-                uint8_t* __restrict__ win) {
+                const double* __restrict__ tw, typename Spec<R>::type* __restrict__ spec, SplitOut so) {
   using CT = typename C2<R>::type;
   constexpr int N = 2 * P, CPB = FtcCpb<R>::v, KS = 2 * FTC_JS;
   const int s = blockIdx.x, ch0 = blockIdx.y * CPB, tid = threadIdx.x;
@@ -2509,7 +2528,7 @@ __global__ void __launch_bounds__(FT_NT, FtcFwdMinB<R>::v)
   __shared__ float csc[8];  // the children's power-of-two scales (mixed)
   if constexpr (sizeof(R) == 4) {
     __shared__ float red[8];
-    source_scales(up, node0, nsurf, red, csc, scode + s, win + 8ll * s);
+    source_scales(up, node0, nsurf, red, csc, so, s);
   }
   const int64_t fstride = (int64_t)N * N * ns * 8;
   for (int j0 = 0; j0 < P; j0 += FTC_JS) {
@@ -2690,7 +2709,7 @@ template <class R, int P>
 __global__ void __launch_bounds__(FT_NT, FtrMinB<R>::v)
     k_m2l_fwd_r(const int* __restrict__ src, int ns, const int* __restrict__ child0, const R* __restrict__ up,
                 int nsurf, const int* __restrict__ conv2surf, const double* __restrict__ tw,
-                typename Spec<R>::type* __restrict__ spec, int* __restrict__ scode, uint8_t* __restrict__ win) {
+                typename Spec<R>::type* __restrict__ spec, SplitOut so) {
   using CT = typename C2<R>::type;
   constexpr int N = 2 * P, H = P + 1, CPB = FtCpb<R>::v, KS = FTR_KS;
   const int s = blockIdx.x, ch0 = blockIdx.y * CPB, tid = threadIdx.x;
@@ -2708,7 +2727,7 @@ __global__ void __launch_bounds__(FT_NT, FtrMinB<R>::v)
   __shared__ float csc[8];  // the children's power-of-two scales (mixed)
   if constexpr (sizeof(R) == 4) {
     __shared__ float red[8];
-    source_scales(up, node0, nsurf, red, csc, scode + s, win + 8ll * s);
+    source_scales(up, node0, nsurf, red, csc, so, s);
   }
   const int64_t fstride = (int64_t)N * H * ns * 8;  // kc -> kc + 1
   for (int k0 = 0; k0 < H; k0 += KS) {
@@ -2918,11 +2937,11 @@ struct Workspace {
   // Hadamard tiling: per group, tiles of TT targets; CSR over (tile, ipos) of (local target, source)
   std::vector<int> had_tile0;  // first tile of each group (ngroups + 1)
   // mixed path: tiles of k_hadamard_h (per group [had_tile0[g], had_tile0[g + 1])), their source slots,
-  // tables and output rows; scode, swin: every source's exponent code and its children's windows of the last
+  // tables and output rows; scode, slevel: every source's exponent code and its children's levels of the last
   // forward transform (one group at a time)
   DBuf<HadTile> hadh_tile;
   DBuf<int> hadh_slots, hadh_rows, scode;
-  DBuf<uint8_t> swin;
+  DBuf<uint8_t> slevel;
   DBuf<uint32_t> hadh_pslots, hadh_tpass;  // k_tile_codes
   DBuf<float> hadh_tinv;
   DBuf<uint2> hadh_tab;
@@ -3093,7 +3112,7 @@ Workspace& workspace(Fmm& f, Tree& t, cudaStream_t s) {
   if (f.mixed()) {
     XREQUIRE(maxn < (int)SPLIT_ROW_MASK, XFMM_ERR_UNSUPPORTED, "too many M2L sources");
     W.scode.alloc(maxn);
-    W.swin.alloc((size_t)maxn * 8);
+    W.slevel.alloc((size_t)maxn * 8);
   }
   int dims[3] = {f.n1, f.n1, f.n1};
   cufftType tf = cplx ? (f.mixed() ? CUFFT_C2C : CUFFT_Z2Z) : (f.mixed() ? CUFFT_R2C : CUFFT_D2Z);
@@ -3405,6 +3424,7 @@ struct Engine {
       const int tab_level = KER == K_LAPLACE ? 0 : g + 1;
       using SP = typename Spec<R>::type;
       SP* spec = (SP*)ws.specB.p;
+      const SplitOut so{ws.scode.p, ws.slevel.p, KER == K_YUKAWA || (KER == K_HELMHOLTZ && f.k_im != 0)};
       if (phase & M2L_FWD) {
         XCUDA(cudaEventRecord(ev[0], s));
         // upward equivalent DFT (fmm_scale_invariant.h:560-604) -> specB [f][s][c]
@@ -3418,8 +3438,7 @@ struct Engine {
                 ws.ft_fwd_smem = smem;
               }
               k_m2l_fwd_r<R, PP><<<dim3(ns, 8 / FtCpb<R>::v), FT_NT, smem, s>>>(
-                  src, ns, t.child0.p, (const R*)ws.up.p, n, f.conv_to_surf_up.p, f.dft_tw.p, spec, ws.scode.p,
-                  ws.swin.p);
+                  src, ns, t.child0.p, (const R*)ws.up.p, n, f.conv_to_surf_up.p, f.dft_tw.p, spec, so);
             });
             XLAUNCH();
             ws.launches++;
@@ -3433,8 +3452,7 @@ struct Engine {
               ws.ft_fwd_smem = smem;
             }
             k_m2l_fwd_c<R, PP><<<dim3(ns, 8 / FtcCpb<R>::v), FT_NT, smem, s>>>(
-                src, ns, t.child0.p, (const CT*)ws.up.p, n, f.conv_to_surf_up.p, f.dft_tw.p, spec, ws.scode.p,
-                  ws.swin.p);
+                src, ns, t.child0.p, (const CT*)ws.up.p, n, f.conv_to_surf_up.p, f.dft_tw.p, spec, so);
           });
           XLAUNCH();
           ws.launches++;
@@ -3448,12 +3466,11 @@ struct Engine {
           exec_fwd(ws.fwd[g], ws.grid.p, ws.specA.p);
           ws.launches++;
           if constexpr (sizeof(R) == 4) {  // -> [f][s][c], split
-            k_source_codes<W><<<ns, 256, 0, s>>>(src, t.child0.p, (const W*)ws.up.p, n, ws.scode.p, ws.swin.p);
+            k_source_codes<W><<<ns, 256, 0, s>>>(src, t.child0.p, (const W*)ws.up.p, n, so);
             XLAUNCH();
             const dim3 grid((nfreq + 31) / 32, ((int64_t)ns * 8 + 31) / 32);
             XREQUIRE(grid.y < 65536, XFMM_ERR_UNSUPPORTED, "transpose too tall");
-            k_transpose_split<<<grid, dim3(32, 8), 0, s>>>((const float2*)ws.specA.p, spec, ns, nfreq, ws.scode.p,
-                                                         ws.swin.p);
+            k_transpose_split<<<grid, dim3(32, 8), 0, s>>>((const float2*)ws.specA.p, spec, ns, nfreq, so);
             XLAUNCH();
             ws.launches++;
           } else {
@@ -3462,7 +3479,7 @@ struct Engine {
         }
         if (const int nht = ws.had_tile0[g + 1] - ws.had_tile0[g]; sizeof(R) == 4 && nht > 0) {
           k_tile_codes<<<nht, 256, 0, s>>>(ws.hadh_tile.p + ws.had_tile0[g], ws.hadh_slots.p, ws.scode.p,
-                                           ws.swin.p, ws.hadh_pslots.p, ws.hadh_tinv.p + ws.had_tile0[g],
+                                           ws.slevel.p, ws.hadh_pslots.p, ws.hadh_tinv.p + ws.had_tile0[g],
                                            ws.hadh_tpass.p + ws.had_tile0[g]);
           XLAUNCH();
           ws.launches++;
@@ -3510,7 +3527,7 @@ struct Engine {
               ws.hadc_btab_nf = nfreq;
             }
             k_hadamard_dc<<<dim3(ws.hadd_ld[g] / 128, (nfreq + HADC_FPB - 1) / HADC_FPB), HADC_NT, HADC_SMEM, s>>>(
-                ws.hadc_btab.p, spec, (CT*)ws.specA.p, ws.swin.p, ws.hadd_tabp.p + ws.hadd_tab0[g], ws.hadd_ld[g],
+                ws.hadc_btab.p, spec, (CT*)ws.specA.p, ws.slevel.p, ws.hadd_tabp.p + ws.hadd_tab0[g], ws.hadd_ld[g],
                 ws.hadd_row.p + ws.hadd_row0[g], ns, nt, nfreq, ws.status.p);
             XLAUNCH();
             ws.launches++;
@@ -3614,7 +3631,7 @@ struct Engine {
   static HadSys had_sys(Workspace& ws, int g, int ns, int nt) {
     return HadSys{(const SplitC*)ws.specB.p,           (float2*)ws.specA.p, ws.hadh_tile.p + ws.had_tile0[g],
                   ws.hadh_pslots.p,                    ws.hadh_tinv.p + ws.had_tile0[g],
-                  ws.hadh_tpass.p + ws.had_tile0[g],   ws.swin.p,
+                  ws.hadh_tpass.p + ws.had_tile0[g],   ws.slevel.p,
                   ws.hadh_tab.p,                       ws.hadh_rows.p,      ns,
                   nt};
   }

@@ -1,9 +1,9 @@
 """The mixed M2L Hadamard keeps its accuracy for sources far weaker than others beside them: the split spectra have
-one exponent per source node with windows for its weak children, a tile takes sources of very different
+one exponent per source node and one of their own for its weak children, a tile takes sources of very different
 exponents in several passes, and the operator's factors have windows of their own.
 
-A screened kernel shows a weak source: the strong one's field is gone where the weak one's targets are (k = 8 to
-15 per box; beyond that the FP32 check potentials limit the mixed path).  Each set of targets is compared with
+A screened kernel shows a weak source: the strong one's field is gone where the weak one's targets are (k per box
+as large as the order's FP32 check potentials allow).  Each set of targets is compared with
 the FP64 path at the same order, by its own norm.  Tolerance: the mixed path's bound, 5e-6 (a source that is
 lost, or held to a few bits, leaves 1e-4 to 1)."""
 import numpy as np
@@ -75,14 +75,15 @@ def _boxes(rng, n, cells):
     return np.concatenate(pts + [np.zeros((1, 3)), np.full((1, 3), 4.0)])
 
 
-def test_weak_child_beside_a_strong_one():
-    """Two siblings, one 1.5e-5 of the other, and targets that only the weak one's field reaches."""
+@pytest.mark.parametrize("k,p", [(15.0, 6), (25.0, 4)])
+def test_weak_child_beside_a_strong_one(k, p):
+    """Two siblings, one 1.5e-5 or 7e-10 of the other, and targets that only the weak one's field reaches."""
     rng = np.random.default_rng(1)
     n = 400
     x = _boxes(rng, n, [(0, 0, 0), (1, 0, 0)])
-    q = np.concatenate([rng.uniform(0.5, 1, n), 50 * np.exp(-15.0) * rng.uniform(0.5, 1, n), np.zeros(2)])
+    q = np.concatenate([rng.uniform(0.5, 1, n), 50 * np.exp(-k) * rng.uniform(0.5, 1, n), np.zeros(2)])
     y = _boxes(rng, n, [(3, 0, 0)])
-    mixed, full = _both("modified_helmholtz", 15.0, 6, 64, x, q, y, depth=2)
+    mixed, full = _both("modified_helmholtz", k, p, 64, x, q, y, depth=2)
     _check(mixed, full, {"targets": slice(0, n)})
 
 
