@@ -125,13 +125,10 @@ constexpr int EVAL_WARPS = 4;
 // values.  W: value type of the upward equivalent densities (M2P sources); the downward equivalent
 // densities (L2P sources) are FP64 (the pinv output).  A leaf by one warp (PARTS 1) or, with few leaves, by
 // the CTA's PARTS warps, each taking every PARTS-th chunk of 32 surface points, their sums added in order.
-#ifndef XFMM_FAR_NS32
-#define XFMM_FAR_NS32 1  // Newton steps of the FP64 far field when the working precision is FP32
-#endif
 template <int KER, class W, int PARTS>
 __global__ void __launch_bounds__(32 * EVAL_WARPS) k_eval(EvalArgs a) {
-  // with an FP32 working precision (W), one Newton step on the FP64 reciprocal square root (~2^-44)
-  using G = Green<KER, double, std::is_same<typename Base<W>::type, float>::value ? XFMM_FAR_NS32 : 2>;
+  // with an FP32 working precision (W), the short form of the FP64 reciprocal square root
+  using G = Green<KER, double, std::is_same<typename Base<W>::type, float>::value ? 1 : 2>;
   using Q = typename G::Q;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, part = PARTS > 1 ? wid : 0;
   const int w = PARTS > 1 ? (int)blockIdx.x : blockIdx.x * EVAL_WARPS + wid;
@@ -244,17 +241,12 @@ __global__ void __launch_bounds__(32 * EVAL_WARPS) k_eval(EvalArgs a) {
 // operations, 10 + 6 / p against 17 when every point's separation is formed anew.  The FP64 pipe (2 cycles
 // per operation and warp) bounds it: at 4M, p = 8 (1.18e9 pairs) 1.54 -> 1.07 ms;
 // FP64 path at 1M 0.70 -> 0.34 (two Newton steps on the instruction, where FP32 gave the seed).
-// 1/r: the FP64 reciprocal-square-root approximation instruction (relative error below 2^-22.9) and NS
-// Newton steps y <- y (3 - r^2 y^2) / 2 (1: 2^-44, for FP32 densities; 2: full FP64), the powers of two
-// carried in the staged densities.  No pair coincides: a target lies at least 1.95 r from its own downward
+// 1/r: the FP64 reciprocal-square-root approximation instruction (rsqrt_approx64) and NS Newton steps
+// y <- y (3 - r^2 y^2) / 2 (1: 2^-39.5, for FP32 densities; 2: full FP64), the powers of two carried in the
+// staged densities.  No pair coincides: a target lies at least 1.95 r from its own downward
 // surface, and W-list nodes are not adjacent to the leaf.
 // Few leaves would leave the chip idle behind the longest of them: FAR_PARTS warps then share a leaf, each
 // taking every FAR_PARTS-th line, and their sums meet in shared memory in a fixed order.
-__device__ __forceinline__ double rsqrt_approx64(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  return y;
-}
 template <int NS> struct FarScale;  // yh = KY / r after NS scaled Newton steps
 template <> struct FarScale<1> { static constexpr double KY = 2.0; };
 template <> struct FarScale<2> { static constexpr double KY = 16.0; };

@@ -47,16 +47,25 @@ __device__ __forceinline__ float2 vadd(float2 a, float2 b) { return make_float2(
 __device__ __forceinline__ double2 vadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 
 // ------------------------------------------------------------ reciprocal square root
-// FP32: the hardware approximation.  FP64: the FP64 approximation instruction (relative error below 2^-22.9)
-// refined by two Newton-Raphson steps y <- y (3 - x y^2) / 2 (quadratic convergence: 2^-44 -> full
-// precision), the same idea as the reference's rsqrt approximation + Newton steps (vec.h:655-670).  One
-// instruction where an FP32 seed needs two conversions beside its own, and no FP32 range limit: FP64 near field
-// at 1M bodies 2.32 -> 1.92 ms, Helmholtz 50k 0.99 -> 0.92; Yukawa far field 0.66 -> 0.59.
-// NS: Newton steps for FP64 (2 for FP64 results; 1, ~2^-44, where the result feeds FP32 work).
+// FP32: the hardware approximation.  FP64: the FP64 approximation instruction (relative error 9.3e-7 = 2^-20.0,
+// measured over two binades: it reads and writes 20 bits) refined by NS steps.  2, for FP64 results: Newton-Raphson
+// steps y <- y (3 - x y^2) / 2 (2^-39.5 after one, 4.0e-16 after two), the same idea as the reference's rsqrt
+// approximation + Newton steps (vec.h:655-670).  1, where the result feeds FP32 work: one third-order step (Householder),
+// y <- y (1 + e / 2 + 3 e^2 / 8) with e = 1 - x y^2, 2.2e-16 for one operation more than a Newton step.
+// One instruction where an FP32 seed needs two conversions beside its own, and no FP32 range limit: FP64 near
+// field at 1M bodies 2.32 -> 1.92 ms, Helmholtz 50k 0.99 -> 0.92.
 template <int NS = 2> __device__ __forceinline__ float rsqrt_any(float x) { return rsqrtf(x); }
-template <int NS = 2> __device__ __forceinline__ double rsqrt_any(double x) {
+__device__ __forceinline__ double rsqrt_approx64(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  return y;
+}
+template <int NS = 2> __device__ __forceinline__ double rsqrt_any(double x) {
+  double y = rsqrt_approx64(x);
+  if constexpr (NS == 1) {
+    const double e = fma(-x * y, y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
+  }
   const double hx = 0.5 * x;
 #pragma unroll
   for (int i = 0; i < NS; i++) y = y * (1.5 - hx * y * y);
