@@ -23,6 +23,7 @@
 #include <cufft.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdlib>
 #include <type_traits>
 #include <cmath>
@@ -2948,8 +2949,7 @@ struct Workspace {
   // workspace is created, by XFMM_HADAMARD_TCGEN05=1 in the environment
   bool had_tc5 = false;
   DBuf<unsigned char> hadc_btab;      // its B blocks per frequency (k_hadc_btab), built for one operator table
-  const void* hadc_btab_T = nullptr;
-  int hadc_btab_nf = 0;
+  uint64_t hadc_btab_id = 0;          // LevelOps::m2l_id of that table
   // M2L transforms: own pruned DFT kernels (real p <= 10, complex p <= 12, shared memory permitting) or
   // cuFFT on the grid
   bool fused = false;
@@ -3509,14 +3509,13 @@ struct Engine {
               ws.hadc_attr = true;
             }
             const LevelOps& op = f.ops[tab_level];
-            if (ws.hadc_btab_T != (const void*)op.m2l_frag.p || ws.hadc_btab_nf != nfreq) {  // B blocks in the MMA layout
+            if (ws.hadc_btab_id != op.m2l_id) {  // B blocks in the MMA layout
               ws.hadc_btab.reserve((size_t)nfreq * HADC_BBYTES);
               k_hadc_btab<<<std::min<int64_t>(nblk((int64_t)nfreq * 26 * 64), 148 * 16), 256, 0, s>>>(
                   (const uint4*)op.m2l_frag.p, op.m2l_binv.p, op.m2l_windows, nfreq, ws.hadc_btab.p);
               XLAUNCH();
               ws.launches++;
-              ws.hadc_btab_T = op.m2l_frag.p;
-              ws.hadc_btab_nf = nfreq;
+              ws.hadc_btab_id = op.m2l_id;
             }
             k_hadamard_dc<<<dim3(ws.hadd_ld[g] / 128, (nfreq + HADC_FPB - 1) / HADC_FPB), HADC_NT, HADC_SMEM, s>>>(
                 ws.hadc_btab.p, spec, (CT*)ws.specA.p, ws.slevel.p, ws.hadd_tabp.p + ws.hadd_tab0[g], ws.hadd_ld[g],
@@ -3791,6 +3790,8 @@ void check_ready(const Fmm& f, const Tree& t) {
 
 // ================================================================ public (internal API)
 void m2l_fragments(LevelOps& op, const double* T64, int nfreq, bool mixed, cudaStream_t s) {
+  static std::atomic<uint64_t> tables{0};
+  op.m2l_id = ++tables;
   if (!mixed) {
     op.m2l_frag.alloc((size_t)nfreq * HAD64_B * sizeof(double));
     k_m2l_fragments64<<<nblk(26ll * nfreq * 32), 256, 0, s>>>((const double2*)T64, nfreq, (double*)op.m2l_frag.p);

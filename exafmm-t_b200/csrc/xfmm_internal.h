@@ -230,6 +230,7 @@ struct LevelOps {
   DBuf<char> m2l_frag;
   DBuf<float> m2l_binv;  // mixed: [window][nfreq][32], undoes the exponent of each block
   int m2l_windows = 1;   // mixed: windows of the factors' exponents (k_m2l_fragments)
+  uint64_t m2l_id = 0;   // another number for every table built: memory addresses come again
   int rank = 0;        // singular values kept by the pinv threshold: B1 columns / B2 rows beyond are zero
   // the same operators in the form the translation GEMMs (translate.cu) read: real [K][N] row-major, a
   // complex operator expanded to [2K][2N] (expand_operator); FP64 for the pinv factors and the FP64
