@@ -27,9 +27,8 @@ from tests.golden_cases import TREE_KEYS
 pytestmark = pytest.mark.gpu
 
 FP64_TOL = 1e-9
-# a target of the M2L Hadamard with at least this many of its 26 relative positions occupied is dense;
-# a group of at least DENSE_GROUP_MIN dense targets runs the dense tensor-core form (k_hadamard_dt)
-DENSE_MIN, DENSE_GROUP_MIN = 12, 256
+# targets in a group that make several full tiles of the mixed M2L Hadamard (512 each, fewer where sources fill up)
+FULL_TILES = 1024
 
 
 def _mods():
@@ -71,15 +70,12 @@ def _reference(kernel, p, ncrit, wavek, x, q, depth):
     return out, d
 
 
-def _dense_targets(dump):
-    """Dense M2L targets per group (one group for Laplace, one per level otherwise)."""
-    m2l = dump["m2l"]
-    occ = (m2l >= 0).sum(axis=1)
-    lev = dump["ni"][:, 1]
-    return {int(l): int(((occ >= DENSE_MIN) & (lev == l)).sum()) for l in np.unique(lev[occ > 0])}
+def _m2l_targets(dump):
+    """M2L targets (nonleaf nodes with sources at some relative position), one group for Laplace."""
+    return int(((dump["m2l"] >= 0).sum(axis=1) > 0).sum())
 
 
-def _check(kernel, p, ncrit, wavek, x, q, depth=None, mixed_tol=1e-6, need_dense=False, need_wx=False):
+def _check(kernel, p, ncrit, wavek, x, q, depth=None, mixed_tol=1e-6, need_tiles=False, need_wx=False):
     ref_out, ref_dump = _reference(kernel, p, ncrit, wavek, x, q, depth)
     if need_wx:  # M2P and P2L interactions exist in this case
         assert len(ref_dump["m2p"]) > 0 and len(ref_dump["p2l"]) > 0
@@ -95,10 +91,8 @@ def _check(kernel, p, ncrit, wavek, x, q, depth=None, mixed_tol=1e-6, need_dense
             for k in TREE_KEYS:
                 assert np.array_equal(d[k], ref_dump[k]), k
             assert d["depth"] == ref_dump["depth"] and d["r0"] == ref_dump["r0"]
-            if need_dense:
-                per_level = _dense_targets(d)
-                dense = sum(per_level.values()) if kernel == "laplace" else max(per_level.values())
-                assert dense >= DENSE_GROUP_MIN, per_level  # the dense Hadamard form runs in this case
+            if need_tiles:
+                assert _m2l_targets(d) >= FULL_TILES  # several full tiles of the mixed Hadamard
         out = m.evaluate(tree, fmm)
         fmm.stage_times(tree)  # raises if a bounded device-side wait ran out
         pe, ge = orc.rel_l2(out, ref_out)
@@ -113,7 +107,7 @@ def test_cfg1_laplace_100k_nonadaptive_p8():
     rng = np.random.default_rng(0)
     x = rng.random((100_000, 3))
     q = rng.uniform(-1.0, 1.0, 100_000)
-    _check("laplace", 8, 64, 0.0, x, q, depth=4, need_dense=True)
+    _check("laplace", 8, 64, 0.0, x, q, depth=4, need_tiles=True)
 
 
 def test_cfg2_laplace_4m_p8():
@@ -122,7 +116,7 @@ def test_cfg2_laplace_4m_p8():
     n = 4_000_000
     x = np.random.default_rng(0).random((n, 3))
     q = np.random.default_rng(1).uniform(-1.0, 1.0, n)
-    _check("laplace", 8, 128, 0.0, x, q, need_dense=True)
+    _check("laplace", 8, 128, 0.0, x, q, need_tiles=True)
 
 
 def test_cfg2_laplace_1m_p10():
@@ -130,7 +124,7 @@ def test_cfg2_laplace_1m_p10():
     n = 1_000_000
     x = np.random.default_rng(0).random((n, 3))
     q = np.random.default_rng(1).uniform(-1.0, 1.0, n)
-    _check("laplace", 10, 128, 0.0, x, q, need_dense=True)
+    _check("laplace", 10, 128, 0.0, x, q, need_tiles=True)
 
 
 def test_cfg3_yukawa_sphere_p10():

@@ -88,7 +88,7 @@ def test_weak_child_beside_a_strong_one(k, p):
 
 
 def test_far_child_beside_a_near_one():
-    """One source cell, and target cells whose operator entries differ by the screening, 1e-9 and less within a block."""
+    """One source cell, and target cells whose operator entries differ by the screening (1e-9 in a block)."""
     rng = np.random.default_rng(2)
     n = 400
     x = _boxes(rng, n, [(0, 0, 0)])

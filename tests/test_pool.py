@@ -47,6 +47,75 @@ def test_reused_blocks_and_return():
     assert torch.cuda.mem_get_info()[0] >= free0 - (8 << 20)
 
 
+def _other(kernel, precision, p):
+    import exafmm.helmholtz as hel
+    import exafmm.laplace as lap
+    import exafmm.modified_helmholtz as yuk
+    m = {"laplace": lap, "modified_helmholtz": yuk, "helmholtz": hel}[kernel]
+    make = {"laplace": lambda: lap.LaplaceFmm(p, 40, precision=precision),
+            "modified_helmholtz": lambda: yuk.ModifiedHelmholtzFmm(p, 40, 4.0, precision=precision),
+            "helmholtz": lambda: hel.HelmholtzFmm(p, 40, 4.0 + 1.0j, precision=precision)}[kernel]
+    return m, make
+
+
+def _solve(kernel, precision, p, seed, n):
+    m, make = _other(kernel, precision, p)
+    fmm = make()
+    rng = np.random.default_rng(seed)
+    g = rng.standard_normal((n, 3))
+    x = g / np.linalg.norm(g, axis=1)[:, None] * (0.05 + rng.random(n) ** 3)[:, None]
+    q = rng.uniform(-1, 1, n) + (1j * rng.uniform(-1, 1, n) if kernel == "helmholtz" else 0)
+    tree = m.setup(m.init_sources(x, q), m.init_targets(x), fmm)
+    return m.evaluate(tree, fmm)
+
+
+# p = 11: the real kernels' transforms run through cuFFT, with grids of their own
+PATHS = [("laplace", "mixed", 6), ("modified_helmholtz", "mixed", 5), ("modified_helmholtz", "fp64", 4),
+         ("helmholtz", "mixed", 5), ("helmholtz", "fp64", 4), ("laplace", "mixed", 11)]
+
+
+def test_blocks_of_one_path_serve_another():
+    """Every path of the evaluate on blocks that held another's tables, counters and spectra."""
+    sizes = [(1, 12000), (2, 3000), (3, 20000)]
+    want = {}
+    for path in PATHS:
+        for s in sizes:
+            want[path, s] = _solve(*path, *s)  # nothing is kept: the handle is freed after each
+            gc.collect()
+    keep = _fmm()
+    for r in range(2):
+        for s in sizes:
+            for path in PATHS[::-1] if r else PATHS:
+                got = _solve(*path, *s)
+                # close pairs of the mixed Laplace path meet in FP64 atomic sums
+                assert np.linalg.norm(got - want[path, s]) <= 1e-13 * np.linalg.norm(want[path, s]), (path, s)
+    del keep
+
+
+def test_batch_on_blocks_of_other_systems():
+    from exafmm.batch import BatchedFmm, batched_workload
+    import exafmm.laplace as lap
+    systems = batched_workload(nsys=6, nmin=2000, nmax=9000, seed=3)
+    for precision, tol in (("fp64", 0.0), ("mixed", 1e-13)):
+        def batch():
+            return BatchedFmm(systems, lambda: lap.LaplaceFmm(4, 64, precision=precision))
+        b = batch()
+        want = [o.clone() for o in b.evaluate_batch(2)]
+        torch.cuda.synchronize()
+        del b
+        gc.collect()
+        keep = _fmm()
+        for path in PATHS[:3]:
+            _solve(*path, 5, 15000)
+        b = batch()
+        got = b.evaluate_batch(2)
+        torch.cuda.synchronize()
+        for g, w in zip(got, want):
+            assert float((g - w).norm()) <= tol * float(w.norm())
+        del b, keep
+        gc.collect()
+
+
 def test_threads():
     want = {s: _step(_fmm(), s, 8000 + 1000 * s) for s in range(4)}
     bad = []
