@@ -1,23 +1,22 @@
 // evaluate.cu -- upward and downward passes of the KIFMM on the GPU.
 //
-// Stage map (reference -> here):
+// Stage map (reference -> here); translation GEMMs: translate.cu, which gathers, scales and scatters the rows:
 //   P2M   fmm_scale_invariant.h:163-195 / fmm.h:156-185  k_surf_pot (Laplace mixed: k_surf_pot_lap_f2) check
-//                                                        potentials + row gather, two FP64 library GEMMs
-//                                                        (pinv factors), scaled scatter (0.5^l)
-//   M2M   fmm_scale_invariant.h:233-253 / fmm.h:221-241  row gather + library GEMM per level, K = 8 nsurf
-//   P2L   fmm_base.h:127-154                             k_p2l
-//   M2L   fmm_scale_invariant.h:407-440, 560-646;        real kernels: k_m2l_fwd_r + k_hadamard_h (opt-in:
-//         fmm.h:395-446, 631-788                         k_hadamard_dc on tcgen05) + k_m2l_bwd_r (FP64:
-//                                                        k_hadamard, k_m2l_bwd); complex kernel (p <= 12): k_m2l_fwd_c
-//                                                        + Hadamard + k_m2l_bwd_c; real p > 10 or p > 12:
-//                                                        k_m2l_grid_up + cuFFT + k_transpose + Hadamard +
-//                                                        k_transpose + cuFFT + k_m2l_gather_dn
-//   L2L   fmm_scale_invariant.h:256-275 / fmm.h:244-263  row gather + library GEMM per level, N = 8 nsurf
-//   L2P   fmm_scale_invariant.h:198-230 / fmm.h:188-218  scaled row gather, two library GEMMs (the mixed
-//                                                        path's first factor FP32), scatter; then the far
-//                                                        part of the target evaluation
-//   M2P   fmm_base.h:97-124                              far part: k_eval (Laplace mixed: k_far_lap)
-//   P2P   fmm_base.h:82-94                               near part: k_near (Laplace mixed: k_near_lap_f2)
+//                                                        potentials, two tgemm_f64 (pinv factors, scale 0.5^l)
+//   M2M   fmm_scale_invariant.h:233-253 / fmm.h:221-241  per level, K = 8 nsurf: tgemm_tc (FP64: tgemm_f64)
+//   P2L   fmm_base.h:127-154                             k_surf_pot
+//   M2L   fmm_scale_invariant.h:407-440, 560-646;        real kernels, p <= 10: k_m2l_fwd_r + Hadamard + k_m2l_bwd_r
+//         fmm.h:395-446, 631-788                         (FP64: k_m2l_bwd); complex kernel, p <= 12: k_m2l_fwd_c +
+//                                                        Hadamard + k_m2l_bwd_c; beyond: k_m2l_grid_up + cuFFT +
+//                                                        k_transpose(_split) + Hadamard + k_transpose + cuFFT +
+//                                                        k_m2l_gather_dn.  Hadamard: k_hadamard_h (opt-in for dense
+//                                                        targets: k_hadamard_dc on tcgen05); FP64: k_hadamard_d64
+//   L2L   fmm_scale_invariant.h:256-275 / fmm.h:244-263  per level, N = 8 nsurf: tgemm_tc (FP64: tgemm_f64)
+//   L2P   fmm_scale_invariant.h:198-230 / fmm.h:188-218  two translation GEMMs (mixed, real kernels: the first
+//                                                        tgemm_tc), then the far part of the target evaluation
+//   M2P   fmm_base.h:97-124                              far part: k_eval (Laplace: k_far_lap)
+//   P2P   fmm_base.h:82-94                               near part: k_near (Laplace mixed: k_near_lap_f2), few
+//                                                        leaves: k_near_parts, k_near_lap_f2_parts
 // Results stay in tree order until get_values scatters them (python/exafmm.cpp:194-207).
 #include <cuda_fp16.h>
 #include <cufft.h>
@@ -63,18 +62,10 @@ template <> __device__ __forceinline__ double2 load_charge<double2>(const double
   return make_double2(s.w, qim[j]);
 }
 
-template <class To> __device__ __forceinline__ To cvt(float v);
-template <class To> __device__ __forceinline__ To cvt(double v);
-template <class To> __device__ __forceinline__ To cvt(float2 v);
-template <class To> __device__ __forceinline__ To cvt(double2 v);
-template <> __device__ __forceinline__ float cvt<float>(float v) { return v; }
-template <> __device__ __forceinline__ float cvt<float>(double v) { return (float)v; }
-template <> __device__ __forceinline__ double cvt<double>(float v) { return (double)v; }
-template <> __device__ __forceinline__ double cvt<double>(double v) { return v; }
-template <> __device__ __forceinline__ float2 cvt<float2>(float2 v) { return v; }
-template <> __device__ __forceinline__ float2 cvt<float2>(double2 v) { return make_float2((float)v.x, (float)v.y); }
-template <> __device__ __forceinline__ double2 cvt<double2>(float2 v) { return make_double2(v.x, v.y); }
-template <> __device__ __forceinline__ double2 cvt<double2>(double2 v) { return v; }
+__device__ __forceinline__ double to64(float v) { return (double)v; }
+__device__ __forceinline__ double to64(double v) { return v; }
+__device__ __forceinline__ double2 to64(float2 v) { return make_double2(v.x, v.y); }
+__device__ __forceinline__ double2 to64(double2 v) { return v; }
 
 // FP64 accumulation of FP32/FP64 partials
 __device__ __forceinline__ void acc64(double& a, float b) { a += (double)b; }
@@ -101,15 +92,14 @@ __device__ __forceinline__ void put_out(double* o, double2 v, double s, int acc)
   o[1] = acc ? o[1] + v.y * s : v.y * s;
 }
 
-// ================================================================ target evaluation (P2P + M2P + L2P)
+// ================================================================ far field (M2P + L2P)
 struct EvalArgs {
-  const int *eval_leafs, *leafs, *nsrcs, *ntrgs, *level;
+  const int *eval_leafs, *leafs, *ntrgs;
   int n_eval;
-  const int64_t *sbeg, *tbeg;
-  const double4 *center, *src4, *trg4;
-  const double* src_qim;
-  const int64_t *p2p_off, *m2p_off;
-  const int *p2p, *m2p;
+  const int64_t* tbeg;
+  const double4 *center, *trg4;
+  const int64_t* m2p_off;
+  const int* m2p;
   const double* surf_base;
   const int* surf_perm;     // surface points in line order (far_surface)
   const double* surf_grid;  // the p grid coordinates of the unit surface
@@ -189,7 +179,7 @@ __global__ void __launch_bounds__(32 * EVAL_WARPS) k_eval(EvalArgs a) {
     for (int64_t e = a.m2p_off[node]; e < a.m2p_off[node + 1]; e++) {
       const int s = a.m2p[e];
       const double4 cs = a.center[s];
-      surface(cs.x - c.x, cs.y - c.y, cs.z - c.z, 1.05 * cs.w, [&](int k) { return cvt<Q>(upv[(int64_t)s * n + k]); });
+      surface(cs.x - c.x, cs.y - c.y, cs.z - c.z, 1.05 * cs.w, [&](int k) { return to64(upv[(int64_t)s * n + k]); });
     }
     // L2P: own downward equivalent surface (2.95 box, fmm_scale_invariant.h:221-228)
     surface(0.0, 0.0, 0.0, 2.95 * c.w, [&](int k) { return eqv[(int64_t)pos * n + k]; });
@@ -2927,8 +2917,7 @@ struct Workspace {
   // M2L
   DBuf<char> grid, specA, specB;
   std::vector<cufftHandle> fwd, bwd;
-  // Hadamard tiling: per group, tiles of TT targets; CSR over (tile, ipos) of (local target, source)
-  std::vector<int> had_tile0;  // first tile of each group (ngroups + 1)
+  std::vector<int> had_tile0;  // first tile of each group (ngroups + 1; k_hadamard_h)
   // mixed path: tiles of k_hadamard_h (per group [had_tile0[g], had_tile0[g + 1])), their source slots,
   // tables and output rows; scode, slevel: every source's exponent code and its children's levels of the last
   // forward transform (one group at a time)
@@ -3629,11 +3618,9 @@ struct Engine {
 
   // the far field (M2P + L2P evaluation), added to the near field's values
   static EvalArgs far_args(Fmm& f, Tree& t, Workspace& ws) {
-    return EvalArgs{t.eval_leafs.p, t.leafs.p, t.nsrcs.p,   t.ntrgs.p, t.level.p, t.n_eval_leafs, t.sbeg.p,
-               t.tbeg.p,       t.center.p, t.src4.p,   t.trg4.p,  t.src_qim.p, t.p2p_off.p,  t.m2p_off.p,
-               t.p2p.p,        t.m2p.p,   f.surf_base.p, f.surf_perm.p, f.surf_grid.p, f.nsurf, ws.up.p,
-               ws.eq.p,        ws.out.p,
-               f.k_re,         f.k_im};
+    return EvalArgs{t.eval_leafs.p, t.leafs.p,     t.ntrgs.p,     t.n_eval_leafs, t.tbeg.p, t.center.p,
+                    t.trg4.p,       t.m2p_off.p,   t.m2p.p,       f.surf_base.p,  f.surf_perm.p, f.surf_grid.p,
+                    f.nsurf,        ws.up.p,       ws.eq.p,       ws.out.p,       f.k_re,   f.k_im};
   }
 
   static NearArgs near_args(Fmm& f, Tree& t, Workspace& ws) {

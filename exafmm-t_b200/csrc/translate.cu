@@ -234,7 +234,7 @@ __device__ __forceinline__ void split_tf32(float x, uint32_t& h, uint32_t& l) {
 // ---------------------------------------------------------------- FP32 accuracy on tcgen05 (TF32 x 3)
 // C = alpha A B on the sm_100 tensor cores (tcgen05).  A CTA owns 128 rows (one per TMEM
 // lane), 64 columns and a range of 16-wide K steps (K split over blockIdx.z when a level has few rows;
-// the parts are then added into C with atomics, C already holding the rows' starting values).
+// k_tc_finish then adds the parts in order).
 // Per step: the rows' A pieces arrive raw by cp.async two steps ahead (16 bytes per lane, coalesced), in
 // place into the stage's A-tail tile or into a raw buffer, and are split into TF32 head and tail one step
 // ahead as K-major core matrices (8 rows x 16 bytes, 128 contiguous bytes each); the operator's head and

@@ -120,7 +120,7 @@ xfmm_status xfmm_tree_dump(const xfmm_tree* tree, double* geo, uint64_t* key, in
 /* Device times (ms, CUDA events) of the last upward + downward pass on this tree: P2M, M2M, P2L,
  * M2L, L2L, L2P check-to-equivalent, target evaluation (P2P + M2P + L2P), total; then the M2L
  * sub-stages forward transform, Hadamard, backward transform; the number of this library's kernel
- * launches in the last evaluate (library GEMM and FFT launches not counted); then the target
+ * launches in the last evaluate (those of cuFFT, at orders beyond the transform kernels, not counted); then the target
  * evaluation split into its near field (P2P) and far field (M2P + L2P) (14 doubles).  Waits for the
  * last pass to finish; XFMM_ERR_TIMEOUT when a bounded device-side wait of that pass ran out (its
  * results are then incomplete). */
