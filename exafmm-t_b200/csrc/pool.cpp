@@ -139,10 +139,12 @@ void pool_unhold() noexcept {
 }
 
 bool Uses::wait() const noexcept {
-  if (captured) return false;
+  if (unknown) return false;
   RelaxedCapture relaxed;
   for (const auto& u : last)
     if (cudaEventSynchronize(u.second->e) != cudaSuccess) return false;
+  for (const auto& u : graphs)
+    if (cudaEventSynchronize(u->e) != cudaSuccess) return false;
   return true;
 }
 
@@ -152,18 +154,25 @@ UseScope::UseScope(cudaStream_t s, std::vector<Uses*> objects)
     std::lock_guard<std::mutex> lock(pool().m);
     begin_ = pool().allocations;
   }
-  if (capturing_)
-    for (Uses* u : objects_) u->captured = true;
   t_scope = this;
 }
 
 UseScope::~UseScope() {
   t_scope = outer_;
-  if (capturing_ || objects_.empty()) return;
+  if (objects_.empty()) return;
   try {
     unsigned long long id = 0;
     std::shared_ptr<Uses::Event> ev;
-    bool ok = cudaStreamGetId(s_, &id) == cudaSuccess;
+    if (capturing_) {
+      ev = std::make_shared<Uses::Event>();
+      if (cudaEventCreateWithFlags(&ev->e, cudaEventDisableTiming) == cudaSuccess &&
+          cudaEventRecordWithFlags(ev->e, s_, cudaEventRecordExternal) == cudaSuccess) {
+        for (Uses* u : objects_)
+          if (u->graphs.empty() || u->graphs.back() != ev) u->graphs.push_back(ev);
+        return;
+      }
+    }
+    bool ok = !capturing_ && cudaStreamGetId(s_, &id) == cudaSuccess;
     // the stream's event of one of the objects, recorded again: all earlier work of the stream is before it
     for (Uses* u : objects_)
       for (auto& l : u->last)
@@ -183,7 +192,7 @@ UseScope::~UseScope() {
     cudaGetLastError();
   } catch (...) {
   }
-  for (Uses* u : objects_) u->captured = true;  // nothing tells the end of this work
+  for (Uses* u : objects_) u->unknown = true;
 }
 
 bool UseScope::idle(uint64_t allocated) const noexcept {

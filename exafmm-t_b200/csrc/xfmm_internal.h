@@ -49,8 +49,8 @@ void pool_release(void* p, size_t capacity) noexcept;
 void pool_hold();            // an Fmm handle was created
 void pool_unhold() noexcept;  // ... was freed
 
-// The device work that used an object: per stream (by its id) an event behind the last of it, and whether some
-// was captured into a graph, which may be replayed at any time.  Like the handles, for one thread at a time.
+// The device work that used an object: per stream (by its id) an event behind the last of it, and per call that was
+// captured an event that every launch of the graph records.  Like the handles, for one thread at a time.
 struct Uses {
   struct Event {
     cudaEvent_t e = nullptr;
@@ -62,8 +62,9 @@ struct Uses {
     }
   };
   std::vector<std::pair<unsigned long long, std::shared_ptr<Event>>> last;
-  bool captured = false;
-  bool wait() const noexcept;  // waits for the work; false: some was captured, or an error
+  std::vector<std::shared_ptr<Event>> graphs;
+  bool unknown = false;        // work that no event tells the end of
+  bool wait() const noexcept;  // waits for the work; false: unknown, or an error
 };
 // One call of the C API: its work on stream s uses the objects; they learn of it at the end of the scope.  Blocks that
 // the scope allocated itself are idle once s is, others once the objects' earlier work is done too.

@@ -168,25 +168,88 @@ def test_freeing_a_tree_leaves_another_threads_capture_alone():
     assert bool((a == 2).all()) and torch.equal(out, want)
 
 
+def _setup_on(stream, fmm, x, q):
+    """laplace.setup with its work on a stream."""
+    import ctypes
+    from exafmm import _core, _lib
+    L, st, h = _lib.lib(), ctypes.c_void_p(stream.cuda_stream), ctypes.c_void_p()
+    p = ctypes.c_void_p(x.data_ptr())
+    _lib.check(L.xfmm_build_tree(fmm._h, p, len(x), p, len(x), -1, 1, st, ctypes.byref(h)))
+    tree = _core.Tree(h, fmm, len(x), len(x))
+    for f in (L.xfmm_build_list, L.xfmm_m2l_setup, L.xfmm_precompute):
+        _lib.check(f(fmm._h, h, st))
+    _lib.check(L.xfmm_set_charges(fmm._h, h, ctypes.c_void_p(q.data_ptr()), 1, st))
+    return tree
+
+
+def _evaluate_on(stream, fmm, tree, out):
+    import ctypes
+    from exafmm import _lib
+    _lib.check(_lib.lib().xfmm_evaluate(fmm._h, tree._h, ctypes.c_void_p(out.data_ptr()), 1,
+                                        ctypes.c_void_p(stream.cuda_stream)))
+
+
+def _inputs(seeds, n):
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    xs = [torch.rand(n, 3, dtype=torch.float64, device="cuda", generator=gen) for _ in seeds]
+    qs = [torch.rand(n, dtype=torch.float64, device="cuda", generator=gen) - 0.5 for _ in seeds]
+    outs = [torch.zeros(n, 4, dtype=torch.float64, device="cuda") for _ in seeds]
+    torch.cuda.synchronize()
+    return xs, qs, outs
+
+
 def test_blocks_of_a_tree_freed_with_work_in_flight():
     """A tree evaluated on one stream and freed at once, the next one set up on another stream in its memory."""
-    import exafmm.laplace as lap
-    fmm = _fmm()
-    seeds, n = range(6), 60000
+    fmm, n, k = _fmm(), 60000, 6
+    xs, qs, outs = _inputs(range(k), n)
+    streams = [torch.cuda.Stream() for _ in range(2)]
     want = []
-    for s in seeds:
-        o = torch.empty(n, 4, dtype=torch.float64, device="cuda")
-        lap.evaluate(_tree(fmm, s, n), fmm, out=o)
+    for i in range(k):
+        o = torch.zeros_like(outs[i])
+        tree = _setup_on(streams[0], fmm, xs[i], qs[i])
+        torch.cuda.synchronize()
+        _evaluate_on(streams[0], fmm, tree, o)
         torch.cuda.synchronize()
         want.append(o)
-    streams, outs = [torch.cuda.Stream() for _ in range(2)], []
-    for s in seeds:
-        with torch.cuda.stream(streams[s % 2]):
-            outs.append(torch.empty(n, 4, dtype=torch.float64, device="cuda"))
-            tree = _tree(fmm, s, n)
-            for _ in range(3):
-                lap.evaluate(tree, fmm, out=outs[-1])
-            del tree
+        del tree
+    for i in range(k):
+        tree = _setup_on(streams[i % 2], fmm, xs[i], qs[i])
+        for _ in range(4):
+            _evaluate_on(streams[i % 2], fmm, tree, outs[i])
+        del tree
     torch.cuda.synchronize()
     for o, w in zip(outs, want):
         assert torch.equal(o, w)
+
+
+def test_memory_of_a_captured_tree_is_reused_only_after_its_replays():
+    """A graph of evaluates launched several times, its tree freed at once, the next one set up in its memory."""
+    fmm, n = _fmm(), 60000
+    (x, x2), (q, q2), (out, other) = _inputs(range(2), n)
+    s, s2 = torch.cuda.Stream(), torch.cuda.Stream()
+    want = torch.zeros_like(out)
+    tree = _setup_on(s, fmm, x, q)
+    _evaluate_on(s, fmm, tree, want)
+    torch.cuda.synchronize()
+    for r in range(3):
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            for _ in range(4):
+                _evaluate_on(s, fmm, tree, out)
+        out.zero_()
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        with torch.cuda.stream(s2):
+            for _ in range(5):
+                g.replay()
+        del tree  # with launches in flight
+        tree = _setup_on(s, fmm, x2, q2)
+        _evaluate_on(s, fmm, tree, other)
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
+        assert r == 0 or torch.cuda.mem_get_info()[0] >= free - (8 << 20)  # the tree's blocks are used again
+        del tree, g
+        tree = _setup_on(s, fmm, x, q)
+        _evaluate_on(s, fmm, tree, out)
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
