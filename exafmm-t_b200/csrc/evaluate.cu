@@ -1448,9 +1448,9 @@ constexpr int HADC_TT = 512;  // padding of its source table
 // twice the targets of a spatially compact tile, each used by up to 26 of them) are brought into shared
 // memory once, on the exponent of the strongest, and every A fragment is read from there with ldmatrix, whose lanes
 // address the rows of a fragment freely: a gather without register moves at 8 shared-memory cycles per 16
-// targets and position.  Measured, Hadamard stage: 1M bodies, p = 10: 2.95 ms (the same products gathered
+// targets and position.  Measured, Hadamard stage: 1M bodies, p = 10: 2.78 ms (the same products gathered
 // row by row from L1 at 14 cycles per 16 targets: 4.03; the TF32 form with per-use conversions before it:
-// 5.26); 4M, p = 8, whose deepest level has ~7 of 26 positions occupied: 4.38 (TF32 with packed rounds of
+// 5.26); 4M, p = 8, whose deepest level has ~7 of 26 positions occupied: 4.10 (TF32 with packed rounds of
 // pairs and atomics: 6.15); Helmholtz 200k, p = 12: 1.71 (3.55).
 // Bank conflicts: a source's slot is 8 k + (octant of the source in its parent).  The sources of 8 sibling
 // targets at one relative position have 8 different octants, so their 64-byte rows (four 16-byte chunks,
@@ -1462,7 +1462,7 @@ constexpr int HADC_TT = 512;  // padding of its source table
 // accumulators: weak sources keep their 22 bits.  The same for the windows of the operator.
 // Tiles with at most 256, 128 or 64 targets split the 26 positions over 2, 4 or 8 warps per 64 targets.
 // Bounds per 64 targets and position and SM (cycles): MMAs 24 x 8 / 4 = 48; shared memory 32 (A) + 8 (B).
-// At 1M, p = 8 the tensor pipe is 54% and the shared-memory pipe 64% busy: 16 warps per SM hide the rest of
+// At 1M, p = 8 the tensor pipe is 58% and the shared-memory pipe 70% busy: 16 warps per SM hide the rest of
 // the latencies only in part.  Smaller tiles at three CTAs per SM (384 targets, 704 slots) close early in
 // full volumes (p = 10: 3.83 ms); several tiles per CTA gain nothing.
 constexpr int HADH_NT = 256, HADH_TT = 512;      // threads, targets per tile
