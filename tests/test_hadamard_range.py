@@ -108,3 +108,46 @@ def test_weak_half_of_a_full_volume(tcgen05, monkeypatch):
     q = rng.uniform(-1, 1, n) * np.where(x[:, 0] < 0.25, 1.0, 1e-9)
     mixed, full = _both("modified_helmholtz", 80.0, 5, 20, x, q, x)
     _check(mixed, full, {"strong": x[:, 0] < 0.25, "weak": x[:, 0] > 0.75})
+
+
+def test_several_tiles_per_cta():
+    """Tiles of several passes and an operator of two windows, one after another in a CTA: the bits of one tile each."""
+    import exafmm.modified_helmholtz as yuk
+    rng = np.random.default_rng(4)
+    n = 60000
+    x = rng.random((n, 3))
+    q = rng.uniform(-1, 1, n) * np.where(x[:, 0] < 0.25, 1.0, 1e-9)
+    fmm = yuk.ModifiedHelmholtzFmm(4, 12, 80.0, precision="mixed")
+    tree = yuk.setup(yuk.init_sources(x, q), yuk.init_targets(x), fmm)
+    ref = yuk.evaluate(tree, fmm)
+    for tiles in (3, 64):
+        tree.set_tuning("sparse_hadamard_tiles_per_cta", tiles)
+        assert np.array_equal(yuk.evaluate(tree, fmm), ref)
+
+
+def test_batch_with_weak_sources():
+    """The batch's one-launch Hadamard takes a tile's passes too: the weak balls' gradients are as near to FP64 as
+    those of single evaluates (which FP32 stages of both bound), within a factor of two for another rounding."""
+    torch = pytest.importorskip("torch")
+    import exafmm.laplace as lap
+    from exafmm.batch import BatchedFmm
+    rng = np.random.default_rng(6)
+    n, systems = 2000, []
+    for k in range(3):
+        x = np.concatenate([_ball(rng, n, (0, 0, 0), 0.05), _ball(rng, n, (1000, 100 * k, 0), 0.05)])
+        q = rng.uniform(-1, 1, 2 * n)
+        q[n:] *= 1e-7
+        systems.append((x, q))
+    full = BatchedFmm(systems, lambda: lap.LaplaceFmm(6, 32, precision="fp64"))
+    want = [o.clone().cpu().numpy() for o in full.evaluate_each()]
+    b = BatchedFmm(systems, lambda: lap.LaplaceFmm(6, 32, precision="mixed"))
+    one = [o.clone().cpu().numpy() for o in b.evaluate_each()]
+    all_ = [o.clone().cpu().numpy() for o in b.evaluate_batch(2)]
+
+    def err(a, w, rows):
+        return np.linalg.norm(a[rows, 1:] - w[rows, 1:]) / np.linalg.norm(w[rows, 1:])
+    for a, o, w in zip(all_, one, want):
+        for rows in (slice(0, n), slice(n, 2 * n)):
+            assert err(a, w, rows) <= 2 * err(o, w, rows)
+        assert err(o, w, slice(n, 2 * n)) < 1e-3  # weak sources dropped: 1e-2
+    torch.cuda.synchronize()
