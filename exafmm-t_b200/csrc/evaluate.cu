@@ -1373,52 +1373,66 @@ __global__ void __launch_bounds__(HAD64_NT, 2)
 // frequency-major, (frequency f, node, child c) at [(f * nrows + node) * 8 + c]: a CTA (one frequency)
 // reads its sources from one block of the spectra and writes its rows contiguously.
 //
-// The mixed path's spectra are stored split: a real x of a child's spectrum is the pair of FP16 values
-// h = fp16(2^e x), t = fp16(2^e x - h): 22 bits of x within 2^-17 of the top (2^15), an absolute error below
-// 2^-39 of it elsewhere.  Every spectrum value of a child is at most the sum of its densities' magnitudes,
-// its bound.  A source node has one exponent e, set by its strongest child.  With the unscreened kernels a weak
-// child's error stays far below the FP32 rounding of its siblings' fields, which reach the same targets at a
-// comparable distance.  A screened kernel shows a weak child (the strong one's field is gone where its own targets
-// are), so there every child has its level, the steps of 2 bits by which its bound lies below the node's, and
-// those from 9 steps on the exponent e + 18, from 18 on e + 36 and so on: every child keeps an error below
-// 2^-21 of its own bound.  A split spectrum has the size of the FP32 one, the products need no conversion (the
+// The mixed path's spectra are stored split: a real x is the pair of FP16 values h = fp16(2^e x) and
+// t = fp16(c (2^e x - h)).  A split spectrum has the size of the FP32 one, the products need no conversion (the
 // operator's blocks are split the same way, k_m2l_fragments), and an FP16 MMA does twice the work of a TF32 one
 // in the same 8 cycles (measured: m16n8k16 f16 and m16n8k8 tf32 both 8.0 cycles per warp and SM quadrant) with
 // the same 11-bit significands.  A child's complex value is the 8 bytes {h.re, h.im, t.re, t.im}.
+// Every spectrum value of a child is at most the sum of its densities' magnitudes, its bound, and no error may
+// show beside the FP32 rounding of what reaches the same targets.  Two forms:
+//  * Laplace, Helmholtz with a real wavenumber: c = 1, one exponent per source node, set by its strongest child.
+//    22 bits within 2^-17 of the top (2^15), an absolute error below 2^-39 of it elsewhere: far below the
+//    rounding of the strongest child's field, which reaches the same targets at a comparable distance.
+//  * Screened kernels (modified Helmholtz, complex wavenumbers) show weak sources, for a strong one's field is
+//    gone where a weak one's targets are: c = 2^11, which keeps 22 bits down to 2^-29 of the top and an
+//    absolute error below 2^-51 of it.  The largest bound of a group's sources (k_source_bounds) sets e0, and the
+//    children are sorted into windows of 2^-28 below it, window w with the exponent e0 + 28 w: the error of
+//    a value is at most 2^-23 of its own child's bound (the FP32 transform itself rounds at 2^-24 of it).
 using SplitC = uint2;
+constexpr float SPLIT_TAIL = 2048.f;  // c of the screened kernels
 __device__ __forceinline__ uint32_t h2_bits(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
 __device__ __forceinline__ float2 h2_float2(uint32_t u) { return __half22float2(*reinterpret_cast<__half2*>(&u)); }
-__device__ __forceinline__ SplitC split16(float re, float im) {
+__device__ __forceinline__ SplitC split16(float re, float im, float c) {
   const __half2 h = __floats2half2_rn(re, im);
   const float2 hf = __half22float2(h);
-  return make_uint2(h2_bits(h), h2_bits(__floats2half2_rn(re - hf.x, im - hf.y)));
+  return make_uint2(h2_bits(h), h2_bits(__floats2half2_rn((re - hf.x) * c, (im - hf.y) * c)));
 }
+__device__ __forceinline__ float pow2f(int e) { return e >= -126 ? __uint_as_float((uint32_t)(127 + e) << 23) : 0.f; }
+__device__ __forceinline__ int float_exp(float b) { return (int)(__float_as_uint(b) >> 23) - 127; }  // b >= 0
 // The exponent e of a node whose spectrum values are at most `bound` in magnitude: 2^e bound < 2^15 (FP16
 // holds 2^16), e odd, as the code k = (127 - e) / 2 in 1..126, so that 2^-e is the float whose exponent
-// field is 2 k.
+// field is 2 k.  SPLIT_ZERO beside it: a node without values.
 __device__ __forceinline__ int split_code(float bound) {
-  int e = bound > 0.f ? 14 - ((int)(__float_as_uint(bound) >> 23) - 127) : 1;
+  int e = bound > 0.f ? 14 - float_exp(bound) : 1;
   e = max(-125, min(125, e));
   if (!(e & 1)) e -= 1;
   return (127 - e) >> 1;
 }
-constexpr int SPLIT_WIN = 9;   // steps of 2 bits between the windows of a node's children and of the operator's pairs
-constexpr int SPLIT_PASS = 10;  // steps that one pass over a tile covers: 2^-18 from its strongest source to its weakest
-constexpr int SPLIT_DEEP = 0x100, SPLIT_ZERO = 0x200;  // beside a source's code: children at levels > 0; no values
-__device__ __forceinline__ float pow2f(int e) { return e >= -126 ? __uint_as_float((uint32_t)(127 + e) << 23) : 0.f; }
-__device__ __forceinline__ float split_scale(int code, int level = 0) {
-  return pow2f(127 - 2 * (code - level / SPLIT_WIN * SPLIT_WIN));
+constexpr int SPLIT_ZERO = 0x100;
+__device__ __forceinline__ float split_scale(int code) { return __uint_as_float((uint32_t)(254 - 2 * code) << 23); }
+// Screened kernels: e0, a window's exponent, the window of a child.
+constexpr int SPLIT_WIN = 28;
+__device__ __forceinline__ int split_exp0(float bound) { return bound > 0.f ? min(126, 14 - float_exp(bound)) : 0; }
+__device__ __forceinline__ int split_exp(int e0, int w) { return min(126, e0 + SPLIT_WIN * w); }
+__device__ __forceinline__ int split_window(float bound, int e0) {
+  return bound > 0.f ? max(0, 14 - e0 - float_exp(bound)) / SPLIT_WIN : 0;
 }
-// the level of a child with bound c of a node with bound b (its scale is still a float)
-__device__ __forceinline__ int split_level(float c, float b, int code) {
-  if (!(c > 0.f)) return 0;
-  const int below = (int)(__float_as_uint(b) >> 23) - (int)(__float_as_uint(c) >> 23);
-  return min(max(0, below) / 2, (code - 1) / SPLIT_WIN * SPLIT_WIN + SPLIT_WIN - 1);
-}
+struct SplitHead {
+  unsigned gmax, done;  // largest bound so far (float bits) and finished blocks: zero between uses
+  int e0;
+  unsigned mask;        // bit w: a child in window w
+};
+// what a forward transform reads and writes beside the spectra; head null: not screened
+struct SplitOut {
+  int* code;
+  const float* bound;
+  uint8_t* win;
+  SplitHead* head;
+};
 // Packed sources: the source row in the low 25 bits (2^25 sources would need 206 GB of spectra at the lowest
 // order) and 7 bits of exponent: in the opt-in tcgen05 form's table the source's code (written by
 // k_pack_sources after every forward transform), in a tile's slot list the source's distance from the tile's
-// largest code in steps (k_tile_codes).  SPLIT_NONE: no source.
+// largest code in steps (k_tile_codes).  Screened kernels: the row alone.  SPLIT_NONE: no source.
 constexpr int SPLIT_ROW_BITS = 25;
 constexpr uint32_t SPLIT_ROW_MASK = (1u << SPLIT_ROW_BITS) - 1;
 constexpr uint32_t SPLIT_NONE = 0xffffffffu;
@@ -1440,7 +1454,7 @@ constexpr int HADC_TT = 512;  // padding of its source table
 // row of A holds its 26 source spectra (8 complex = 16 reals each, zeros where a position is empty) and B
 // holds each position's 8x8 complex block as 2x2 real blocks ([re, im] -> [re, im]).  Warp-level m16n8k16
 // FP16 MMAs with FP32 accumulators: A and B are FP16 heads and tails, and each position's
-// At Bh + Ah Bt + Ah Bh (small terms first; the tail-tail product, 2^-22 relative, is dropped) is formed in
+// (At Bh + Ah Bt) / c + Ah Bh (small terms first; the tail-tail product, 2^-22 relative, is dropped) is formed in
 // a fresh MMA accumulator, scaled by the block's exponent and added to FP32 running sums in one fused
 // multiply-add (the MMA's own accumulation is not rounded to nearest).
 //
@@ -1456,10 +1470,10 @@ constexpr int HADC_TT = 512;  // padding of its source table
 // targets at one relative position have 8 different octants, so their 64-byte rows (four 16-byte chunks,
 // swizzled by (slot / 2) % 4) fall on different banks; empty positions read one of 8 zero slots, chosen to
 // stay off the banks of the other rows.
-// A tile whose sources (screened kernels: whose children) lie within 2^-18 of the strongest has one pass: all
-// Laplace tiles of cubes, Plummer spheres and surfaces of up to 4M bodies with charges in (-1, 1), 2 to 9 steps of
-// 2 bits.  Otherwise pass w takes those 10 w .. 10 w + 9 steps below, the others at zero, over the same
-// accumulators: weak sources keep their 22 bits.  The same for the windows of the operator.
+// A tile whose sources lie within 2^-18 of the strongest has one pass: all tiles of cubes, Plummer spheres and
+// surfaces of up to 4M bodies with charges in (-1, 1), 2 to 9 steps of 2 bits.  Otherwise pass w takes the sources
+// 10 w .. 10 w + 9 steps below, the others at zero, over the same accumulators: weak sources keep their bits.  With
+// the screened kernels the passes are the windows of the tile's children, each with every window of the operator.
 // Tiles with at most 256, 128 or 64 targets split the 26 positions over 2, 4 or 8 warps per 64 targets.
 // Bounds per 64 targets and position and SM (cycles): MMAs 24 x 8 / 4 = 48; shared memory 32 (A) + 8 (B).
 // At 1M, p = 8 the tensor pipe is 58% and the shared-memory pipe 70% busy: 16 warps per SM hide the rest of
@@ -1472,7 +1486,7 @@ constexpr int HADH_B = 26 * 2 * 32;              // B fragments (uint4) in share
 constexpr int HADH_FB = HADH_B / 2;              // and as stored
 constexpr size_t HADH_SMEM = (size_t)HADH_SLOTS * 64 + (size_t)HADH_B * 16 + 32 * sizeof(float);
 static_assert(2 * (HADH_SMEM + 1024) <= 228 * 1024, "two CTAs per SM");
-constexpr uint32_t TILE_DEEP = 1u << 31;
+constexpr int SPLIT_PASS = 10;                   // steps of 2 bits that one pass over a tile covers
 struct HadTile {
   int nslots;   // slots used (a multiple of 8, the zero slots included)
   int groups;   // 1, 2, 4 or 8 groups of 64 targets
@@ -1486,8 +1500,9 @@ struct HadSys {
   const HadTile* tiles;
   const uint32_t* slots;  // packed source of each slot (k_tile_codes)
   const float* tinv;      // per tile: undoes its exponent
-  const uint32_t* tpass;  // per tile: bit w: pass w has sources; TILE_DEEP: children with exponents of their own
-  const uint8_t* level;   // of every source's children
+  const uint32_t* tpass;  // per tile: bit w: pass w has sources
+  const SplitHead* head;  // screened kernels: exponents, and the window of every source's children
+  const uint8_t* win;
   const uint2* tab;
   const int* rows;
   int nsrc, ntrg;
@@ -1521,10 +1536,10 @@ __device__ __forceinline__ void tf32_split(float x, uint32_t& h, uint32_t& t) {
 // those of g + 1 (imaginary outputs: (Im, Re)) are the same values swapped (hadh_odd).
 // inv[(v * nfreq + f) * 32 + ipos] undoes the exponent.  One warp per block.
 // v: the operator's window.  The factors of a screened kernel's child pairs differ by e^(-k (distance)): a
-// pair whose largest factor over the frequencies (k_pair_max) is more than 2^-18 below the largest of its
+// pair whose largest factor over the frequencies (k_pair_max) is more than 2^-28 below the largest of its
 // position goes to the next window, with an exponent of its own, as the sources' children do; pwin[ipos * 64 + pair]
-// is the pair's window.  One window for Laplace and for Helmholtz with a real wavenumber; modified Helmholtz takes a
-// second from k (box size) of about 4.6 on.
+// is the pair's window (null: one window, the unscreened kernels).  Modified Helmholtz takes a second from
+// k (box size) of about 7 on.
 __global__ void __launch_bounds__(256)
     k_pair_max(const double2* __restrict__ T, int nfreq, unsigned* __restrict__ pmax) {
   const int pair = threadIdx.x & 63, ipos = blockIdx.y;
@@ -1535,14 +1550,14 @@ __global__ void __launch_bounds__(256)
   }
   atomicMax(pmax + ipos * 64 + pair, __float_as_uint(m));
 }
-__global__ void k_m2l_fragments(const double2* __restrict__ T, int nfreq, const uint8_t* __restrict__ pwin,
+__global__ void k_m2l_fragments(const double2* __restrict__ T, int nfreq, const uint8_t* __restrict__ pwin, double tail,
                                 uint4* __restrict__ frag, float* __restrict__ inv) {
   const int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31, win = blockIdx.y;
   if (w >= 26ll * nfreq) return;
   const int f = (int)(w / 26), ipos = (int)(w % 26);
   const double2* blk = T + ((int64_t)ipos * nfreq + f) * 64;
-  auto entry = [&](int pair) { return pwin[ipos * 64 + pair] == win ? blk[pair] : make_double2(0.0, 0.0); };
+  auto entry = [&](int pair) { return !pwin || pwin[ipos * 64 + pair] == win ? blk[pair] : make_double2(0.0, 0.0); };
   const double2 u = entry(lane), v = entry(32 + lane);
   float m = (float)fmax(fmax(fabs(u.x), fabs(u.y)), fmax(fabs(v.x), fabs(v.y)));
 #pragma unroll
@@ -1558,7 +1573,7 @@ __global__ void k_m2l_fragments(const double2* __restrict__ T, int nfreq, const 
     const __half2 hh = __halves2half2(__double2half(re), __double2half(im));
     const float2 hf = __half22float2(hh);
     hd[c] = h2_bits(hh);
-    tl[c] = h2_bits(__halves2half2(__double2half(re - hf.x), __double2half(im - hf.y)));
+    tl[c] = h2_bits(__halves2half2(__double2half((re - hf.x) * tail), __double2half((im - hf.y) * tail)));
   }
   const int64_t row = (int64_t)win * nfreq + f;
   frag[row * HADH_FB + ipos * 32 + lane] = make_uint4(hd[0], hd[1], tl[0], tl[1]);
@@ -1569,13 +1584,12 @@ __device__ __forceinline__ uint4 hadh_odd(const uint4& e) {
   auto sw = [](uint32_t v) { return __byte_perm(v, v, 0x1032) ^ 0x8000u; };
   return make_uint4(sw(e.x), sw(e.y), sw(e.z), sw(e.w));
 }
-// After a forward transform, per tile (one CTA each): the largest exponent code of its sources, whose exponent is
-// the tile's, the slot list packed with every source's distance d from it (SPLIT_NONE: no source, or one
-// without values), and the passes that the tile needs.
+// After a forward transform of an unscreened kernel, per tile (one CTA each): the largest exponent code of its
+// sources, whose exponent is the tile's, the slot list packed with every source's distance d from it (SPLIT_NONE:
+// no source, or one without values), and the passes that the tile needs.
 __global__ void __launch_bounds__(256)
     k_tile_codes(const HadTile* __restrict__ tiles, const int* __restrict__ slots, const int* __restrict__ scode,
-                 const uint8_t* __restrict__ level, uint32_t* __restrict__ pslots, float* __restrict__ tinv,
-                 uint32_t* __restrict__ tpass) {
+                 uint32_t* __restrict__ pslots, float* __restrict__ tinv, uint32_t* __restrict__ tpass) {
   __shared__ int smax;
   __shared__ uint32_t spass;
   const HadTile T = tiles[blockIdx.x];
@@ -1589,9 +1603,9 @@ __global__ void __launch_bounds__(256)
   for (int i = 0; i < (HADH_SLOTS + 255) / 256; i++) {
     const int q = threadIdx.x + 256 * i;
     src[i] = q < T.nslots ? slots[T.slot0 + q] : -1;
-    code[i] = src[i] >= 0 ? scode[src[i]] : 0;
+    code[i] = src[i] >= 0 ? scode[src[i]] : SPLIT_ZERO;
     if (code[i] & SPLIT_ZERO) src[i] = -1;
-    if (src[i] >= 0) kmax = max(kmax, code[i] & 0x7f);
+    else kmax = max(kmax, code[i]);
   }
   atomicMax(&smax, __reduce_max_sync(0xffffffffu, kmax));
   __syncthreads();
@@ -1599,20 +1613,10 @@ __global__ void __launch_bounds__(256)
   uint32_t pass = 0u;
 #pragma unroll
   for (int i = 0; i < (HADH_SLOTS + 255) / 256; i++) {
-    const int q = threadIdx.x + 256 * i, d = kmax - (code[i] & 0x7f);
+    const int q = threadIdx.x + 256 * i, d = kmax - code[i];
     if (q < T.nslots)
       pslots[T.slot0 + q] = src[i] >= 0 ? (uint32_t)src[i] | (uint32_t)d << SPLIT_ROW_BITS : SPLIT_NONE;
-    if (src[i] < 0) continue;
-    if (code[i] & SPLIT_DEEP) {
-#pragma unroll
-      for (int c = 0; c < 8; c++) {
-        const int l = level[(int64_t)src[i] * 8 + c];
-        pass |= 1u << ((d + l) / SPLIT_PASS);
-        if (l >= SPLIT_WIN) pass |= TILE_DEEP;
-      }
-    } else {
-      pass |= 1u << (d / SPLIT_PASS);
-    }
+    if (src[i] >= 0) pass |= 1u << (d / SPLIT_PASS);
   }
   pass = __reduce_or_sync(0xffffffffu, pass);
   if ((threadIdx.x & 31) == 0) atomicOr(&spass, pass);
@@ -1634,6 +1638,7 @@ __host__ __device__ __forceinline__ uint32_t hadh_entry(int slot) { return (uint
 
 // one tile at frequency f; with `fill` it also brings the frequency's B fragments and block scales (frag, binv: those
 // of f; bstride frequencies between the operator's nbw windows) into shared memory
+template <bool SCREENED>
 __device__ __forceinline__ void hadh_tile(const HadSys& S, int tile, int f, unsigned char* sA, uint4* sB, float* sInv,
                                           const uint4* __restrict__ frag, const float* __restrict__ binv, int nbw,
                                           int bstride, bool fill, int tid) {
@@ -1671,33 +1676,55 @@ __device__ __forceinline__ void hadh_tile(const HadSys& S, int tile, int f, unsi
     const __half2 m = __float2half2_rn(__uint_as_float((uint32_t)(127 - 2 * d) << 23));
     return h2_bits(__hmul2(*reinterpret_cast<__half2*>(&v), m));
   };
-  auto moved = [](uint32_t v, int s) {  // times 2^(2 s), |s| <= 9
-    const uint32_t m = (uint32_t)(15 + s) << 10;
-    const __half2 f = __halves2half2(__ushort_as_half((unsigned short)m), __ushort_as_half((unsigned short)m));
-    return h2_bits(__hmul2(__hmul2(*reinterpret_cast<__half2*>(&v), f), f));
-  };
-  // the children of pass w alone, at the exponent 20 w above the tile's
+  // pass w alone: the sources 10 w .. 10 w + 9 steps below the tile's exponent, at the exponent 20 w above it
+  // (stored 2 d above); screened: the children of window w, as they are stored
   auto load_pass = [&](int w) {
     for (int q = tid >> 2; q < T.nslots; q += QS) {
       const uint32_t e = slots[q];
       uint4 v = make_uint4(0u, 0u, 0u, 0u);
       if (e != SPLIT_NONE) {
-        const int64_t row = e & SPLIT_ROW_MASK;
-        const uchar2 l = reinterpret_cast<const uchar2*>(S.level)[row * 4 + c];
-        const int d = (int)(e >> SPLIT_ROW_BITS);
-        const uint4 u = __ldg(inf + row * 4 + c);
-        // stored 2 d + 18 (level / 9) above the tile's exponent
-        const int s0 = SPLIT_PASS * w - d - l.x / SPLIT_WIN * SPLIT_WIN, s1 = SPLIT_PASS * w - d - l.y / SPLIT_WIN * SPLIT_WIN;
-        if ((d + l.x) / SPLIT_PASS == w) v.x = moved(u.x, s0), v.y = moved(u.y, s0);
-        if ((d + l.y) / SPLIT_PASS == w) v.z = moved(u.z, s1), v.w = moved(u.w, s1);
+        if constexpr (SCREENED) {
+          const uchar2 cw = reinterpret_cast<const uchar2*>(S.win)[(int64_t)e * 4 + c];
+          v = __ldg(inf + (int64_t)e * 4 + c);
+          if (cw.x != w) v.x = v.y = 0u;
+          if (cw.y != w) v.z = v.w = 0u;
+        } else {
+          const int d = (int)(e >> SPLIT_ROW_BITS) - SPLIT_PASS * w;
+          if (d >= 0 && d < SPLIT_PASS) {
+            v = __ldg(inf + (int64_t)(e & SPLIT_ROW_MASK) * 4 + c);
+            v = make_uint4(scaled(v.x, d), scaled(v.y, d), scaled(v.z, d), scaled(v.w, d));
+          }
+        }
       }
       store_a(q, v);
     }
   };
   uint4 fb[NF];
   if (fill) load_b(frag, fb);
-  uint32_t todo = S.tpass[tile];  // the passes left, the open one included
-  if (todo == 1u) {
+  uint32_t todo;  // the passes left, the open one included
+  int x0 = 0, xt = 0;
+  if constexpr (SCREENED) {
+    x0 = S.head->e0;
+    todo = S.head->mask;
+    if (todo != 1u) {  // the windows of the tile's own sources
+      __shared__ uint32_t stodo;
+      if (tid == 0) stodo = 0u;
+      __syncthreads();
+      uint32_t m = 0u;
+      for (int q = tid; q < T.nslots; q += HADH_NT) {
+        const uint32_t e = slots[q];
+        for (int k = 0; e != SPLIT_NONE && k < 8; k++) m |= 1u << S.win[(int64_t)e * 8 + k];
+      }
+      m = __reduce_or_sync(0xffffffffu, m);
+      if (lane == 0) atomicOr(&stodo, m);
+      __syncthreads();
+      todo = stodo ? stodo : 1u;
+    }
+    xt = split_exp(x0, __ffs(todo) - 1);  // the sums are formed at the tile's strongest window's exponent
+  } else {
+    todo = S.tpass[tile];
+  }
+  if (SCREENED ? S.head->mask == 1u : todo == 1u) {
     uint32_t src[NB];
 #pragma unroll
     for (int i = 0; i < NB; i++) {
@@ -1708,19 +1735,21 @@ __device__ __forceinline__ void hadh_tile(const HadSys& S, int tile, int f, unsi
 #pragma unroll
     for (int i = 0; i < NB; i++) {
       const uint32_t e = src[i];
-      v[i] = e != SPLIT_NONE ? __ldg(inf + (int64_t)(e & SPLIT_ROW_MASK) * 4 + c) : make_uint4(0u, 0u, 0u, 0u);
+      const int64_t row = SCREENED ? e : e & SPLIT_ROW_MASK;
+      v[i] = e != SPLIT_NONE ? __ldg(inf + row * 4 + c) : make_uint4(0u, 0u, 0u, 0u);
     }
 #pragma unroll
     for (int i = 0; i < NB; i++) {
       const int q = (tid >> 2) + QS * i;
       if (q >= T.nslots) break;
-      const int d = src[i] != SPLIT_NONE ? (int)(src[i] >> SPLIT_ROW_BITS) : 0;
       uint4 w = v[i];
-      if (d > 0) w = make_uint4(scaled(w.x, d), scaled(w.y, d), scaled(w.z, d), scaled(w.w, d));
+      if constexpr (!SCREENED) {
+        const int d = src[i] != SPLIT_NONE ? (int)(src[i] >> SPLIT_ROW_BITS) : 0;
+        if (d > 0) w = make_uint4(scaled(w.x, d), scaled(w.y, d), scaled(w.z, d), scaled(w.w, d));
+      }
       store_a(q, w);
     }
   } else {
-    todo &= ~TILE_DEEP;
     load_pass(__ffs(todo) - 1);
   }
   if (fill) store_b(fb, binv);
@@ -1772,7 +1801,12 @@ __device__ __forceinline__ void hadh_tile(const HadSys& S, int tile, int f, unsi
 #pragma unroll
       for (int jj = 0; jj < 2; jj++)
 #pragma unroll
-        for (int h = 0; h < 2; h++) mma_f16(d[jj][h], xh[jj][0], xh[jj][1], xh[jj][2], xh[jj][3], b[h].x, b[h].y);
+        for (int h = 0; h < 2; h++) {
+          if constexpr (SCREENED)
+#pragma unroll
+            for (int i = 0; i < 4; i++) d[jj][h][i] *= 1.f / SPLIT_TAIL;
+          mma_f16(d[jj][h], xh[jj][0], xh[jj][1], xh[jj][2], xh[jj][3], b[h].x, b[h].y);
+        }
 #pragma unroll
       for (int jj = 0; jj < 2; jj++)
 #pragma unroll
@@ -1795,7 +1829,7 @@ __device__ __forceinline__ void hadh_tile(const HadSys& S, int tile, int f, unsi
   if (bw == 0) {
     const int w = __ffs(todo) - 1;
     load_pass(w);
-    pscale = pow2f(-2 * SPLIT_PASS * w);
+    pscale = pow2f(SCREENED ? xt - split_exp(x0, w) : -2 * SPLIT_PASS * w);
   }
   __syncthreads();
   }
@@ -1827,7 +1861,7 @@ __device__ __forceinline__ void hadh_tile(const HadSys& S, int tile, int f, unsi
     }
   }
   // D fragment: row g (and g + 8), columns 2t, 2t + 1 of half h = target component 4 h + t (re, im)
-  const float inv = S.tinv[tile];
+  const float inv = SCREENED ? pow2f(-xt) : S.tinv[tile];
   float2* of = S.out + (int64_t)f * S.ntrg * 8;
   const int* rows = S.rows + T.row0 + gr * 64 + g;
 #pragma unroll
@@ -1843,6 +1877,7 @@ __device__ __forceinline__ void hadh_tile(const HadSys& S, int tile, int f, unsi
 }
 
 // tiles [blockIdx.x * tpc, ...) at frequency blockIdx.y share one copy of the frequency's B fragments
+template <bool SCREENED>
 __global__ void __launch_bounds__(HADH_NT, 2)
     k_hadamard_h(const uint4* __restrict__ frag, const float* __restrict__ binv, int nbw, HadSys S, int ntiles, int tpc) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1851,16 +1886,16 @@ __global__ void __launch_bounds__(HADH_NT, 2)
   const int f = blockIdx.y, tid = threadIdx.x;
   const int te = min(ntiles, ((int)blockIdx.x + 1) * tpc);
   for (int k = blockIdx.x * tpc; k < te; k++) {
-    hadh_tile(S, k, f, smem_raw, sB, sInv, frag + (int64_t)f * HADH_FB, binv + f * 32, nbw, gridDim.y,
-              nbw > 1 || k == (int)blockIdx.x * tpc, tid);
+    hadh_tile<SCREENED>(S, k, f, smem_raw, sB, sInv, frag + (int64_t)f * HADH_FB, binv + f * 32, nbw, gridDim.y,
+                        nbw > 1 || k == (int)blockIdx.x * tpc, tid);
     if (k + 1 < te) __syncthreads();
   }
 }
 // the same over the tiles of many systems that share one operator table (a batch of Laplace systems):
 // tiles[k] = (system, its tile)
 __global__ void __launch_bounds__(HADH_NT, 2)
-    k_hadamard_h_batch(const uint4* __restrict__ frag, const float* __restrict__ binv, int nbw,
-                       const HadSys* __restrict__ sys, const int2* __restrict__ tiles, int ntiles, int tpc) {
+    k_hadamard_h_batch(const uint4* __restrict__ frag, const float* __restrict__ binv, const HadSys* __restrict__ sys,
+                       const int2* __restrict__ tiles, int ntiles, int tpc) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   uint4* sB = reinterpret_cast<uint4*>(smem_raw + (size_t)HADH_SLOTS * 64);
   float* sInv = reinterpret_cast<float*>(sB + HADH_B);
@@ -1868,8 +1903,8 @@ __global__ void __launch_bounds__(HADH_NT, 2)
   const int te = min(ntiles, ((int)blockIdx.x + 1) * tpc);
   for (int k = blockIdx.x * tpc; k < te; k++) {
     const int2 tl = tiles[k];
-    hadh_tile(sys[tl.x], tl.y, f, smem_raw, sB, sInv, frag + (int64_t)f * HADH_FB, binv + f * 32, nbw, gridDim.y,
-              nbw > 1 || k == (int)blockIdx.x * tpc, tid);
+    hadh_tile<false>(sys[tl.x], tl.y, f, smem_raw, sB, sInv, frag + (int64_t)f * HADH_FB, binv + f * 32, 1, gridDim.y,
+                     k == (int)blockIdx.x * tpc, tid);
     if (k + 1 < te) __syncthreads();
   }
 }
@@ -1922,8 +1957,8 @@ __host__ __device__ __forceinline__ uint32_t hadc_boff(int n, int c) {
 // btab[f] (HADC_BBYTES per frequency): factor m(sc, tc) of position ipos (head + tail of the stored
 // fragments) -> the real 2 x 2 block (outputs 2 tc, 2 tc + 1; inputs 2 sc, 2 sc + 1) =
 // [[Re m, -Im m], [Im m, Re m]], TF32 head then tail
-__global__ void k_hadc_btab(const uint4* __restrict__ frag, const float* __restrict__ binv, int nbw, int nfreq,
-                            unsigned char* __restrict__ btab) {
+__global__ void k_hadc_btab(const uint4* __restrict__ frag, const float* __restrict__ binv, int nbw, float itail,
+                            int nfreq, unsigned char* __restrict__ btab) {
   const int64_t total = (int64_t)nfreq * 26 * 64;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     const int f = (int)(e / (26 * 64)), ipos = (int)(e / 64 % 26), sc = (int)(e >> 3 & 7), tc = (int)(e & 7);
@@ -1933,8 +1968,8 @@ __global__ void k_hadc_btab(const uint4* __restrict__ frag, const float* __restr
       const uint4 q = frag[row * HADH_FB + (ipos * 2 + (tc >> 2)) * 16 + 4 * (tc & 3) + (sc & 3)];
       const float2 hd = h2_float2(sc < 4 ? q.x : q.y), tl = h2_float2(sc < 4 ? q.z : q.w);
       const float bi = binv[row * 32 + ipos];
-      m.x += (hd.x + tl.x) * bi;
-      m.y -= (hd.y + tl.y) * bi;
+      m.x += fmaf(tl.x, itail, hd.x) * bi;
+      m.y -= fmaf(tl.y, itail, hd.y) * bi;
     }
     const float v[4] = {m.x, -m.y, m.y, m.x};
     unsigned char* blk = btab + (int64_t)f * HADC_BBYTES + ipos * 2048;
@@ -1953,10 +1988,11 @@ __device__ __forceinline__ bool hadc_wait(uint32_t mbar, uint32_t parity) {
   return __all_sync(0xffffffffu, tc5::mbar_wait(mbar, parity, HADC_WAIT));
 }
 
+template <bool SCREENED>
 __global__ void __launch_bounds__(HADC_NT, 2)
     k_hadamard_dc(const unsigned char* __restrict__ btab, const SplitC* __restrict__ in, float2* __restrict__ out,
-                  const uint8_t* __restrict__ level, const uint32_t* __restrict__ tab, int ld,
-                  const int* __restrict__ rows, int nsrc, int ntrg, int nfreq, int* __restrict__ status) {
+                  const SplitHead* __restrict__ head, const uint8_t* __restrict__ win, const uint32_t* __restrict__ tab,
+                  int ld, const int* __restrict__ rows, int nsrc, int ntrg, int nfreq, int* __restrict__ status) {
   using namespace tc5;
   extern __shared__ __align__(16) unsigned char smem_raw[];  // B blocks of the current frequency, gather ring
   __shared__ __align__(8) uint64_t mbar[2 * HADC_S + 2];       // full[S], done[S], B half 0, B half 1
@@ -2042,6 +2078,8 @@ __global__ void __launch_bounds__(HADC_NT, 2)
     const int k = blockIdx.x * 128 + tid;  // this lane's target slot = TMEM lane tid
     const uint32_t tw = tm + ((uint32_t)(wid * 32) << 16);
     const int row = rows[k];
+    const int x0 = SCREENED ? head->e0 : 0;
+    auto row_of = [](uint32_t e) { return (int64_t)(SCREENED ? e : e & SPLIT_ROW_MASK); };
     float acc[16];
 #pragma unroll
     for (int i = 0; i < 16; i++) acc[i] = 0.f;
@@ -2075,7 +2113,7 @@ __global__ void __launch_bounds__(HADC_NT, 2)
       for (int i = 0; i < 4; i++) {
         const uint32_t e = __shfl_sync(0xffffffffu, ent, g + 8 * i);
         cp_async16(slot + i * 32 * 16,
-                   e != SPLIT_NONE ? (const void*)(inf + (int64_t)(e & SPLIT_ROW_MASK) * 4 + q) : (const void*)in,
+                   e != SPLIT_NONE ? (const void*)(inf + row_of(e) * 4 + q) : (const void*)in,
                    e != SPLIT_NONE ? 16u : 0u);
       }
       cp_async_commit();
@@ -2102,12 +2140,18 @@ __global__ void __launch_bounds__(HADC_NT, 2)
         for (int i = 0; i < 4; i++) {  // head + tail, exponents undone: children 2 q and 2 q + 1
           const uint4 v = sl[i * 32];
           const uint32_t e = __shfl_sync(0xffffffffu, entg, g + 8 * i);
-          uchar2 l = make_uchar2(0, 0);
-          if (e != SPLIT_NONE) l = reinterpret_cast<const uchar2*>(level)[(int64_t)(e & SPLIT_ROW_MASK) * 4 + q];
-          const float s0 = split_inv(e) * pow2f(-2 * SPLIT_WIN * (l.x / SPLIT_WIN));
-          const float s1 = split_inv(e) * pow2f(-2 * SPLIT_WIN * (l.y / SPLIT_WIN));
           const float2 h0 = h2_float2(v.x), t0 = h2_float2(v.y), h1 = h2_float2(v.z), t1 = h2_float2(v.w);
-          x[i] = make_float4((h0.x + t0.x) * s0, (h0.y + t0.y) * s0, (h1.x + t1.x) * s1, (h1.y + t1.y) * s1);
+          if constexpr (SCREENED) {
+            uchar2 cw = make_uchar2(0, 0);
+            if (e != SPLIT_NONE) cw = reinterpret_cast<const uchar2*>(win)[row_of(e) * 4 + q];
+            const float s0 = pow2f(-split_exp(x0, cw.x)), s1 = pow2f(-split_exp(x0, cw.y));
+            constexpr float it = 1.f / SPLIT_TAIL;
+            x[i] = make_float4(fmaf(t0.x, it, h0.x) * s0, fmaf(t0.y, it, h0.y) * s0, fmaf(t1.x, it, h1.x) * s1,
+                               fmaf(t1.y, it, h1.y) * s1);
+          } else {
+            const float sc = split_inv(e);
+            x[i] = make_float4((h0.x + t0.x) * sc, (h0.y + t0.y) * sc, (h1.x + t1.x) * sc, (h1.y + t1.y) * sc);
+          }
         }
       }
       if (gi >= HADC_S) {  // the stage's previous position is done: take its products, then reuse it
@@ -2200,26 +2244,68 @@ size_t ft_bwd_smem(int p) { return ft_fwd_smem<R>(p); }
 template <class R> struct Spec;
 template <> struct Spec<float> {
   using type = SplitC;
-  static __device__ __forceinline__ type make(float2 v, float scale) { return split16(v.x * scale, v.y * scale); }
+  static __device__ __forceinline__ type make(float2 v, float scale, float c) {
+    return split16(v.x * scale, v.y * scale, c);
+  }
 };
 template <> struct Spec<double> {
   using type = double2;
-  static __device__ __forceinline__ type make(double2 v, float) { return v; }
+  static __device__ __forceinline__ type make(double2 v, float, float) { return v; }
 };
 __device__ __forceinline__ float abs1(float v) { return fabsf(v); }
 __device__ __forceinline__ float abs1(float2 v) { return fabsf(v.x) + fabsf(v.y); }
-// The scales of source node s (children at node0 .. node0 + 7).  One warp per child; red: 8 floats of shared memory;
-// csc: the children's scales, ready after the caller's next barrier.  Called by a whole CTA of 256 threads;
-// writes the source's exponent code and its children's levels (all 0 unless the kernel is screened).
-struct SplitOut {
-  int* code;
-  uint8_t* level;
-  int screened;
-};
+// Screened kernels: the bound of every source's children (at child0[src[s]] + 0 .. 7).  Warp per child; the block
+// that finishes last sets the group's e0 from the largest.  A pass of its own over the sources' densities, since
+// the exponents of all sources stand on it (Yukawa sphere 300k: 0.02 ms).
 template <class W>
-__device__ __forceinline__ void source_scales(const W* __restrict__ up, int64_t node0, int nsurf, float* red, float* csc,
-                                              const SplitOut& so, int64_t s) {
+__global__ void __launch_bounds__(256)
+    k_source_bounds(const int* __restrict__ src, int ns, const int* __restrict__ child0, const W* __restrict__ up,
+                    int nsurf, float* __restrict__ bound, SplitHead* head) {
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float b = 0.f;
+  for (int64_t e = blockIdx.x * 8ll + wid; e < 8ll * ns; e += gridDim.x * 8ll) {
+    const W* u = up + ((int64_t)child0[src[e >> 3]] + (e & 7)) * nsurf;
+    float m = 0.f;
+    for (int k = lane; k < nsurf; k += 32) m += abs1(__ldg(u + k));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m += __shfl_xor_sync(0xffffffffu, m, o);
+    if (lane == 0) bound[e] = m;
+    b = fmaxf(b, m);
+  }
+  __shared__ float red[8];
+  if (lane == 0) red[wid] = b;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int k = 1; k < 8; k++) b = fmaxf(b, red[k]);
+    atomicMax(&head->gmax, __float_as_uint(b));
+    __threadfence();
+    if (atomicAdd(&head->done, 1u) == gridDim.x - 1) {
+      head->e0 = split_exp0(__uint_as_float(atomicExch(&head->gmax, 0u)));
+      head->mask = 1u;
+      head->done = 0u;
+    }
+  }
+}
+// the window of child r (8 source + child), recorded on request, and its scale
+__device__ __forceinline__ float child_scale(const SplitOut& so, int64_t r, bool record) {
+  const int e0 = so.head->e0, w = split_window(so.bound[r], e0);
+  if (record) {
+    so.win[r] = (uint8_t)w;
+    if (w > 0) atomicOr(&so.head->mask, 1u << w);
+  }
+  return pow2f(split_exp(e0, w));
+}
+// The scale of every child of source node s (children at node0 .. node0 + 7) to csc, ready after the caller's
+// next barrier; returns the tails' c.  red: 8 floats of shared memory.  Called by a whole CTA of 256 threads.  Not
+// screened: one scale from the bound of the strongest child (one warp per child), and the node's code.
+template <class W>
+__device__ __forceinline__ float source_scales(const W* __restrict__ up, int64_t node0, int nsurf, float* red, float* csc,
+                                               const SplitOut& so, int64_t s) {
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (so.head) {
+    if (threadIdx.x < 8) csc[lane] = child_scale(so, 8 * s + lane, true);
+    return SPLIT_TAIL;
+  }
   const W* u = up + (node0 + wid) * nsurf;
   float m = 0.f;
   for (int k = lane; k < nsurf; k += 32) m += abs1(__ldg(u + k));
@@ -2231,12 +2317,11 @@ __device__ __forceinline__ void source_scales(const W* __restrict__ up, int64_t 
     float b = red[0];
 #pragma unroll
     for (int c = 1; c < 8; c++) b = fmaxf(b, red[c]);
-    const int code = split_code(b), l = so.screened ? split_level(red[lane], b, code) : 0;
-    csc[lane] = split_scale(code, l);
-    so.level[8 * s + lane] = (uint8_t)l;
-    const bool deep = __any_sync(0xffu, l > 0);
-    if (lane == 0) so.code[s] = code | (deep ? SPLIT_DEEP : 0) | (b == 0.f ? SPLIT_ZERO : 0);
+    const int code = split_code(b);
+    csc[lane] = split_scale(code);
+    if (lane == 0) so.code[s] = code | (b == 0.f ? SPLIT_ZERO : 0);
   }
+  return 1.f;
 }
 // DFT factors as compile-time constants: where the loops unroll, an index (j k mod N) is known to the compiler and the
 // factor becomes an operand of the multiply-add instead of a shared-memory load or a register.  cos and
@@ -2292,7 +2377,7 @@ __device__ __forceinline__ void wfma(CT& acc, const CT& a, const CT& w) {
   }
 }
 
-// The cuFFT path (orders beyond the DFT kernels): each source's exponent code and levels ...
+// The cuFFT path (orders beyond the DFT kernels): each source's exponent code or windows ...
 template <class W>
 __global__ void __launch_bounds__(256)
     k_source_codes(const int* __restrict__ src, const int* __restrict__ child0, const W* __restrict__ up, int nsurf,
@@ -2313,9 +2398,9 @@ __global__ void k_transpose_split(const float2* __restrict__ in, SplitC* __restr
   for (int i = threadIdx.y; i < 32; i += 8) {
     const int64_t c = c0 + i, r = r0 + threadIdx.x;
     if (r >= nr || c >= nfreq) continue;
-    const float sc = split_scale(so.code[r >> 3] & 0x7f, so.level[r]);
+    const float sc = so.head ? child_scale(so, r, false) : split_scale(so.code[r >> 3] & 0x7f);
     const float2 v = tile[threadIdx.x][i];
-    out[c * nr + r] = split16(v.x * sc, v.y * sc);
+    out[c * nr + r] = split16(v.x * sc, v.y * sc, so.head ? SPLIT_TAIL : 1.f);
   }
 }
 
@@ -2509,9 +2594,10 @@ __global__ void __launch_bounds__(FT_NT, FtcFwdMinB<R>::v)
   }
   const int64_t node0 = (int64_t)child0[src[s]] + ch0;
   __shared__ float csc[8];  // the children's power-of-two scales (mixed)
+  float tail = 1.f;
   if constexpr (sizeof(R) == 4) {
     __shared__ float red[8];
-    source_scales(up, node0, nsurf, red, csc, so, s);
+    tail = source_scales(up, node0, nsurf, red, csc, so, s);
   }
   const int64_t fstride = (int64_t)N * N * ns * 8;
   for (int j0 = 0; j0 < P; j0 += FTC_JS) {
@@ -2558,7 +2644,7 @@ __global__ void __launch_bounds__(FT_NT, FtcFwdMinB<R>::v)
 #pragma unroll
       for (int c = 0; c < P; c++) x[c] = sB[((c * N + kb) * CPB + ch) * KS + sl];
       auto* o = spec + ((int64_t)(kb * N + ka) * ns + s) * 8 + ch0 + ch;
-      ftc_dft_p<P>(x, ConstW<CT, N, -1>(), [&](int kc, CT v) { o[kc * fstride] = Spec<R>::make(v, csc[ch]); });
+      ftc_dft_p<P>(x, ConstW<CT, N, -1>(), [&](int kc, CT v) { o[kc * fstride] = Spec<R>::make(v, csc[ch], tail); });
     }
   }
 }
@@ -2708,9 +2794,10 @@ __global__ void __launch_bounds__(FT_NT, FtrMinB<R>::v)
   }
   const int64_t node0 = (int64_t)child0[src[s]] + ch0;
   __shared__ float csc[8];  // the children's power-of-two scales (mixed)
+  float tail = 1.f;
   if constexpr (sizeof(R) == 4) {
     __shared__ float red[8];
-    source_scales(up, node0, nsurf, red, csc, so, s);
+    tail = source_scales(up, node0, nsurf, red, csc, so, s);
   }
   const int64_t fstride = (int64_t)N * H * ns * 8;  // kc -> kc + 1
   for (int k0 = 0; k0 < H; k0 += KS) {
@@ -2759,7 +2846,7 @@ __global__ void __launch_bounds__(FT_NT, FtrMinB<R>::v)
 #pragma unroll
       for (int c = 0; c < P; c++) x[c] = sB[((c * N + kb) * CPB + ch) * KS + sl];
       auto* o = spec + ((int64_t)(kb * H + ka) * ns + s) * 8 + ch0 + ch;
-      ftc_dft_p<P>(x, ConstW<CT, N, -1>(), [&](int kc, CT v) { o[kc * fstride] = Spec<R>::make(v, csc[ch]); });
+      ftc_dft_p<P>(x, ConstW<CT, N, -1>(), [&](int kc, CT v) { o[kc * fstride] = Spec<R>::make(v, csc[ch], tail); });
     }
   }
 }
@@ -2919,11 +3006,13 @@ struct Workspace {
   std::vector<cufftHandle> fwd, bwd;
   std::vector<int> had_tile0;  // first tile of each group (ngroups + 1; k_hadamard_h)
   // mixed path: tiles of k_hadamard_h (per group [had_tile0[g], had_tile0[g + 1])), their source slots,
-  // tables and output rows; scode, slevel: every source's exponent code and its children's levels of the last
-  // forward transform (one group at a time)
+  // tables and output rows; every source's exponent code (screened kernels: its children's bounds and windows)
+  // of the last forward transform (one group at a time)
   DBuf<HadTile> hadh_tile;
   DBuf<int> hadh_slots, hadh_rows, scode;
-  DBuf<uint8_t> slevel;
+  DBuf<float> sbound;
+  DBuf<uint8_t> swin;
+  DBuf<SplitHead> shead;
   DBuf<uint32_t> hadh_pslots, hadh_tpass;  // k_tile_codes
   DBuf<float> hadh_tinv;
   DBuf<uint2> hadh_tab;
@@ -3093,7 +3182,12 @@ Workspace& workspace(Fmm& f, Tree& t, cudaStream_t s) {
   if (f.mixed()) {
     XREQUIRE(maxn < (int)SPLIT_ROW_MASK, XFMM_ERR_UNSUPPORTED, "too many M2L sources");
     W.scode.alloc(maxn);
-    W.slevel.alloc((size_t)maxn * 8);
+    if (f.kernel != XFMM_LAPLACE) {
+      W.sbound.alloc((size_t)maxn * 8);
+      W.swin.alloc((size_t)maxn * 8);
+      W.shead.alloc(1);
+      XCUDA(cudaMemsetAsync(W.shead.p, 0, W.shead.bytes(), s));
+    }
   }
   int dims[3] = {f.n1, f.n1, f.n1};
   cufftType tf = cplx ? (f.mixed() ? CUFFT_C2C : CUFFT_Z2Z) : (f.mixed() ? CUFFT_R2C : CUFFT_D2Z);
@@ -3405,9 +3499,18 @@ struct Engine {
       const int tab_level = KER == K_LAPLACE ? 0 : g + 1;
       using SP = typename Spec<R>::type;
       SP* spec = (SP*)ws.specB.p;
-      const SplitOut so{ws.scode.p, ws.slevel.p, KER == K_YUKAWA || (KER == K_HELMHOLTZ && f.k_im != 0)};
+      const bool screened = KER != K_LAPLACE && f.screened();
+      const SplitOut so{ws.scode.p, ws.sbound.p, ws.swin.p, screened ? ws.shead.p : nullptr};
       if (phase & M2L_FWD) {
         XCUDA(cudaEventRecord(ev[0], s));
+        if constexpr (sizeof(R) == 4) {
+          if (screened) {
+            k_source_bounds<W><<<std::min(ns, 148 * 8), 256, 0, s>>>(src, ns, t.child0.p, (const W*)ws.up.p, n,
+                                                                   ws.sbound.p, ws.shead.p);
+            XLAUNCH();
+            ws.launches++;
+          }
+        }
         // upward equivalent DFT (fmm_scale_invariant.h:560-604) -> specB [f][s][c]
         if constexpr (KER != K_HELMHOLTZ) {
           if (ws.fused) {
@@ -3458,14 +3561,14 @@ struct Engine {
             transpose<CT>((const CT*)ws.specA.p, (CT*)ws.specB.p, (int64_t)ns * 8, nfreq, s);  // -> [f][s][c]
           }
         }
-        if (const int nht = ws.had_tile0[g + 1] - ws.had_tile0[g]; sizeof(R) == 4 && nht > 0) {
+        if (const int nht = ws.had_tile0[g + 1] - ws.had_tile0[g]; sizeof(R) == 4 && nht > 0 && !screened) {
           k_tile_codes<<<nht, 256, 0, s>>>(ws.hadh_tile.p + ws.had_tile0[g], ws.hadh_slots.p, ws.scode.p,
-                                           ws.slevel.p, ws.hadh_pslots.p, ws.hadh_tinv.p + ws.had_tile0[g],
+                                           ws.hadh_pslots.p, ws.hadh_tinv.p + ws.had_tile0[g],
                                            ws.hadh_tpass.p + ws.had_tile0[g]);
           XLAUNCH();
           ws.launches++;
         }
-        if (sizeof(R) == 4 && ws.hadd_ld[g] > 0) {  // the tcgen05 form's table
+        if (sizeof(R) == 4 && ws.hadd_ld[g] > 0 && !screened) {  // the tcgen05 form's table
           const int64_t nd = (int64_t)26 * ws.hadd_ld[g];
           k_pack_sources<<<std::min<int64_t>(nblk(nd), 148 * 8), 256, 0, s>>>(
               ws.hadd_tab.p + ws.hadd_tab0[g], nd, ws.scode.p, ws.hadd_tabp.p + ws.hadd_tab0[g]);
@@ -3481,33 +3584,39 @@ struct Engine {
           XREQUIRE(nfreq < 65536, XFMM_ERR_UNSUPPORTED, "too many frequencies for the Hadamard grid");
           if (ntiles > 0 && (phase & M2L_HAD_TILES)) {
             if (!ws.hadh_attr) {
-              XCUDA(cudaFuncSetAttribute(k_hadamard_h, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HADH_SMEM));
+              for (auto kern : {k_hadamard_h<false>, k_hadamard_h<true>})
+                XCUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HADH_SMEM));
               ws.hadh_attr = true;
             }
             const int tpc = t.hadr_tpc > 0 ? t.hadr_tpc : HADH_TPC;
-            const HadSys S = had_sys(ws, g, ns, nt);
+            const HadSys S = had_sys(ws, g, ns, nt, screened);
             const LevelOps& op = f.ops[tab_level];
-            k_hadamard_h<<<dim3((ntiles + tpc - 1) / tpc, nfreq), HADH_NT, HADH_SMEM, s>>>(
+            const auto kern = screened ? k_hadamard_h<true> : k_hadamard_h<false>;
+            kern<<<dim3((ntiles + tpc - 1) / tpc, nfreq), HADH_NT, HADH_SMEM, s>>>(
                 (const uint4*)op.m2l_frag.p, op.m2l_binv.p, op.m2l_windows, S, ntiles, tpc);
             XLAUNCH();
             ws.launches++;
           }
           if (ws.hadd_ld[g] > 0 && (phase & M2L_HAD_DENSE)) {
             if (!ws.hadc_attr) {
-              XCUDA(cudaFuncSetAttribute(k_hadamard_dc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HADC_SMEM));
+              for (auto kern : {k_hadamard_dc<false>, k_hadamard_dc<true>})
+                XCUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HADC_SMEM));
               ws.hadc_attr = true;
             }
             const LevelOps& op = f.ops[tab_level];
             if (ws.hadc_btab_id != op.m2l_id) {  // B blocks in the MMA layout
               ws.hadc_btab.reserve((size_t)nfreq * HADC_BBYTES);
               k_hadc_btab<<<std::min<int64_t>(nblk((int64_t)nfreq * 26 * 64), 148 * 16), 256, 0, s>>>(
-                  (const uint4*)op.m2l_frag.p, op.m2l_binv.p, op.m2l_windows, nfreq, ws.hadc_btab.p);
+                  (const uint4*)op.m2l_frag.p, op.m2l_binv.p, op.m2l_windows, screened ? 1.f / SPLIT_TAIL : 1.f, nfreq,
+                  ws.hadc_btab.p);
               XLAUNCH();
               ws.launches++;
               ws.hadc_btab_id = op.m2l_id;
             }
-            k_hadamard_dc<<<dim3(ws.hadd_ld[g] / 128, (nfreq + HADC_FPB - 1) / HADC_FPB), HADC_NT, HADC_SMEM, s>>>(
-                ws.hadc_btab.p, spec, (CT*)ws.specA.p, ws.slevel.p, ws.hadd_tabp.p + ws.hadd_tab0[g], ws.hadd_ld[g],
+            const auto kern = screened ? k_hadamard_dc<true> : k_hadamard_dc<false>;
+            const uint32_t* tab = screened ? (const uint32_t*)ws.hadd_tab.p : ws.hadd_tabp.p;  // -1 is SPLIT_NONE
+            kern<<<dim3(ws.hadd_ld[g] / 128, (nfreq + HADC_FPB - 1) / HADC_FPB), HADC_NT, HADC_SMEM, s>>>(
+                ws.hadc_btab.p, spec, (CT*)ws.specA.p, ws.shead.p, ws.swin.p, tab + ws.hadd_tab0[g], ws.hadd_ld[g],
                 ws.hadd_row.p + ws.hadd_row0[g], ns, nt, nfreq, ws.status.p);
             XLAUNCH();
             ws.launches++;
@@ -3608,12 +3717,13 @@ struct Engine {
   }
 
   // the tiles of group g of the mixed path's Hadamard
-  static HadSys had_sys(Workspace& ws, int g, int ns, int nt) {
-    return HadSys{(const SplitC*)ws.specB.p,           (float2*)ws.specA.p, ws.hadh_tile.p + ws.had_tile0[g],
-                  ws.hadh_pslots.p,                    ws.hadh_tinv.p + ws.had_tile0[g],
-                  ws.hadh_tpass.p + ws.had_tile0[g],   ws.slevel.p,
-                  ws.hadh_tab.p,                       ws.hadh_rows.p,      ns,
-                  nt};
+  static HadSys had_sys(Workspace& ws, int g, int ns, int nt, bool screened = false) {
+    return HadSys{(const SplitC*)ws.specB.p,         (float2*)ws.specA.p,
+                  ws.hadh_tile.p + ws.had_tile0[g],  screened ? (const uint32_t*)ws.hadh_slots.p : ws.hadh_pslots.p,
+                  ws.hadh_tinv.p + ws.had_tile0[g],  ws.hadh_tpass.p + ws.had_tile0[g],
+                  ws.shead.p,                        ws.swin.p,
+                  ws.hadh_tab.p,                     ws.hadh_rows.p,
+                  ns,                                nt};
   }
 
   // the far field (M2P + L2P evaluation), added to the near field's values
@@ -3776,7 +3886,7 @@ void check_ready(const Fmm& f, const Tree& t) {
 }  // namespace
 
 // ================================================================ public (internal API)
-void m2l_fragments(LevelOps& op, const double* T64, int nfreq, bool mixed, cudaStream_t s) {
+void m2l_fragments(LevelOps& op, const double* T64, int nfreq, bool mixed, bool screened, cudaStream_t s) {
   static std::atomic<uint64_t> tables{0};
   op.m2l_id = ++tables;
   if (!mixed) {
@@ -3785,31 +3895,32 @@ void m2l_fragments(LevelOps& op, const double* T64, int nfreq, bool mixed, cudaS
     XLAUNCH();
     return;
   }
-  // every child pair's window (k_m2l_fragments)
-  DBuf<unsigned> pmax(26 * 64);
-  XCUDA(cudaMemsetAsync(pmax.p, 0, pmax.bytes(), s));
-  k_pair_max<<<dim3(std::min((nfreq + 3) / 4, 64), 26), 256, 0, s>>>((const double2*)T64, nfreq, pmax.p);
-  XLAUNCH();
-  const std::vector<unsigned> hm = pmax.download(s);  // the bits of floats >= 0
-  std::vector<uint8_t> hw(26 * 64, 255);              // 255: no factors, or below the FP32 range
-  op.m2l_windows = 1;
-  for (int i = 0; i < 26; i++) {
-    const int top = (int)(*std::max_element(hm.begin() + 64 * i, hm.begin() + 64 * (i + 1)) >> 23);
-    for (int k = 64 * i; k < 64 * (i + 1); k++) {
-      const int x = (int)(hm[k] >> 23);
-      if (x == 0) continue;
-      hw[k] = (uint8_t)((top - x) / (2 * SPLIT_WIN));
-      op.m2l_windows = std::max(op.m2l_windows, (int)hw[k] + 1);
-    }
-  }
   DBuf<uint8_t> pwin;
-  pwin.upload(hw, s);
+  op.m2l_windows = 1;
+  if (screened) {  // every child pair's window (k_m2l_fragments)
+    DBuf<unsigned> pmax(26 * 64);
+    XCUDA(cudaMemsetAsync(pmax.p, 0, pmax.bytes(), s));
+    k_pair_max<<<dim3(std::min((nfreq + 3) / 4, 64), 26), 256, 0, s>>>((const double2*)T64, nfreq, pmax.p);
+    XLAUNCH();
+    const std::vector<unsigned> hm = pmax.download(s);  // the bits of floats >= 0
+    std::vector<uint8_t> hw(26 * 64, 255);              // 255: no factors, or below the FP32 range
+    for (int i = 0; i < 26; i++) {
+      const int top = (int)(*std::max_element(hm.begin() + 64 * i, hm.begin() + 64 * (i + 1)) >> 23);
+      for (int k = 64 * i; k < 64 * (i + 1); k++) {
+        const int x = (int)(hm[k] >> 23);
+        if (x == 0) continue;
+        hw[k] = (uint8_t)((top - x) / SPLIT_WIN);
+        op.m2l_windows = std::max(op.m2l_windows, (int)hw[k] + 1);
+      }
+    }
+    pwin.upload(hw, s);
+  }
   op.m2l_frag.alloc((size_t)op.m2l_windows * nfreq * HADH_FB * sizeof(uint4));
   op.m2l_binv.alloc((size_t)op.m2l_windows * nfreq * 32);
   k_m2l_fragments<<<dim3(nblk(26ll * nfreq * 32), op.m2l_windows), 256, 0, s>>>(
-      (const double2*)T64, nfreq, pwin.p, (uint4*)op.m2l_frag.p, op.m2l_binv.p);
+      (const double2*)T64, nfreq, pwin.p, screened ? SPLIT_TAIL : 1.0, (uint4*)op.m2l_frag.p, op.m2l_binv.p);
   XLAUNCH();
-  XCUDA(cudaStreamSynchronize(s));  // pwin is released here
+  if (screened) XCUDA(cudaStreamSynchronize(s));  // pwin is released here
 }
 void set_charges(Fmm& f, Tree& t, const double* q, bool on_device, cudaStream_t s) {
   const int64_t n = t.nsrc;
@@ -4273,8 +4384,7 @@ void batch_evaluate(Batch* b, const double* const* charges, double* const* outs,
     if (b->nhtiles > 0) {
       const int tpc = std::max(1, b->had_tpc);
       k_hadamard_h_batch<<<dim3((b->nhtiles + tpc - 1) / tpc, b->had_nfreq), HADH_NT, HADH_SMEM, s>>>(
-          (const uint4*)b->had_op->m2l_frag.p, b->had_op->m2l_binv.p, b->had_op->m2l_windows, b->hsys.p, b->htiles.p,
-          b->nhtiles, tpc);
+          (const uint4*)b->had_op->m2l_frag.p, b->had_op->m2l_binv.p, b->hsys.p, b->htiles.p, b->nhtiles, tpc);
       XLAUNCH();
     }
     per_system(2 * E, 0, M2L_BWD, false);

@@ -613,7 +613,7 @@ void precompute(Fmm& f, int depth, cudaStream_t s) {
         if (named) dat.m2l[ti] = T64.download(s);
       }
       LevelOps& op = f.ops[l];
-      m2l_fragments(op, (const double*)T64.p, nfreq, single, s);
+      m2l_fragments(op, (const double*)T64.p, nfreq, single, f.screened(), s);
     }
     XCUDA(cudaStreamSynchronize(s));
     if (plan) cufftDestroy(plan);

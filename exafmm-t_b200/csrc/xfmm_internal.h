@@ -262,6 +262,8 @@ struct Fmm {
   std::vector<double> h_surf_base;
   double stage_ms[11] = {0};
   bool is_complex() const { return kernel == XFMM_HELMHOLTZ; }
+  // the field falls off exponentially
+  bool screened() const { return kernel == XFMM_MODIFIED_HELMHOLTZ || (kernel == XFMM_HELMHOLTZ && k_im != 0); }
   bool mixed() const { return precision == XFMM_MIXED; }
 };
 
@@ -275,7 +277,7 @@ void precompute(Fmm& fmm, int depth, cudaStream_t s);
 void host_surface_base(int p, std::vector<double>& out);
 void host_surface_lines(int p, const std::vector<double>& base, std::vector<int>& perm, std::vector<double>& grid);
 // evaluate.cu
-void m2l_fragments(LevelOps& op, const double* T64, int nfreq, bool mixed, cudaStream_t s);
+void m2l_fragments(LevelOps& op, const double* T64, int nfreq, bool mixed, bool screened, cudaStream_t s);
 void set_charges(Fmm& fmm, Tree& t, const double* q, bool on_device, cudaStream_t s);
 void clear_values(Fmm& fmm, Tree& t, cudaStream_t s);
 void upward_pass(Fmm& fmm, Tree& t, cudaStream_t s);
