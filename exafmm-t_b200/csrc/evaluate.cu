@@ -1462,9 +1462,9 @@ constexpr int HADC_TT = 512;  // padding of its source table
 // twice the targets of a spatially compact tile, each used by up to 26 of them) are brought into shared
 // memory once, on the exponent of the strongest, and every A fragment is read from there with ldmatrix, whose lanes
 // address the rows of a fragment freely: a gather without register moves at 8 shared-memory cycles per 16
-// targets and position.  Measured, Hadamard stage: 1M bodies, p = 10: 2.78 ms (the same products gathered
+// targets and position.  Measured, Hadamard stage: 1M bodies, p = 10: 2.8 ms (the same products gathered
 // row by row from L1 at 14 cycles per 16 targets: 4.03; the TF32 form with per-use conversions before it:
-// 5.26); 4M, p = 8, whose deepest level has ~7 of 26 positions occupied: 4.10 (TF32 with packed rounds of
+// 5.26); 4M, p = 8, whose deepest level has ~7 of 26 positions occupied: 4.1 (TF32 with packed rounds of
 // pairs and atomics: 6.15); Helmholtz 200k, p = 12: 1.71 (3.55).
 // Bank conflicts: a source's slot is 8 k + (octant of the source in its parent).  The sources of 8 sibling
 // targets at one relative position have 8 different octants, so their 64-byte rows (four 16-byte chunks,
@@ -2256,7 +2256,8 @@ __device__ __forceinline__ float abs1(float v) { return fabsf(v); }
 __device__ __forceinline__ float abs1(float2 v) { return fabsf(v.x) + fabsf(v.y); }
 // Screened kernels: the bound of every source's children (at child0[src[s]] + 0 .. 7).  Warp per child; the block
 // that finishes last sets the group's e0 from the largest.  A pass of its own over the sources' densities, since
-// the exponents of all sources stand on it (Yukawa sphere 300k: 0.02 ms).
+// the exponents of all sources stand on it (Yukawa sphere 300k: the forward stage 0.62 ms; with the bounds taken in the
+// transform and k_tile_codes after it 0.61).
 template <class W>
 __global__ void __launch_bounds__(256)
     k_source_bounds(const int* __restrict__ src, int ns, const int* __restrict__ child0, const W* __restrict__ up,

@@ -1,6 +1,6 @@
-"""The mixed M2L Hadamard keeps its accuracy for sources far weaker than others beside them: the split spectra have
-one exponent per source node and one of their own for its weak children, a tile takes sources of very different
-exponents in several passes, and the operator's factors have windows of their own.
+"""The mixed M2L Hadamard keeps its accuracy for sources far weaker than others beside them: a tile takes sources of
+very different size in several passes, and with the screened kernels children and the operator's factors have
+exponents by windows of 2^-28.
 
 A screened kernel shows a weak source: the strong one's field is gone where the weak one's targets are (k per box
 as large as the order's FP32 check potentials allow).  Each set of targets is compared with
